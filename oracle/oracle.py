@@ -301,9 +301,15 @@ def ref_root():
     return os.environ.get("PROTOMOL3_REF", "/root/reference")
 
 
+def have_ref_sources():
+    """Whether the reference's sources are there to compile (a directory with something in it)."""
+    root = ref_root()
+    return os.path.isdir(root) and bool(os.listdir(root))
+
+
 def build_ref(ref_root=None):
     ref_root = ref_root or globals()["ref_root"]()
-    if os.path.isdir(ref_root):
+    if os.path.isdir(ref_root) and os.listdir(ref_root):
         subprocess.check_call(["make", "-s", "-j8", "-C", HERE, "ref", "REF=" + ref_root])
     return ref_available()
 
