@@ -287,6 +287,9 @@ struct pmb_system {
   // events that fork it from and join it to the system stream
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_slots = nullptr, ev_join = nullptr;
+  // third stream, of the same priority: exclusion corrections and bonded terms beside the PME chain
+  cudaStream_t terms = nullptr;
+  cudaEvent_t ev_terms = nullptr;
   bool own_stream = false;
   Allocs a;
   std::vector<BoxDev> hbox;
@@ -371,6 +374,8 @@ struct pmb_system {
     if (h_status) cudaFreeHost(h_status);
     if (own_stream && stream) cudaStreamDestroy(stream);
     if (side) cudaStreamDestroy(side);
+    if (terms) cudaStreamDestroy(terms);
+    if (ev_terms) cudaEventDestroy(ev_terms);
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_slots) cudaEventDestroy(ev_slots);
     if (ev_join) cudaEventDestroy(ev_join);
@@ -402,10 +407,14 @@ int sort_cells(double edge, double min_edge) {
   return nc;
 }
 
+constexpr int PAIR_WARPS_PER_SM = 20;   // 5 CTAs of 4 warps
+constexpr int PAIR_UNITS_PER_WARP = 2;  // see nblist_alloc
+
 // Neighbour-list storage sized for list cutoff rl.
 int nblist_alloc(pmb_system *s, double rl) {
   cudaStreamSynchronize(s->stream);  // no kernel of the system may still read the old storage
   if (s->side) cudaStreamSynchronize(s->side);
+  if (s->terms) cudaStreamSynchronize(s->terms);
   s->nb_gen++;
   s->nba.~Allocs();
   new (&s->nba) Allocs();
@@ -417,7 +426,22 @@ int nblist_alloc(pmb_system *s, double rl) {
   nb.nslot = nblk * BLOCK;
   if ((long long)nblk * BLOCK >= JSAME) return fail(PMB_ERR_CAPACITY, "too many atoms for one system");
   std::vector<int> blk_box(nblk), jcap_off(nblk + 1, 0);
-  long long tiles = 0;
+  // Unit size of the pair kernel: about PAIR_UNITS_PER_WARP units for each warp the chip holds, so
+  // that the claims even out the load of a system of ordinary size (with 8-tile units one of 15,000
+  // atoms has about one unit per warp and one of 648 atoms keeps 100 warps busy for 29 us, with
+  // 2-tile units 13 us), up to UNIT_TILES for a large one, whose units then cost least (27,000
+  // atoms: 4.00 ms a run of 25 steps at 2 units per warp, 4.31 at 4 or 8).  Results do not depend
+  // on it.
+  int dev = 0;
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(&nb.n_sm, cudaDevAttrMultiProcessorCount, dev));
+  double tiles_est = 0.0;
+  for (const BoxDev &b : s->hbox)
+    tiles_est += b.nblk * (1.0 + std::min((double)b.natoms, b.natoms / (b.L[0] * b.L[1] * b.L[2]) * (4.0 / 3.0) * M_PI *
+                                                                std::pow(rl + 2.0, 3)) / (2 * JCHUNK));
+  const double per_warp = tiles_est / (nb.n_sm * PAIR_WARPS_PER_SM * PAIR_UNITS_PER_WARP);
+  nb.unit_tiles = std::max(CLOSE_TILES, std::min(UNIT_TILES, (int)(per_warp / CLOSE_TILES) * CLOSE_TILES));
+  long long units = 0;
   for (int bi = 0; bi < s->nbox; bi++) {
     const BoxDev &b = s->hbox[bi];
     // the box average, but at least a condensed-phase density (0.11 atoms/A^3): the atoms may
@@ -429,32 +453,29 @@ int nblist_alloc(pmb_system *s, double rl) {
     for (int k = 0; k < b.nblk; k++) {
       blk_box[b.blk0 + k] = bi;
       jcap_off[b.blk0 + k + 1] = cap;
-      tiles += 1 + cap / 32;
+      units += (cap / 32 + nb.unit_tiles - 1) / nb.unit_tiles + 1;
     }
   }
   for (int k = 0; k < nblk; k++) jcap_off[k + 1] += jcap_off[k];
-  tiles += (long long)s->nbox * (TILE_CHUNK - 1);  // each box's tiles start at a multiple of TILE_CHUNK
-  if (tiles > 0x7fffffffLL || jcap_off[nblk] < 0) return fail(PMB_ERR_CAPACITY, "neighbour list too large");
-  nb.tile_cap = (int)tiles;
+  if (units > 0x7fffffffLL || jcap_off[nblk] < 0) return fail(PMB_ERR_CAPACITY, "neighbour list too large");
+  nb.unit_cap = (int)units;
   int *d_blk_box, *d_jcap;
   if (upload(s->nba, d_blk_box, blk_box) || upload(s->nba, d_jcap, jcap_off)) return PMB_ERR_CUDA;
   nb.blk_box = d_blk_box;
   nb.jcap_off = d_jcap;
   nb.blk_lo = s->nba.get<uint4>(nblk);
   nb.blk_hi = s->nba.get<uint4>(nblk);
-  nb.nsblk = (nblk + 31) / 32;
-  nb.sblk_lo = s->nba.get<uint4>(nb.nsblk);
-  nb.sblk_hi = s->nba.get<uint4>(nb.nsblk);
+  for (const BoxDev &b : s->hbox) {
+    nb.nsblk += (b.nblk + 31) / 32;
+    nb.max_box_atoms = std::max(nb.max_box_atoms, b.natoms);
+  }
   nb.blk_c = s->nba.get<uint4>(nblk);
   nb.blk_h = s->nba.get<uint4>(nblk);
   nb.sblk_c = s->nba.get<uint4>(nb.nsblk);
   nb.sblk_h = s->nba.get<uint4>(nb.nsblk);
   nb.jcount = s->nba.get<int>(nblk + 1);
   nb.jlist = s->nba.get<int>((size_t)jcap_off[nblk], false);
-  nb.tile_off = s->nba.get<int>(nblk + 1);
-  nb.tile_start = s->nba.get<int>(nblk + 1);
-  nb.tile_blk = s->nba.get<int>(nb.tile_cap);
-  nb.tile_k = s->nba.get<int>(nb.tile_cap);
+  nb.units = s->nba.get<int4>(nb.unit_cap, false);
   nb.status = s->nba.get<int>(4);
   nb.slot_orig = s->nba.get<int>(nb.nslot, false);
   if (nb.slot_orig) cudaMemset(nb.slot_orig, 0xff, sizeof(int) * nb.nslot);  // -1 padding
@@ -464,24 +485,19 @@ int nblist_alloc(pmb_system *s, double rl) {
   nb.slot_meta = s->nba.get<int4>(nb.nslot);
   nb.fslot = s->nba.get<long long>(3 * (size_t)nb.nslot);
   // sort bins
-  std::vector<int> bin_box;
-  for (int bi = 0; bi < s->nbox; bi++) {
-    int ncm = std::max(s->hbox[bi].nc[0], std::max(s->hbox[bi].nc[1], s->hbox[bi].nc[2]));
-    long long nk = (long long)ncm * ncm * ncm;
-    bin_box.insert(bin_box.end(), (size_t)nk, bi);
-  }
-  nb.nkeys = (int)bin_box.size();
-  int *d_bin_box;
-  if (upload(s->nba, d_bin_box, bin_box)) return PMB_ERR_CUDA;
-  nb.bin_box = d_bin_box;
+  long long nkeys = 0;
+  for (const BoxDev &b : s->hbox) nkeys += std::max(4LL, (long long)b.nc[0] * b.nc[0] * b.nc[0]);
+  if (nkeys > 0x7fffffffLL) return fail(PMB_ERR_CAPACITY, "too many sort cells");
+  nb.nkeys = (int)nkeys;
   nb.key = s->nba.get<int>(s->natoms);
   nb.rank = s->nba.get<int>(s->natoms);
-  nb.bin_count = s->nba.get<int>(nb.nkeys + 1);
-  nb.bin_start = s->nba.get<int>(nb.nkeys + 1);
-  int maxn = std::max(nb.nkeys, nblk) + 1;
-  nb.scan_tmp = s->nba.get<int>(maxn / 4096 + 2);
+  nb.bin_count = s->nba.get<int>(nb.nkeys);
+  nb.bin_start = s->nba.get<int>(nb.nkeys);
+  nb.slot_raw = s->nba.get<int>(nb.nslot);
+  nb.slot_of = s->nba.get<int>(s->natoms, false);
+  if (nb.slot_of) cudaMemset(nb.slot_of, 0xff, sizeof(int) * s->natoms);  // -1: no slot yet
   nb.xref = s->nba.get<double>(3 * (size_t)s->natoms);
-  nb.ctl = s->nba.get<unsigned>(12);
+  nb.ctl = s->nba.get<unsigned>(CTL_WORDS);
   nb.vext = s->nba.get<int>(6 * (size_t)s->nbox);
   if (nb.vext) {
     std::vector<int> ext(6 * (size_t)s->nbox);
@@ -492,25 +508,16 @@ int nblist_alloc(pmb_system *s, double rl) {
   nb.nbox = s->nbox;
   nb.box_d2 = s->nba.get<unsigned>(s->nbox);
   nb.box_rb = s->nba.get<unsigned>(s->nbox);
-  nb.box_shift = s->nba.get<int>(s->nbox);
-  {
-    std::vector<int> order(s->nbox);
-    for (int b = 0; b < s->nbox; b++) order[b] = b;
-    std::sort(order.begin(), order.end(), [&](int a, int b) { return s->hbox[a].blk0 < s->hbox[b].blk0; });
-    int *d_order;
-    if (upload(s->nba, d_order, order)) return PMB_ERR_CUDA;
-    nb.box_order = d_order;
-  }
-  if (!nb.xref || !nb.ctl || !nb.vext || !nb.box_d2 || !nb.box_rb || !nb.box_shift || !nb.tile_start)
+  nb.box_done = s->nba.get<unsigned>(s->nbox);
+  if (!nb.xref || !nb.ctl || !nb.vext || !nb.box_d2 || !nb.box_rb || !nb.box_done || !nb.slot_of || !nb.slot_raw)
     return fail(PMB_ERR_CUDA, "cudaMalloc failed for the neighbour list");
-  // {max displacement, rebuild, finished blocks, forced rebuild, builds (64-bit), pair chunk
-  // counter and finished warps of the two pair launches, vacuum extent check}; first use builds
-  // the list
-  const unsigned ctl0[12] = {0u, 0u, 0u, 1u, 0u, 0u, 0u, 0u, 0u, 0u, s->vacuum ? 1u : 0u, 0u};
+  unsigned ctl0[CTL_WORDS] = {};
+  ctl0[CTL_FORCED] = 1u;  // the first use builds the list
+  ctl0[CTL_VACUUM] = s->vacuum ? 1u : 0u;
   CK(cudaMemcpy(nb.ctl, ctl0, sizeof(ctl0), cudaMemcpyHostToDevice));
   s->nb_build_rl = -1.0;
-  if (!nb.blk_lo || !nb.sblk_lo || !nb.sblk_hi || !nb.blk_c || !nb.blk_h || !nb.sblk_c || !nb.sblk_h || !nb.jlist || !nb.tile_blk || !nb.slot_meta || !nb.fslot ||
-      !nb.scan_tmp || !nb.bin_start)
+  if (!nb.blk_lo || !nb.blk_hi || !nb.blk_c || !nb.blk_h || !nb.sblk_c || !nb.sblk_h || !nb.jlist || !nb.units ||
+      !nb.slot_meta || !nb.fslot || !nb.key || !nb.rank || !nb.bin_count || !nb.bin_start)
     return fail(PMB_ERR_CUDA, "cudaMalloc failed for the neighbour list");
   s->nb_cutoff = rl;
   s->nb_ready = true;
@@ -605,15 +612,20 @@ void mark(void *ctx, const char *name) {
 }
 
 // Enqueues every force of the set on the system stream; accumulators must be zero.
-// The second (higher-priority) stream of the system and its fork / join events.
+// Captured kernels keep the priority of the stream they were captured on: without the flag a graph
+// runs at the priority of the stream it is launched into, and the PME kernels queue behind every
+// block of the pair kernel.
+constexpr unsigned GRAPH_FLAGS = cudaGraphInstantiateFlagUseNodePriority;
+
+// The second and third (higher-priority) streams of the system and the fork / join events.
 int ensure_side_stream(pmb_system *s) {
-  if (s->side) return PMB_OK;
+  if (s->terms) return PMB_OK;  // (made last)
   int lo = 0, hi = 0;
   CK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
-  CK(cudaStreamCreateWithPriority(&s->side, cudaStreamNonBlocking, hi));
-  CK(cudaEventCreateWithFlags(&s->ev_fork, cudaEventDisableTiming));
-  CK(cudaEventCreateWithFlags(&s->ev_slots, cudaEventDisableTiming));
-  CK(cudaEventCreateWithFlags(&s->ev_join, cudaEventDisableTiming));
+  if (!s->side) CK(cudaStreamCreateWithPriority(&s->side, cudaStreamNonBlocking, hi));
+  for (cudaEvent_t *e : {&s->ev_fork, &s->ev_slots, &s->ev_join, &s->ev_terms})
+    if (!*e) CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+  CK(cudaStreamCreateWithPriority(&s->terms, cudaStreamNonBlocking, hi));
   return PMB_OK;
 }
 
@@ -639,65 +651,76 @@ int enqueue_forces(pmb_system *s, pmb_force *const *fs, int n, int virial) {
   s->last_used_list = need_list;
   // PME, exclusion corrections and bonded terms run on the side stream beside the list build and
   // the pair kernel (every sum is an integer atomic, so the interleaving does not change a bit):
-  // the corrections and bonded terms from the start, the PME chain once this step's slot records
-  // are packed.  The stage profiler keeps everything in one stream to time each stage.
+  // both fork once this step's slot records are packed (beside the displacement check the terms
+  // held it up: 6 -> 12 us at 98,304 atoms), the PME chain and the terms each on a stream.  The
+  // stage profiler keeps everything in one stream to time each stage.
   bool others = false;
   for (int i = 0; i < n; i++) others |= fs[i]->kind == PMB_FORCE_PME || fs[i]->kind == PMB_FORCE_BONDED;
   bool split = !s->prof && !jobs.empty() && others && st != cudaStreamLegacy;
-  if (split && !s->side) {
+  if (split && !s->terms) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(st, &cs));
     if (cs != cudaStreamCaptureStatusNone) split = false;  // created outside a capture only
     else if (int rc = ensure_side_stream(s)) return rc;
   }
-  cudaStream_t so = st;
-  if (split) {
-    CK(cudaEventRecord(s->ev_fork, st));
-    CK(cudaStreamWaitEvent(s->side, s->ev_fork, 0));
-    so = s->side;
-  }
+  cudaStream_t so = split ? s->side : st, sterms = split ? s->terms : st;
   auto launch_recip = [&](pmb_force *f) {
     f->pm.virial = virial;
     pme_recip_launch(sd, s->nb, f->pm, so, mark, s);
   };
-  auto launch_atom_terms = [&](pmb_force *f) {  // exclusion corrections, bonded: no list needed
-    if (f->kind == PMB_FORCE_PME && f->d.correction) {
-      f->pm.virial = virial;
-      pme_correction_launch(sd, f->pm, s->d_excl_pairs, s->d_excl_kind, (int)s->h_excl_kind.size(),
-                            s->coulomb_scaling, so);
-      mark(s, "pme_correction");
-    } else if (f->kind == PMB_FORCE_BONDED) {
-      BondedDev b = s->bonded;
-      b.virial = virial;
-      bonded_launch(sd, b, so);
-      mark(s, "bonded");
+  // exclusion corrections, bonded terms: no list needed; a PME force's corrections and a bonded
+  // force share a launch, except under the stage profiler
+  auto launch_atom_terms = [&](pmb_force *c, pmb_force *b) {
+    CorrectionDev cd{};
+    if (c)
+      cd = CorrectionDev{(int)s->h_excl_kind.size(), s->d_excl_pairs, s->d_excl_kind, c->pm.alpha, c->pm.a2pi,
+                         s->coulomb_scaling, virial};
+    BondedDev bd = s->bonded;
+    bd.virial = virial;
+    atom_terms_launch(sd, c ? &cd : nullptr, b ? &bd : nullptr, sterms);
+    mark(s, c ? "pme_correction" : "bonded");
+  };
+  auto launch_all_atom_terms = [&]() {
+    std::vector<pmb_force *> corr, bonded;
+    for (int i = 0; i < n; i++) {
+      if (fs[i]->kind == PMB_FORCE_PME && fs[i]->d.correction) corr.push_back(fs[i]);
+      if (fs[i]->kind == PMB_FORCE_BONDED) bonded.push_back(fs[i]);
+    }
+    for (size_t k = 0; k < std::max(corr.size(), bonded.size()); k++) {
+      pmb_force *c = k < corr.size() ? corr[k] : nullptr, *b = k < bonded.size() ? bonded[k] : nullptr;
+      if (s->prof && c && b) {
+        launch_atom_terms(c, nullptr);
+        launch_atom_terms(nullptr, b);
+      } else {
+        launch_atom_terms(c, b);
+      }
     }
   };
-  if (split)
-    for (int i = 0; i < n; i++) launch_atom_terms(fs[i]);
   if (need_list) {
     const double rlist = list_radius(s, fs, n);
     int rc = ensure_nblist(s, rlist);
     if (rc) return rc;
     if (rlist != s->nb_build_rl) {  // a list built for another radius cannot be reused
-      CK(cudaMemsetAsync(s->nb.ctl + 3, 1, 1, st));
+      CK(cudaMemsetAsync(s->nb.ctl + CTL_FORCED, 1, 1, st));
       s->nb_build_rl = rlist;
     }
     nblist_sort(sd, s->nb, st);
-    if (split && need_pme_slots) {
+    if (split) {
       CK(cudaEventRecord(s->ev_slots, st));
       CK(cudaStreamWaitEvent(s->side, s->ev_slots, 0));
+      CK(cudaStreamWaitEvent(s->terms, s->ev_slots, 0));
       for (int i = 0; i < n; i++)
         if (fs[i]->kind == PMB_FORCE_PME && fs[i]->d.reciprocal) launch_recip(fs[i]);
+      launch_all_atom_terms();
     }
     nblist_lists(sd, s->nb, rlist, st);
     mark(s, "nblist");
   }
-  if (!split)
-    for (int i = 0; i < n; i++) {
+  if (!split) {
+    for (int i = 0; i < n; i++)
       if (fs[i]->kind == PMB_FORCE_PME && fs[i]->d.reciprocal) launch_recip(fs[i]);
-      launch_atom_terms(fs[i]);
-    }
+    launch_all_atom_terms();
+  }
   for (size_t q = 0; q < jobs.size(); q++) {
     const PairJob &j = jobs[q];
     PairLaunch pl;
@@ -707,38 +730,31 @@ int enqueue_forces(pmb_system *s, pmb_force *const *fs, int n, int virial) {
     pl.lattice = j.lattice;
     pl.multi = 0;
     pl.ctas_per_sm = s->pair_ctas;
-    pl.blk_lo = 0;
-    pl.blk_hi = s->nb.nblk_total;
+    pl.unit_kinds = 3;
     pl.wslot = 0;
-    int split_blk = -1;  // first block of the lattice-image suffix
-    if (j.p.coul_mode == 2 && j.lattice) {
-      int first = s->nb.nblk_total, nmulti = 0;
-      for (const BoxDev &b : s->hbox)
-        if (b.multi_image) {
-          pl.multi = 1;
-          first = std::min(first, b.blk0);
-          nmulti += b.nblk;
-        }
-      if (pl.multi && first > 0 && first + nmulti == s->nb.nblk_total) split_blk = first;
-    }
-    if (split_blk > 0) {
-      // the boxes that need no lattice image on the faster instance, the rest (a suffix of the
-      // tile map) on the lattice-image one, each with its own chunk counter
-      PairLaunch pa = pl, pb = pl;
-      pa.multi = 0;
-      pa.blk_hi = split_blk;
-      pb.blk_lo = split_blk;
+    int rc = 0;
+    bool single = false, multi = false;  // boxes without / with lattice images
+    for (const BoxDev &b : s->hbox) (b.multi_image ? multi : single) = true;
+    if (j.p.coul_mode == 2 && j.lattice && multi) {
+      // the boxes that need no lattice image on the faster instance, the rest on the
+      // lattice-image one, each with its own unit counter
+      PairLaunch pb = pl;
+      pb.multi = 1;
+      pb.unit_kinds = 2;
       pb.wslot = 1;
-      if (pair_launch(sd, s->nb, pa, st) || pair_launch(sd, s->nb, pb, st))
-        return fail(PMB_ERR_UNSUPPORTED, "too many LJ types");
-    } else if (pair_launch(sd, s->nb, pl, st)) {
-      return fail(PMB_ERR_UNSUPPORTED, "too many LJ types");
+      pl.unit_kinds = 1;
+      rc = (single && pair_launch(sd, s->nb, pl, st)) || pair_launch(sd, s->nb, pb, st);
+    } else {
+      rc = pair_launch(sd, s->nb, pl, st);
     }
+    if (rc) return fail(PMB_ERR_UNSUPPORTED, "too many LJ types");
     mark(s, "pair");
   }
   if (split) {
     CK(cudaEventRecord(s->ev_join, so));
     CK(cudaStreamWaitEvent(st, s->ev_join, 0));
+    CK(cudaEventRecord(s->ev_terms, sterms));
+    CK(cudaStreamWaitEvent(st, s->ev_terms, 0));
   }
   // slot-ordered pair forces -> facc (a plain read-modify-write: after the join)
   if (!jobs.empty()) pair_fold(sd, s->nb, st);
@@ -789,7 +805,7 @@ int eval_graph_launch(pmb_system *s, pmb_force *const *fs, int n, int virial, bo
     int rc = ensure_nblist(s, rlist);
     if (rc) return rc;
     if (rlist != s->nb_build_rl) {
-      CK(cudaMemsetAsync(s->nb.ctl + 3, 1, 1, st));
+      CK(cudaMemsetAsync(s->nb.ctl + CTL_FORCED, 1, 1, st));
       s->nb_build_rl = rlist;
     }
   }
@@ -855,7 +871,7 @@ int eval_graph_launch(pmb_system *s, pmb_force *const *fs, int n, int virial, bo
     ng.gen = s->nb_gen;
     ng.rlist = rlist;
     ng.used_list = s->last_used_list;
-    e = cudaGraphInstantiate(&ng.exec, graph, 0);
+    e = cudaGraphInstantiate(&ng.exec, graph, GRAPH_FLAGS);
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) return fail(PMB_ERR_CUDA, std::string("evaluation graph: ") + cudaGetErrorString(e));
     if ((int)s->eval_graphs.size() >= pmb_system::EVAL_GRAPHS) {
@@ -977,7 +993,7 @@ pmb_system *pmb_system_create(const pmb_box_desc *boxes, int n_boxes, int precis
     b.key0 = key0;
     b.nlat = 1;
     blk += b.nblk;
-    key0 += ncm * ncm * ncm;
+    key0 += std::max(4, ncm * ncm * ncm);  // (a multiple of 4: bins are read four at a time)
     s->hbox.push_back(b);
     int mmax = 0;
     for (int i = 0; i < d.n_atoms; i++) {
@@ -1057,10 +1073,12 @@ pmb_system *pmb_system_create(const pmb_box_desc *boxes, int n_boxes, int precis
     for (int bi = 0; bi < s->nbox; bi++) order[bi] = bi;
     auto min_edge = [&](int bi) { return std::min(s->hbox[bi].L[0], std::min(s->hbox[bi].L[1], s->hbox[bi].L[2])); };
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return min_edge(a) > min_edge(b); });
-    int b0 = 0;
+    int b0 = 0, sb0 = 0;
     for (int bi : order) {
       s->hbox[bi].blk0 = b0;
+      s->hbox[bi].sblk0 = sb0;
       b0 += s->hbox[bi].nblk;
+      sb0 += (s->hbox[bi].nblk + 31) / 32;
     }
   }
   int rc = 0;
@@ -1160,7 +1178,7 @@ int pmb_system_set_tuning(pmb_system *s, const pmb_tuning *t) {
       for (int k = 0; k < 3; k++) ncm = std::max(ncm, sort_cells(b.L[k], s->sort_cell));
       b.nc[0] = b.nc[1] = b.nc[2] = ncm;
       b.key0 = key0;
-      key0 += ncm * ncm * ncm;
+      key0 += std::max(4, ncm * ncm * ncm);
     }
     CK(cudaMemcpy(s->d_box, s->hbox.data(), sizeof(BoxDev) * s->hbox.size(), cudaMemcpyHostToDevice));
     s->nb_ready = false;
@@ -1193,7 +1211,7 @@ int pmb_system_list_builds(pmb_system *s, long long *n) {
   *n = 0;
   if (!s->nb_ready) return PMB_OK;
   unsigned long long v = 0;
-  CK(cudaMemcpyAsync(&v, s->nb.ctl + 4, sizeof(v), cudaMemcpyDeviceToHost, s->stream));
+  CK(cudaMemcpyAsync(&v, s->nb.ctl + CTL_BUILDS, sizeof(v), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
   *n = (long long)v;
   return PMB_OK;
@@ -1204,7 +1222,7 @@ int pmb_system_list_tiles(pmb_system *s, long long *tiles) {
   *tiles = 0;
   if (!s->nb_ready) return PMB_OK;
   int v = 0;
-  CK(cudaMemcpyAsync(&v, s->nb.tile_start + s->nb.nblk_total, sizeof(v), cudaMemcpyDeviceToHost, s->stream));
+  CK(cudaMemcpyAsync(&v, s->nb.ctl + CTL_TILES, sizeof(v), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
   *tiles = v;
   return PMB_OK;
@@ -1878,7 +1896,7 @@ int md_prepare_list(pmb_md *m) {
   int rc = ensure_nblist(s, rlist);
   if (rc) return rc;
   if (rlist != s->nb_build_rl) {
-    CK(cudaMemsetAsync(s->nb.ctl + 3, 1, 1, s->stream));
+    CK(cudaMemsetAsync(s->nb.ctl + CTL_FORCED, 1, 1, s->stream));
     s->nb_build_rl = rlist;
   }
   return PMB_OK;
@@ -1906,7 +1924,7 @@ int md_capture(pmb_md *m, double kick, cudaGraphExec_t *out) {
       }
     m->kernels_per_step = kern;
   }
-  e = cudaGraphInstantiate(out, g, 0);
+  e = cudaGraphInstantiate(out, g, GRAPH_FLAGS);
   cudaGraphDestroy(g);
   if (e != cudaSuccess) return fail(PMB_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
   return PMB_OK;
@@ -2177,7 +2195,7 @@ int pmb_md_set_checkpoint(pmb_md *m, const double *pos, const double *vel, const
       // build is deterministic), so that every later step sums the same tiles in the same order
       CK(cudaMemcpyAsync(s->d_pos, list_reference, bytes, cudaMemcpyHostToDevice, s->stream));
       s->have_pos = true;
-      if (s->nb_ready) CK(cudaMemsetAsync(s->nb.ctl + 3, 1, 1, s->stream));  // rebuild
+      if (s->nb_ready) CK(cudaMemsetAsync(s->nb.ctl + CTL_FORCED, 1, 1, s->stream));  // rebuild
       zero_accumulators(sd, s->stream);
       rc = enqueue_forces(s, m->forces.data(), (int)m->forces.size(), m->virial ? 1 : 0);
       if (rc) return rc;

@@ -29,11 +29,9 @@ constexpr int BLOCK = 8;           // atoms per i-cluster (a lane group; the j-c
 constexpr int GROUPS = 32 / BLOCK; // lane groups per warp
 static_assert(BLOCK == 8 || BLOCK == 16, "i-cluster of 8 or 16 atoms");
 constexpr int JCHUNK = 32;         // j-atoms per tile
-#ifndef PAIR_TILE_CHUNK
-#define PAIR_TILE_CHUNK 8
-#endif
-constexpr int TILE_CHUNK = PAIR_TILE_CHUNK;  // consecutive tiles per warp assignment of the pair
-                                             // kernel; each box's tiles start at a multiple of it
+constexpr int UNIT_TILES = 8;   // most tiles of one list per warp assignment of the pair kernel
+constexpr int CLOSE_TILES = 2;  // tiles of a list after which its floating-point sums are closed
+                                // in fixed point; units start at multiples of it
 constexpr int JSAME = 1 << 30;     // j-list flag: the j-atom shares a molecule with the i-cluster
 constexpr int MAX_LJ_TYPES = 32;   // LJ table kept in shared memory up to this many types
 
@@ -46,7 +44,7 @@ struct BoxDev {
   int nc[3];             // sort grid (cells per edge)
   int multi_image;       // Ewald real space must loop lattice images (edge < 2 cutoff)
   int lat0, nlat;        // lattice vectors for multi-image boxes (first is (0,0,0))
-  int pad_;
+  int sblk0;             // first superblock (run of 32 blocks) of this box
 };
 
 // Switching function constants (switch/C1SwitchingFunction.cpp:12-16, C2SwitchingFunction.cpp:12-18).
@@ -98,47 +96,67 @@ __device__ inline long long warp_sum_ll(long long v) {
   return v;
 }
 
-// Adds one energy (slot) and optionally a symmetric virial (xx xy xz yy yz zz) per lane to the
-// per-box accumulators.  Every term is rounded to fixed point on its own, so a box's sum does not
-// depend on which terms of other boxes share its warps; when every valid lane of the warp belongs
-// to the same box the warp adds the integers first (one atomic per warp instead of 32 on the
-// same address).
-__device__ inline void box_accumulate(long long *eacc, int box, bool valid, int slot, double e,
-                                      const double *vir6) {
-  const int lane = threadIdx.x & 31;
-  const unsigned act = __ballot_sync(0xffffffffu, valid);
-  if (!act) return;
-  const int b0 = __shfl_sync(0xffffffffu, box, __ffs(act) - 1);
-  const bool same = __all_sync(0xffffffffu, !valid || box == b0);
-  const int map[6][2] = {{0, 0}, {1, 3}, {2, 6}, {4, 4}, {5, 7}, {8, 8}};
-  const long long ev = valid ? f2fix(e, ENERGY_SCALE) : 0;
-  long long vv[6] = {0, 0, 0, 0, 0, 0};
-  if (vir6 && valid)
-    for (int c = 0; c < 6; c++) vv[c] = f2fix(vir6[c], ENERGY_SCALE);
-  if (same) {
-    const long long es = warp_sum_ll(ev);
-    long long vs[6];
-    if (vir6)
-      for (int c = 0; c < 6; c++) vs[c] = warp_sum_ll(vv[c]);
-    if (lane == 0) {
-      long long *acc = eacc + (long long)b0 * ACC_PER_BOX;
-      red_add(acc + slot, es);
-      if (vir6)
-        for (int c = 0; c < 6; c++) {
-          red_add(acc + E_VIR + map[c][0], vs[c]);
-          if (map[c][1] != map[c][0]) red_add(acc + E_VIR + map[c][1], vs[c]);
-        }
-    }
-  } else if (valid) {
+// One energy (slot) and optionally a symmetric virial (xx xy xz yy yz zz) per lane and call, added to
+// the per-box accumulators.  Every term is rounded to fixed point on its own, so a box's sum does
+// not depend on which terms of other boxes share its warps; while every valid lane of the warp
+// belongs to the same box the integers are kept per lane, and the warp adds them together once
+// (one atomic per warp instead of 32 per call on the same address) when the box changes and at the
+// end.  All lanes of the warp make every call.
+template <bool VIR>
+struct BoxSums {
+  long long *eacc;
+  int slot, box = -1;
+  long long e = 0, v[VIR ? 6 : 1] = {};
+  __device__ BoxSums(long long *acc, int s) : eacc(acc), slot(s) {}
+  __device__ static void add(long long *eacc, int box, int slot, long long ev, const long long *vv) {
     long long *acc = eacc + (long long)box * ACC_PER_BOX;
-    red_add(acc + slot, ev);
-    if (vir6)
+    if (ev) red_add(acc + slot, ev);
+    if constexpr (VIR) {
+      const int map[6][2] = {{0, 0}, {1, 3}, {2, 6}, {4, 4}, {5, 7}, {8, 8}};
+#pragma unroll
       for (int c = 0; c < 6; c++) {
         red_add(acc + E_VIR + map[c][0], vv[c]);
         if (map[c][1] != map[c][0]) red_add(acc + E_VIR + map[c][1], vv[c]);
       }
+    }
   }
-}
+  __device__ void flush() {
+    if (box < 0) return;
+    long long s = warp_sum_ll(e), w[VIR ? 6 : 1] = {};
+    if constexpr (VIR)
+#pragma unroll
+      for (int c = 0; c < 6; c++) w[c] = warp_sum_ll(v[c]);
+    if ((threadIdx.x & 31) == 0) add(eacc, box, slot, s, w);
+    e = 0;
+    if constexpr (VIR)
+#pragma unroll
+      for (int c = 0; c < 6; c++) v[c] = 0;
+  }
+  __device__ void term(int b, bool valid, double en, const double *vir6) {
+    const unsigned act = __ballot_sync(0xffffffffu, valid);
+    if (!act) return;
+    const int b0 = __shfl_sync(0xffffffffu, b, __ffs(act) - 1);
+    const bool same = __all_sync(0xffffffffu, !valid || b == b0);
+    const long long ev = valid ? f2fix(en, ENERGY_SCALE) : 0;
+    long long vv[VIR ? 6 : 1] = {};
+    if constexpr (VIR)
+      if (valid)
+#pragma unroll
+        for (int c = 0; c < 6; c++) vv[c] = f2fix(vir6[c], ENERGY_SCALE);
+    if (same) {
+      if (b0 != box) {
+        flush();
+        box = b0;
+      }
+      e += ev;
+      if constexpr (VIR)
+#pragma unroll
+        for (int c = 0; c < 6; c++) v[c] += vv[c];
+    } else if (valid) {
+      add(eacc, b, slot, ev, vv);
+    }
+  }
+};
 
 // Switching function value and derivative/r (same branch structure as the reference).
 template <typename T>

@@ -35,6 +35,19 @@ inline int device_slot() {
 }
 
 // ------------------------------------------------------------------ neighbour list (nblist.cu)
+// Control words of a list.
+enum {
+  CTL_REBUILD = 1,  // some box rebuilds this step
+  CTL_BLOCKS = 2,   // finished blocks of the displacement check
+  CTL_FORCED = 3,   // every box rebuilds at the next check
+  CTL_BUILDS = 4,   // list builds so far (64 bits)
+  CTL_PAIR = 6,     // the pair kernel's next unit and finished warps, two launches; zero between them
+  CTL_VACUUM = 10,  // check the extent of vacuum boxes
+  CTL_CLAIM = 11,   // the list build's next block
+  CTL_UNITS = 12,   // pair units of boxes without and with lattice images
+  CTL_TILES = 14,   // tiles of all lists
+  CTL_WORDS = 16
+};
 struct NbListDev {
   // per block
   int nblk_total;
@@ -42,19 +55,17 @@ struct NbListDev {
   float4 *blk_center;          // [nblk] fractional-fixed centre (as uint bits) and count
   uint4 *blk_lo, *blk_hi;      // [nblk] fixed-point extents (x, y, z)
   uint4 *blk_c, *blk_h;        // [nblk] the same as centre (.w = atoms) and half extent
-  int nsblk;                   // superblocks: runs of 32 consecutive blocks
-  uint4 *sblk_lo, *sblk_hi;    // [nsblk] union of their blocks' extents, .w = atoms
-  uint4 *sblk_c, *sblk_h;      // [nsblk] the same as centre (.w = atoms) and half extent
+  int nsblk;                   // superblocks: runs of 32 consecutive blocks of a box
+  uint4 *sblk_c, *sblk_h;      // [nsblk] union of their blocks' extents: centre (.w = atoms), half extent
   int *jcap_off;               // [nblk+1] offset of each block's j-slot list region
   int *jcount;                 // [nblk] tiles per block (its j-list, own slots first, in 32s)
   int *jlist;                  // [jcap_off[nblk]] j slots (-1 padding), JSAME flag bit
-  int *tile_off;               // [nblk+1] exclusive scan of jcount
-  int *tile_start;             // [nblk+1] first tile of each block: tile_off moved on so that
-                               // each box's tiles start at a multiple of TILE_CHUNK (a box's
-                               // last block is followed by up to TILE_CHUNK - 1 empty tiles)
-  int *tile_blk;               // [tile_cap] block of each tile (-1: empty)
-  int *tile_k;                 // [tile_cap] tile index within the block
-  int tile_cap;
+  int4 *units;                 // [unit_cap] pair kernel work: block, first tile, tiles, offset of the
+                               // first tile in jlist; boxes that
+                               // need lattice images from the end of the array, the others from
+                               // the front (ctl[CTL_UNITS + 1] and ctl[CTL_UNITS] of them)
+  int unit_cap;
+  int unit_tiles;              // most tiles of a unit: CLOSE_TILES .. UNIT_TILES
   int *status;                 // [4]: list / tile overflow, non-finite position, vacuum extent
   // per slot
   int nslot;
@@ -66,29 +77,27 @@ struct NbListDev {
                                // folded into facc and cleared after the pair kernels
   // sort
   int nkeys;
-  int *key;                    // [natoms]
+  int *key;                    // [natoms] sort bin within the atom's box
   int *rank;                   // [natoms]
-  int *bin_count;              // [nkeys + 1]
-  int *bin_start;              // [nkeys + 1]
-  int *scan_tmp;               // scratch for scans
-  const int *bin_box;          // [nkeys] box of each sort bin
+  int *bin_count;              // [nkeys] zero between builds
+  int *bin_start;              // [nkeys] relative to the box's first slot
+  int *slot_raw;               // [nslot] atoms by bin, before they are ordered within the bins
+  int *slot_of;                // [natoms] slot of each atom (-1 before the first build)
+  int max_box_atoms, n_sm;     // largest box; SMs of the device
   int want_fp64;               // also pack raw double positions
   // list reuse: the list is built with cutoff + skin and rebuilt only once some atom moved more
   // than skin/2 since the last build (decided on the device, every step)
   double *xref;                // [3 natoms] positions at the last build
-  unsigned *ctl;               // [8] max displacement^2 (float bits), rebuild flag, block counter,
-                               // force flag, list builds (64-bit counter in [4..5]), the pair
-                               // kernel's next chunk and finished warps ([6], [7]; zero between launches)
+  unsigned *ctl;               // [CTL_WORDS], see below
   float half_skin2;
   // per box: rebuilds are decided box by box (a box's list, slot order and therefore its
-  // rounding do not depend on the other boxes of the system); ctl[1] says whether any box rebuilds
+  // rounding do not depend on the other boxes of the system); ctl[CTL_REBUILD]: any box rebuilds
   int nbox;
   unsigned *box_d2;            // [nbox] max displacement^2 since the box's last build (float bits)
   unsigned *box_rb;            // [nbox] 1: the box rebuilds this step
-  const int *box_order;        // [nbox] the boxes in ascending order of their first block
-  int *box_shift;              // [nbox] tiles of padding before the box's first tile
+  unsigned *box_done;          // [nbox] finished CTAs of the histogram; zero between launches
   int *vext;                   // [6 nbox] vacuum extent per box: smallest and largest x, y, z as
-                               // order-preserving int images of their float values (ctl[10] on)
+                               // order-preserving int images of their float values (CTL_VACUUM on)
 };
 
 struct SystemDev {
@@ -116,8 +125,9 @@ struct PairLaunch {
   const double *lattice;          // [nlat_total*3]
   int multi;                      // some box needs Ewald lattice images
   int ctas_per_sm;                // resident CTAs per SM of the persistent kernel (0: all that fit)
-  int blk_lo, blk_hi;             // the blocks whose tiles this launch evaluates
-  int wslot;                      // which chunk counter of the list's ctl words it uses (0 or 1)
+  int unit_kinds;                 // units it evaluates: bit 0 those of boxes without lattice images,
+                                  // bit 1 those of boxes with
+  int wslot;                      // which unit counter of the list's ctl words it uses (0 or 1)
   PairParams p;
 };
 int pair_launch(const SystemDev &s, const NbListDev &nb, const PairLaunch &pl, cudaStream_t st);
@@ -182,8 +192,6 @@ int pme_line_capacity();
 // Exact Ewald reciprocal sum of one box (pmb_ewald.cu): S, C [nk] and the box's forces in fout.
 int ewald_recip_launch(const double *pos, const double *charge, int atom0, int n, const double3 *kv,
                        const double *a, int nk, double *S, double *Cc, double *fout, cudaStream_t st);
-int pme_correction_launch(const SystemDev &s, const PmeDev &pm, const int *excl_pairs,
-                          const int *excl_kind, int nexcl, double coulomb_scaling, cudaStream_t st);
 
 // ------------------------------------------------------------------ bonded / integrator (md.cu)
 struct BondedDev {
@@ -194,7 +202,15 @@ struct BondedDev {
   const double *angle_k, *angle_theta0, *ub_k, *ub_r0;
   int virial;
 };
-int bonded_launch(const SystemDev &s, const BondedDev &b, cudaStream_t st);
+// Exclusion corrections of a PME force: the pairs, and its splitting parameter.
+struct CorrectionDev {
+  int n;
+  const int *pairs, *kind;
+  double alpha, a2pi, coulomb_scaling;
+  int virial;
+};
+// Exclusion corrections and bonded terms in one launch (either may be null).
+int atom_terms_launch(const SystemDev &s, const CorrectionDev *c, const BondedDev *b, cudaStream_t st);
 // out = base + the accumulated forces (base may be null)
 int forces_to_double(const SystemDev &s, double *out, cudaStream_t st, const double *base = nullptr);
 int energies_to_double(const SystemDev &s, const double *const_e, double *out, cudaStream_t st);

@@ -15,8 +15,38 @@ namespace pmb {
 
 namespace {
 
-__global__ void k_bonds(const SystemDev s, BondedDev b) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
+// Exclusion correction in FP64 with the exact erf (NonbondedPMEwaldSystemForce.h:874-911).
+template <bool VIR>
+__device__ __forceinline__ void correction_term(const SystemDev &s, BoxSums<VIR> &sums, const CorrectionDev &c, int k) {
+  bool valid = k < c.n;
+  double en = 0.0, vir[6] = {0, 0, 0, 0, 0, 0};
+  int box = -1;
+  if (valid) {
+    int a1 = c.pairs[2 * k], a2 = c.pairs[2 * k + 1];
+    box = s.atom_box[a1];
+    const BoxDev &b = s.box[box];
+    double rij[3];
+    double r2 = min_diff(b, s.pos + 3 * a1, s.pos + 3 * a2, rij);
+    double qq = s.charge[a1] * s.charge[a2];
+    if (c.kind[k] == 1) qq *= 1 - c.coulomb_scaling;
+    double r = sqrt(r2), rr = 1 / r, e = erf(c.alpha * r) * rr;
+    en = -qq * e;
+    double fs = qq * (c.a2pi * exp(-c.alpha * c.alpha * r2) - e) * rr * rr;
+    double fij[3] = {rij[0] * fs, rij[1] * fs, rij[2] * fs};
+    long long *f1 = s.facc + 3 * (long long)a1, *f2 = s.facc + 3 * (long long)a2;
+    for (int q = 0; q < 3; q++) {
+      long long v = f2fix(fij[q], FORCE_SCALE);
+      red_add(f1 + q, -v);
+      red_add(f2 + q, v);
+    }
+    vir[0] = fij[0] * rij[0]; vir[1] = fij[0] * rij[1]; vir[2] = fij[0] * rij[2];
+    vir[3] = fij[1] * rij[1]; vir[4] = fij[1] * rij[2]; vir[5] = fij[2] * rij[2];
+  }
+  sums.term(box, valid, en, vir);
+}
+
+template <bool VIR>
+__device__ __forceinline__ void bond_term(const SystemDev &s, BoxSums<VIR> &sums, const BondedDev &b, int k) {
   bool valid = k < b.nbonds;
   int box = -1;
   double en = 0.0, vir[6] = {0, 0, 0, 0, 0, 0};
@@ -37,11 +67,11 @@ __global__ void k_bonds(const SystemDev s, BondedDev b) {
     vir[0] = f1[0] * r12[0]; vir[1] = f1[0] * r12[1]; vir[2] = f1[0] * r12[2];
     vir[3] = f1[1] * r12[1]; vir[4] = f1[1] * r12[2]; vir[5] = f1[2] * r12[2];
   }
-  box_accumulate(s.eacc, box, valid, E_BOND, en, b.virial ? vir : nullptr);
+  sums.term(box, valid, en, vir);
 }
 
-__global__ void k_angles(const SystemDev s, BondedDev b) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
+template <bool VIR>
+__device__ __forceinline__ void angle_term(const SystemDev &s, BoxSums<VIR> &sums, const BondedDev &b, int k) {
   bool valid = k < b.nangles;
   int box = -1;
   double en = 0.0, vir[6] = {0, 0, 0, 0, 0, 0};
@@ -81,7 +111,29 @@ __global__ void k_angles(const SystemDev s, BondedDev b) {
     vir[2] = f1[0] * r12[2] + f3[0] * r32[2]; vir[3] = f1[1] * r12[1] + f3[1] * r32[1];
     vir[4] = f1[1] * r12[2] + f3[1] * r32[2]; vir[5] = f1[2] * r12[2] + f3[2] * r32[2];
   }
-  box_accumulate(s.eacc, box, valid, E_ANGLE, en, b.virial ? vir : nullptr);
+  sums.term(box, valid, en, vir);
+}
+
+// Corrections, bonds and angles side by side, each on its own blocks: one launch for three.
+// Latency-bound (a few dependent loads and FP64 functions); a block takes `per` consecutive terms,
+// so that the sums of a large system meet in a few hundred atomics on the same words and not in
+// one per 32 terms.
+constexpr int ATOM_TERM_THREADS = 128;
+constexpr int ATOM_TERM_BLOCKS = 592;  // about this many blocks for a large system: 4 per SM
+template <bool VIR>
+__global__ void __launch_bounds__(ATOM_TERM_THREADS)
+    k_atom_terms(const SystemDev s, CorrectionDev c, BondedDev b, int per, int angle_blocks, int corr_blocks) {
+  int blk = blockIdx.x;  // the longest terms first
+  const int kind = blk < angle_blocks ? 0 : blk < angle_blocks + corr_blocks ? 1 : 2;
+  blk -= kind == 0 ? 0 : kind == 1 ? angle_blocks : angle_blocks + corr_blocks;
+  BoxSums<VIR> sums(s.eacc, kind == 0 ? E_ANGLE : kind == 1 ? E_COUL : E_BOND);
+  for (int q = 0; q < per; q += ATOM_TERM_THREADS) {
+    const int k = blk * per + q + threadIdx.x;
+    if (kind == 0) angle_term<VIR>(s, sums, b, k);
+    else if (kind == 1) correction_term<VIR>(s, sums, c, k);
+    else bond_term<VIR>(s, sums, b, k);
+  }
+  sums.flush();
 }
 
 __global__ void k_forces_to_double(const SystemDev s, double *out, const double *base) {
@@ -706,10 +758,16 @@ int fp32_peak_probe(double *tflops) {
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-int bonded_launch(const SystemDev &s, const BondedDev &b, cudaStream_t st) {
-  const int T = 256;
-  if (b.nbonds > 0) k_bonds<<<(b.nbonds + T - 1) / T, T, 0, st>>>(s, b);
-  if (b.nangles > 0) k_angles<<<(b.nangles + T - 1) / T, T, 0, st>>>(s, b);
+int atom_terms_launch(const SystemDev &s, const CorrectionDev *c, const BondedDev *b, cudaStream_t st) {
+  const CorrectionDev c0 = c ? *c : CorrectionDev{};
+  const BondedDev b0 = b ? *b : BondedDev{};
+  const int T = ATOM_TERM_THREADS;
+  const long long all = (long long)b0.nangles + c0.n + b0.nbonds;
+  const int per = (int)(all / ATOM_TERM_BLOCKS / T + 1) * T;
+  const int na = (b0.nangles + per - 1) / per, nc = (c0.n + per - 1) / per, nb = (b0.nbonds + per - 1) / per;
+  if (na + nc + nb <= 0) return 0;
+  if (c0.virial || b0.virial) k_atom_terms<true><<<na + nc + nb, T, 0, st>>>(s, c0, b0, per, na, nc);
+  else k_atom_terms<false><<<na + nc + nb, T, 0, st>>>(s, c0, b0, per, na, nc);
   return 0;
 }
 

@@ -13,8 +13,6 @@ namespace pmb {
 
 namespace {
 
-constexpr int SCAN_CHUNK = 4096;  // elements per CTA (1024 threads x 4)
-
 // Index of cell (x, y, z) along a 3-D Hilbert curve over a 2^bits grid (J. Skilling, "Programming
 // the Hilbert curve", AIP Conf. Proc. 707, 381 (2004): axes -> transposed index, then bit
 // interleave).  Consecutive cells are face neighbours, so a run of slots never jumps across the
@@ -89,62 +87,14 @@ __device__ int block_exclusive_scan(int v, int *total) {
   return off + x - v;
 }
 
-__global__ void k_scan_reduce(const int *in, int n, int *chunk, const unsigned *go) {
-  if (go && !go[1]) return;
-  long long base = (long long)blockIdx.x * SCAN_CHUNK + threadIdx.x * 4;
-  int s = 0;
-#pragma unroll
-  for (int k = 0; k < 4; k++)
-    if (base + k < n) s += in[base + k];
-  int tot;
-  block_exclusive_scan(s, &tot);
-  if (threadIdx.x == 0) chunk[blockIdx.x] = tot;
-}
-
-__global__ void k_scan_chunks(int *chunk, int nchunk, const unsigned *go) {
-  if (go && !go[1]) return;
-  __shared__ int carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (int b = 0; b < nchunk; b += blockDim.x) {
-    int i = b + threadIdx.x;
-    int v = i < nchunk ? chunk[i] : 0;
-    int tot;
-    int ex = block_exclusive_scan(v, &tot);
-    if (i < nchunk) chunk[i] = carry + ex;
-    __syncthreads();
-    if (threadIdx.x == 0) carry += tot;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) chunk[nchunk] = carry;
-}
-
-__global__ void k_scan_apply(const int *in, int n, const int *chunk, int *out, const unsigned *go) {
-  if (go && !go[1]) return;
-  long long base = (long long)blockIdx.x * SCAN_CHUNK + threadIdx.x * 4;
-  int v[4], s = 0;
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    v[k] = (base + k < n) ? in[base + k] : 0;
-    s += v[k];
-  }
-  int ex = block_exclusive_scan(s, nullptr) + chunk[blockIdx.x];
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    if (base + k < n) out[base + k] = ex;
-    ex += v[k];
-  }
-  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = chunk[gridDim.x];
-}
-
 // ---------------------------------------------------------------- binning and sort
 // Rebuild decision, box by box: max |x - x_ref|^2 over each box's atoms (box_d2), then the last
-// block sets box_rb[b] for every box that moved more than half the skin and ctl[1] when any did
-// (no host round trip); ctl = {-, any box rebuilds, finished blocks, forced rebuild of all}.
+// block sets box_rb[b] for every box that moved more than half the skin and ctl[CTL_REBUILD] when
+// any did (no host round trip).
 // It reads every position of every evaluation, so it also raises status[2] for a non-finite
 // one (the host reports PMB_ERR_NUMERIC; every later kernel maps such a position to an in-range
 // cell and grid index, so nothing reads out of bounds meanwhile), and, for a system whose boxes
-// stand in for vacuum (ctl[10]), status[3] once the atoms of a box spread over half an edge
+// stand in for vacuum (ctl[CTL_VACUUM]), status[3] once the atoms of a box spread over half an edge
 // (the minimal image would no longer be the plain difference).
 __device__ __forceinline__ int ford(float f) {  // order-preserving int image of a float
   const int i = __float_as_int(f);
@@ -152,14 +102,31 @@ __device__ __forceinline__ int ford(float f) {  // order-preserving int image of
 }
 __device__ __forceinline__ float fuord(int o) { return __int_as_float(o >= 0 ? o : o ^ 0x7fffffff); }
 
-__global__ void k_disp_check(SystemDev s, NbListDev nb) {
+//
+// The same pass writes this step's coordinates into the atom's slot record (the slot it got at
+// its box's last build; a box that is rebuilt packs its records again afterwards), so a step
+// without a rebuild has no pass of its own for that.
+__global__ void k_update(SystemDev s, NbListDev nb) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   float d2 = 0.f;
   int box = -1;
-  const bool vacuum = nb.ctl[10] != 0u;
+  const bool vacuum = nb.ctl[CTL_VACUUM] != 0u;
   if (i < s.natoms) {
     box = s.atom_box[i];
     const double x = s.pos[3 * i], y = s.pos[3 * i + 1], z = s.pos[3 * i + 2];
+    const int sl = nb.slot_of[i];
+    if (sl >= 0) {
+      const BoxDev &b = s.box[box];
+      // x, y, z of the record; the charge in its last word stays
+      uint4 *f = nb.slot_fx + sl;
+      *reinterpret_cast<uint2 *>(f) = make_uint2(frac_fixed(x, b.Lr[0]), frac_fixed(y, b.Lr[1]));
+      f->z = frac_fixed(z, b.Lr[2]);
+      if (nb.want_fp64) {
+        double4 *q = nb.slot_pq + sl;
+        *reinterpret_cast<double2 *>(q) = make_double2(x, y);
+        q->z = z;
+      }
+    }
     if (!(isfinite(x) && isfinite(y) && isfinite(z))) atomicExch(&nb.status[2], 1);
     if (vacuum) {
       int *e = nb.vext + 6 * s.atom_box[i];
@@ -216,11 +183,11 @@ __global__ void k_disp_check(SystemDev s, NbListDev nb) {
   __threadfence();
   __syncthreads();
   __shared__ bool last;
-  if (threadIdx.x == 0) last = atomicAdd(&nb.ctl[2], 1u) == gridDim.x - 1;
+  if (threadIdx.x == 0) last = atomicAdd(&nb.ctl[CTL_BLOCKS], 1u) == gridDim.x - 1;
   __syncthreads();
   if (!last) return;
   __threadfence();
-  const bool forced = nb.ctl[3] != 0u;
+  const bool forced = nb.ctl[CTL_FORCED] != 0u;
   int any = 0;
   for (int b = threadIdx.x; b < s.nbox; b += blockDim.x) {
     const float mx = __uint_as_float(atomicExch(&nb.box_d2[b], 0u));  // read and reset
@@ -237,156 +204,217 @@ __global__ void k_disp_check(SystemDev s, NbListDev nb) {
   }
   any = __syncthreads_or(any);
   if (threadIdx.x == 0) {
-    nb.ctl[1] = any ? 1u : 0u;
-    if (any) ++*reinterpret_cast<unsigned long long *>(nb.ctl + 4);
-    nb.ctl[2] = 0u;
-    nb.ctl[3] = 0u;
-  }
-}
-
-__global__ void k_zero_bins(int *bin_count, int n, const unsigned *go) {
-  if (!go[1]) return;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i <= n) bin_count[i] = 0;
-}
-
-__global__ void k_bin(SystemDev s, int *key, int *rank, int *bin_count, const unsigned *go, const unsigned *rb) {
-  if (!go[1]) return;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= s.natoms) return;
-  const int bi = s.atom_box[i];
-  if (!rb[bi]) return;  // the box keeps its slots
-  const BoxDev &b = s.box[bi];
-  unsigned c[3];
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    unsigned f = frac_fixed(s.pos[3 * i + k], b.Lr[k]);
-    c[k] = (unsigned)(((unsigned long long)f * (unsigned)b.nc[k]) >> 32);
-  }
-  int kk = b.key0 + (int)hilbert3(c[0], c[1], c[2], __ffs(b.nc[0]) - 1);
-  key[i] = kk;
-  rank[i] = atomicAdd(&bin_count[kk], 1);
-}
-
-__global__ void k_scatter(SystemDev s, const int *key, const int *rank, const int *bin_start,
-                          int *slot_orig, const unsigned *go, const unsigned *rb) {
-  if (!go[1]) return;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= s.natoms) return;
-  const int bi = s.atom_box[i];
-  if (!rb[bi]) return;
-  const BoxDev &b = s.box[bi];
-  int base = b.blk0 * BLOCK - bin_start[b.key0];
-  slot_orig[base + bin_start[key[i]] + rank[i]] = i;
-}
-
-// Makes the within-bin order deterministic (ascending original index).
-__global__ void k_sort_bins(SystemDev s, const int *bin_box, const int *bin_start,
-                            const int *bin_count, int nkeys, int *slot_orig, const unsigned *go) {
-  if (!go[1]) return;
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nkeys) return;
-  int cnt = bin_count[k];
-  if (cnt < 2) return;
-  const BoxDev &b = s.box[bin_box[k]];
-  int *p = slot_orig + b.blk0 * BLOCK - bin_start[b.key0] + bin_start[k];
-  for (int a = 1; a < cnt; a++) {
-    int v = p[a], j = a - 1;
-    while (j >= 0 && p[j] > v) {
-      p[j + 1] = p[j];
-      j--;
+    nb.ctl[CTL_REBUILD] = any ? 1u : 0u;
+    if (any) {
+      ++*reinterpret_cast<unsigned long long *>(nb.ctl + CTL_BUILDS);
+      // the build starts its list of pair units anew
+      nb.ctl[CTL_CLAIM] = nb.ctl[CTL_UNITS] = nb.ctl[CTL_UNITS + 1] = nb.ctl[CTL_TILES] = 0u;
     }
-    p[j + 1] = v;
+    nb.ctl[CTL_BLOCKS] = 0u;
+    nb.ctl[CTL_FORCED] = 0u;
   }
 }
 
-__global__ void k_pack(SystemDev s, NbListDev nb, int want_fp64) {
-  int sl = blockIdx.x * blockDim.x + threadIdx.x;
-  if (sl >= nb.nslot) return;
-  int o = nb.slot_orig[sl];
-  if (o < 0) {
-    nb.slot_meta[sl] = make_int4(-1, -1, 0, nb.blk_box[sl / BLOCK]);
-    nb.slot_fx[sl] = make_uint4(0, 0, 0, 0);
-    if (want_fp64) nb.slot_pq[sl] = make_double4(0, 0, 0, 0);
-    return;
-  }
-  int bi = s.atom_box[o];
-  const BoxDev &b = s.box[bi];
-  double x = s.pos[3 * o], y = s.pos[3 * o + 1], z = s.pos[3 * o + 2], q = s.charge[o];
-  if (nb.ctl[1] && nb.box_rb[bi]) {  // the box's list is rebuilt this step: new reference positions
-    nb.xref[3 * o] = x;
-    nb.xref[3 * o + 1] = y;
-    nb.xref[3 * o + 2] = z;
-  }
-  nb.slot_meta[sl] = make_int4(o, s.molecule[o], s.type[o], bi);
-  nb.slot_fx[sl] = make_uint4(frac_fixed(x, b.Lr[0]), frac_fixed(y, b.Lr[1]),
-                              frac_fixed(z, b.Lr[2]), __float_as_uint((float)q));
-  if (want_fp64) nb.slot_pq[sl] = make_double4(x, y, z, q);
-}
-
-// Bounding box of every BLOCK-slot block in fractional fixed point; a warp covers GROUPS blocks.
-__global__ void k_block_bbox(NbListDev nb) {
-  if (!nb.ctl[1]) return;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  int blk = t / BLOCK, lane = threadIdx.x & 31;
-  bool inr = blk < nb.nblk_total;
-  int sl = inr ? t : 0;
-  bool valid = inr && nb.slot_orig[sl] >= 0;
-  uint4 f = inr ? nb.slot_fx[sl] : make_uint4(0, 0, 0, 0);
-  unsigned lo[3] = {valid ? f.x : 0xffffffffu, valid ? f.y : 0xffffffffu, valid ? f.z : 0xffffffffu};
-  unsigned hi[3] = {valid ? f.x : 0u, valid ? f.y : 0u, valid ? f.z : 0u};
-#pragma unroll
-  for (int o = BLOCK / 2; o > 0; o >>= 1)
+// ---- the sort into slots, a deterministic counting sort: histogram of the atoms over the
+// Hilbert-ordered cells, exclusive scan, scatter, placing (an atom's slot is its bin's start plus
+// the number of smaller atom indices in the bin) with the slot records, then the extents of the
+// 8-slot blocks and of the runs of 32 blocks (superblocks, per box).  Each phase is a loop of
+// thread t of T over one box; bins and slots are counted from the box's first.  Loads of what
+// other threads of the same launch may have written go past L1.
+__device__ __forceinline__ void sort_bin(const SystemDev &s, const NbListDev &nb, const BoxDev &b, int t, int T) {
+  const int nc = b.nc[0], bits = __ffs(nc) - 1;
+  for (int p = t; p < b.natoms; p += T) {
+    const int i = b.atom0 + p;
+    unsigned c[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-      lo[k] = min(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
-      hi[k] = max(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
+      const unsigned f = frac_fixed(s.pos[3 * i + k], b.Lr[k]);
+      c[k] = (unsigned)(((unsigned long long)f * (unsigned)nc) >> 32);
     }
-  unsigned bal = __ballot_sync(0xffffffffu, valid);
-  int cnt = __popc(bal & (((1u << BLOCK) - 1u) << (lane & ~(BLOCK - 1))));
-  if (inr && (lane & (BLOCK - 1)) == 0 && nb.box_rb[nb.blk_box[blk]]) {
-    if (cnt == 0) lo[0] = lo[1] = lo[2] = hi[0] = hi[1] = hi[2] = 0;
-    nb.blk_lo[blk] = make_uint4(lo[0], lo[1], lo[2], (unsigned)cnt);
-    nb.blk_hi[blk] = make_uint4(hi[0], hi[1], hi[2], 0u);
-    nb.blk_c[blk] = make_uint4(lo[0] + (hi[0] - lo[0]) / 2u, lo[1] + (hi[1] - lo[1]) / 2u,
-                               lo[2] + (hi[2] - lo[2]) / 2u, (unsigned)cnt);
-    nb.blk_h[blk] = make_uint4((hi[0] - lo[0]) / 2u + 1u, (hi[1] - lo[1]) / 2u + 1u, (hi[2] - lo[2]) / 2u + 1u, 0u);
+    const int kk = (int)hilbert3(c[0], c[1], c[2], bits);
+    nb.key[i] = kk;
+    nb.rank[i] = atomicAdd(nb.bin_count + b.key0 + kk, 1);  // (the bins are zero between builds)
+  }
+}
+// by one CTA
+__device__ __forceinline__ void sort_scan(const NbListDev &nb, const BoxDev &b) {
+  const int nk = b.nc[0] * b.nc[0] * b.nc[0], T = blockDim.x;
+  const int *count = nb.bin_count + b.key0;
+  int *start = nb.bin_start + b.key0;
+  __shared__ int carry;
+  if (threadIdx.x == 0) carry = 0;
+  __syncthreads();
+  constexpr int PER = 16;  // bins of a thread per round
+  for (int k0 = 0; k0 < nk; k0 += PER * T) {
+    const int k = k0 + PER * threadIdx.x;
+    int4 v[PER / 4];
+    int sum = 0;
+#pragma unroll
+    for (int q = 0; q < PER / 4; q++) {  // nk is 1 or a multiple of 8; regions start at multiples of 4
+      v[q] = make_int4(0, 0, 0, 0);
+      if (k + 4 * q < nk) v[q] = __ldcg(reinterpret_cast<const int4 *>(count + k + 4 * q));
+      sum += v[q].x + v[q].y + v[q].z + v[q].w;
+    }
+    int tot;
+    int ex = carry + block_exclusive_scan(sum, &tot);
+#pragma unroll
+    for (int q = 0; q < PER / 4; q++) {
+      if (k + 4 * q < nk)
+        *reinterpret_cast<int4 *>(start + k + 4 * q) =
+            make_int4(ex, ex + v[q].x, ex + v[q].x + v[q].y, ex + v[q].x + v[q].y + v[q].z);
+      ex += v[q].x + v[q].y + v[q].z + v[q].w;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) carry += tot;
+    __syncthreads();
+  }
+}
+__device__ __forceinline__ void sort_scatter(const NbListDev &nb, const BoxDev &b, int t, int T) {
+  const int *start = nb.bin_start + b.key0;
+  int *raw = nb.slot_raw + b.blk0 * BLOCK;
+  for (int p = t; p < b.natoms; p += T) {
+    const int i = b.atom0 + p;
+    raw[__ldcg(start + nb.key[i]) + nb.rank[i]] = i;
+  }
+}
+__device__ __forceinline__ void sort_place(const SystemDev &s, const NbListDev &nb, const BoxDev &b, int bi, int t, int T) {
+  const int *count = nb.bin_count + b.key0, *start = nb.bin_start + b.key0;
+  const int *raw = nb.slot_raw + b.blk0 * BLOCK;
+  for (int p = t; p < b.nblk * BLOCK; p += T) {
+    if (p >= b.natoms) {  // padding of the last block
+      const int sl = b.blk0 * BLOCK + p;
+      nb.slot_orig[sl] = -1;
+      nb.slot_meta[sl] = make_int4(-1, -1, 0, bi);
+      nb.slot_fx[sl] = make_uint4(0, 0, 0, 0);
+      if (nb.want_fp64) nb.slot_pq[sl] = make_double4(0, 0, 0, 0);
+      continue;
+    }
+    const int i = __ldcg(raw + p);
+    const int k = __ldcg(nb.key + i);
+    const double x = s.pos[3 * i], y = s.pos[3 * i + 1], z = s.pos[3 * i + 2], q = s.charge[i];
+    const int mol = s.molecule[i], type = s.type[i];
+    const int s0 = __ldcg(start + k), s1 = s0 + __ldcg(count + k);
+    int below = 0;
+    for (int r = s0; r < s1; r++) below += __ldcg(raw + r) < i;
+    const int sl = b.blk0 * BLOCK + s0 + below;
+    nb.slot_of[i] = sl;
+    nb.slot_orig[sl] = i;
+    nb.slot_meta[sl] = make_int4(i, mol, type, bi);
+    nb.slot_fx[sl] = make_uint4(frac_fixed(x, b.Lr[0]), frac_fixed(y, b.Lr[1]), frac_fixed(z, b.Lr[2]),
+                                __float_as_uint((float)q));
+    if (nb.want_fp64) nb.slot_pq[sl] = make_double4(x, y, z, q);
+    nb.xref[3 * i] = x;  // the box's new reference positions
+    nb.xref[3 * i + 1] = y;
+    nb.xref[3 * i + 2] = z;
+  }
+}
+// extents in fractional fixed point, a warp per superblock and GROUPS blocks at a time; also
+// clears the bins for the next build
+__device__ __forceinline__ void sort_extents(const NbListDev &nb, const BoxDev &b, int t, int T) {
+  const int nk = b.nc[0] * b.nc[0] * b.nc[0];
+  for (int k = t; k < nk; k += T) nb.bin_count[b.key0 + k] = 0;
+  const int lane = threadIdx.x & 31, li = lane & (BLOCK - 1), g = lane / BLOCK;
+  for (int S = t >> 5; S * 32 < b.nblk; S += T / 32) {
+    unsigned slo[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, shi[3] = {0u, 0u, 0u};
+    int scnt = 0;
+#pragma unroll 2
+    for (int j0 = S * 32; j0 < min(b.nblk, S * 32 + 32); j0 += GROUPS) {
+      const int j = j0 + g;
+      const bool inr = j < b.nblk;
+      const int blk = b.blk0 + j;
+      const bool valid = inr && j * BLOCK + li < b.natoms;
+      uint4 f = make_uint4(0, 0, 0, 0);
+      if (valid) f = __ldcg(nb.slot_fx + (long long)blk * BLOCK + li);
+      unsigned lo[3] = {valid ? f.x : 0xffffffffu, valid ? f.y : 0xffffffffu, valid ? f.z : 0xffffffffu};
+      unsigned hi[3] = {f.x, f.y, f.z};
+#pragma unroll
+      for (int o = BLOCK / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+          lo[k] = min(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
+          hi[k] = max(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
+        }
+      const unsigned bal = __ballot_sync(0xffffffffu, valid);
+      const int cnt = __popc(bal & (((1u << BLOCK) - 1u) << (lane & ~(BLOCK - 1))));
+      if (inr && li == 0) {  // (a box's blocks all hold at least one atom)
+        nb.blk_lo[blk] = make_uint4(lo[0], lo[1], lo[2], (unsigned)cnt);
+        nb.blk_hi[blk] = make_uint4(hi[0], hi[1], hi[2], 0u);
+        nb.blk_c[blk] = make_uint4(lo[0] + (hi[0] - lo[0]) / 2u, lo[1] + (hi[1] - lo[1]) / 2u,
+                                   lo[2] + (hi[2] - lo[2]) / 2u, (unsigned)cnt);
+        nb.blk_h[blk] = make_uint4((hi[0] - lo[0]) / 2u + 1u, (hi[1] - lo[1]) / 2u + 1u, (hi[2] - lo[2]) / 2u + 1u, 0u);
+      }
+      if (inr) {
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+          slo[k] = min(slo[k], lo[k]);
+          shi[k] = max(shi[k], hi[k]);
+        }
+        scnt += cnt;
+      }
+    }
+#pragma unroll
+    for (int o = 16; o >= BLOCK; o >>= 1) {
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        slo[k] = min(slo[k], __shfl_xor_sync(0xffffffffu, slo[k], o));
+        shi[k] = max(shi[k], __shfl_xor_sync(0xffffffffu, shi[k], o));
+      }
+      scnt += __shfl_xor_sync(0xffffffffu, scnt, o);
+    }
+    if (lane == 0) {
+      nb.sblk_c[b.sblk0 + S] = make_uint4(slo[0] + (shi[0] - slo[0]) / 2u, slo[1] + (shi[1] - slo[1]) / 2u,
+                                          slo[2] + (shi[2] - slo[2]) / 2u, (unsigned)scnt);
+      nb.sblk_h[b.sblk0 + S] = make_uint4((shi[0] - slo[0]) / 2u + 1u, (shi[1] - slo[1]) / 2u + 1u,
+                                          (shi[2] - slo[2]) / 2u + 1u, 0u);
+    }
   }
 }
 
-// Union extents of each run of 32 consecutive blocks (one warp per superblock).  Blocks of
-// different boxes may share a superblock: the union then only enlarges, which never culls a
-// true candidate.
-__global__ void k_superblock_bbox(NbListDev nb) {
-  if (!nb.ctl[1]) return;
-  const int S = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (S >= nb.nsblk) return;
-  const int J = S * 32 + lane;
-  uint4 lo = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0u), hi = make_uint4(0u, 0u, 0u, 0u);
-  if (J < nb.nblk_total) {
-    const uint4 l = nb.blk_lo[J];
-    if (l.w > 0) {
-      lo = l;
-      hi = nb.blk_hi[J];
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    lo.x = min(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, o));
-    lo.y = min(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, o));
-    lo.z = min(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, o));
-    lo.w += __shfl_xor_sync(0xffffffffu, lo.w, o);
-    hi.x = max(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, o));
-    hi.y = max(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, o));
-    hi.z = max(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, o));
-  }
-  if (lane == 0) {
-    if (lo.w == 0) lo.x = lo.y = lo.z = hi.x = hi.y = hi.z = 0;
-    nb.sblk_lo[S] = lo;
-    nb.sblk_hi[S] = hi;
-    nb.sblk_c[S] = make_uint4(lo.x + (hi.x - lo.x) / 2u, lo.y + (hi.y - lo.y) / 2u, lo.z + (hi.z - lo.z) / 2u, lo.w);
-    nb.sblk_h[S] = make_uint4((hi.x - lo.x) / 2u + 1u, (hi.y - lo.y) / 2u + 1u, (hi.z - lo.z) / 2u + 1u, 0u);
-  }
+// Every phase in one launch, a CTA per box: small boxes, and systems of many.
+constexpr int SORT_THREADS = 512;
+__global__ void __launch_bounds__(SORT_THREADS) k_sort_box(SystemDev s, NbListDev nb) {
+  if (!nb.ctl[CTL_REBUILD]) return;
+  const int bi = blockIdx.x, t = threadIdx.x;
+  if (!nb.box_rb[bi]) return;  // the box keeps its slots
+  const BoxDev &b = s.box[bi];
+  sort_bin(s, nb, b, t, SORT_THREADS);
+  __syncthreads();
+  sort_scan(nb, b);
+  __syncthreads();
+  sort_scatter(nb, b, t, SORT_THREADS);
+  __syncthreads();
+  sort_place(s, nb, b, bi, t, SORT_THREADS);
+  __syncthreads();
+  sort_extents(nb, b, t, SORT_THREADS);
+}
+
+// One launch per phase over the whole chip (blockIdx.y: box): large boxes.  The last CTA of a box
+// to finish its histogram also scans the box's bins.
+__global__ void __launch_bounds__(SORT_THREADS) k_sort_bin(SystemDev s, NbListDev nb) {
+  if (!nb.ctl[CTL_REBUILD] || !nb.box_rb[blockIdx.y]) return;
+  const BoxDev &b = s.box[blockIdx.y];
+  sort_bin(s, nb, b, blockIdx.x * SORT_THREADS + threadIdx.x, gridDim.x * SORT_THREADS);
+  __threadfence();
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(nb.box_done + blockIdx.y, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  if (threadIdx.x == 0) nb.box_done[blockIdx.y] = 0u;
+  sort_scan(nb, b);
+}
+__global__ void __launch_bounds__(SORT_THREADS) k_sort_scatter(SystemDev s, NbListDev nb) {
+  if (!nb.ctl[CTL_REBUILD] || !nb.box_rb[blockIdx.y]) return;
+  sort_scatter(nb, s.box[blockIdx.y], blockIdx.x * SORT_THREADS + threadIdx.x, gridDim.x * SORT_THREADS);
+}
+__global__ void __launch_bounds__(SORT_THREADS) k_sort_place(SystemDev s, NbListDev nb) {
+  if (!nb.ctl[CTL_REBUILD] || !nb.box_rb[blockIdx.y]) return;
+  sort_place(s, nb, s.box[blockIdx.y], blockIdx.y, blockIdx.x * SORT_THREADS + threadIdx.x, gridDim.x * SORT_THREADS);
+}
+__global__ void __launch_bounds__(SORT_THREADS) k_sort_extents(SystemDev s, NbListDev nb) {
+  if (!nb.ctl[CTL_REBUILD] || !nb.box_rb[blockIdx.y]) return;
+  sort_extents(nb, s.box[blockIdx.y], blockIdx.x * SORT_THREADS + threadIdx.x, gridDim.x * SORT_THREADS);
 }
 
 // Gap^2 (A^2) between the box (c1, h1 half extents in A) and the box (c2, h2 fixed-point half
@@ -413,25 +441,45 @@ __device__ __forceinline__ float gap2f(const float sL[3], const unsigned c1[3], 
 constexpr int BL_THREADS = BL_BLOCK_THREADS;
 constexpr int BL_CAP = 128;  // candidate blocks buffered per warp before their atoms are tested
 
-// One warp per block I: its own slots, then the candidate blocks J > I of the same box by
+// Appends I's list to the pair kernel's work as units of at most nb.unit_tiles tiles (about equal
+// parts of the list, starting at multiples of CLOSE_TILES tiles); a block of a box that keeps its
+// list appends the units it has.  The units of boxes that need lattice images grow from the end
+// of the array.  Their order varies from build to build and changes no result: the pair kernel
+// closes its floating-point sums every CLOSE_TILES tiles of a list.
+__device__ __forceinline__ void append_units(NbListDev &nb, int I, int tiles, bool multi, int lane) {
+  const int nc = (tiles + CLOSE_TILES - 1) / CLOSE_TILES;
+  const int per = nb.unit_tiles / CLOSE_TILES, nu = (nc + per - 1) / per;
+  if (nu == 0) return;
+  int at = 0;
+  if (lane == 0) {
+    at = (int)atomicAdd(nb.ctl + CTL_UNITS + (multi ? 1 : 0), (unsigned)nu);
+    atomicAdd(nb.ctl + CTL_TILES, (unsigned)tiles);
+  }
+  at = __shfl_sync(0xffffffffu, at, 0);
+  for (int p = lane; p < nu; p += 32) {
+    const int k0 = (int)((long long)nc * p / nu) * CLOSE_TILES;
+    const int k1 = min(tiles, (int)((long long)nc * (p + 1) / nu) * CLOSE_TILES);
+    const int u = at + p;  // (within the array: it is sized for full lists)
+    nb.units[multi ? nb.unit_cap - 1 - u : u] = make_int4(I, k0, k1 - k0, nb.jcap_off[I] + k0 * JCHUNK);
+  }
+}
+
+// One warp per block I (claimed from a counter, in ascending order: the early blocks' lists are
+// the longest): its own slots, then the candidate blocks J > I of the same box by
 // bounding-box gap (superblocks of 32 blocks first), compacted into a shared-memory list, then
 // the atoms of GROUPS listed blocks per pass within the list cutoff of I's box, compacted into
 // I's j-list (tiles of 32 entries).  The loads of the next pass are issued before the current
 // pass is tested.
-__global__ void __launch_bounds__(BL_THREADS, BL_MINB) k_build_lists(SystemDev s, NbListDev nb, double rlist2) {
-  __shared__ int cand_all[BL_THREADS / 32][BL_CAP];
-  if (!nb.ctl[1]) return;
-  const int I = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (I >= nb.nblk_total) return;
-  int *cl = cand_all[threadIdx.x >> 5];
+// One block's list; cl [BL_CAP] and ipos [BLOCK] are the warp's shared memory.
+__device__ __forceinline__ void build_block(const SystemDev &s, NbListDev &nb, double rlist2, int I, int *cl, float4 *ipos) {
+  const int lane = threadIdx.x & 31;
   const int bi = nb.blk_box[I];
-  if (!nb.box_rb[bi]) return;  // the box keeps its list
   const BoxDev &b = s.box[bi];
-  const uint4 cIv = nb.blk_c[I], hIv = nb.blk_h[I];
-  if (cIv.w == 0) {
-    if (lane == 0) nb.jcount[I] = 0;
+  if (!nb.box_rb[bi]) {  // the box keeps its list
+    append_units(nb, I, nb.jcount[I], b.multi_image != 0, lane);
     return;
   }
+  const uint4 cIv = nb.blk_c[I], hIv = nb.blk_h[I];
   const float sL[3] = {(float)(b.L[0] * (1.0 / 4294967296.0)), (float)(b.L[1] * (1.0 / 4294967296.0)),
                        (float)(b.L[2] * (1.0 / 4294967296.0))};
   const unsigned cI[3] = {cIv.x, cIv.y, cIv.z};
@@ -450,8 +498,6 @@ __global__ void __launch_bounds__(BL_THREADS, BL_MINB) k_build_lists(SystemDev s
   // pair (the bounding-box gap alone would list about a third more atoms)
   // (in shared memory, FP32 relative to the block's first atom; padding atoms far away)
   // stored as pairs of atoms {t, t + BLOCK/2}: x x' y y' | z z' (two-wide FP32 tests)
-  __shared__ float4 ipos_all[BL_THREADS / 32][BLOCK];
-  float4 *ipos = ipos_all[threadIdx.x >> 5];
   int imol[BLOCK];
   unsigned r0[3];
   {
@@ -561,18 +607,18 @@ __global__ void __launch_bounds__(BL_THREADS, BL_MINB) k_build_lists(SystemDev s
     __syncwarp();
   };
 
-  // superblocks (runs of 32 blocks), 32 per ballot; then the 32 blocks of each candidate one
-  const int send = (jend + 31) / 32;
-  for (int S0 = (I + 1) / 32; S0 < send && !overflow; S0 += 32) {
+  // superblocks (the box's runs of 32 blocks), 32 per ballot; then the 32 blocks of each candidate
+  const int send = (b.nblk + 31) / 32;
+  for (int S0 = (I + 1 - b.blk0) / 32; S0 < send && !overflow; S0 += 32) {
     const int S = S0 + lane;
     bool scand = false;
     if (S < send) {
-      const uint4 cS = nb.sblk_c[S];
-      if (cS.w > 0) scand = multi || gap2f(sL, cI, hI, cS, nb.sblk_h[S]) <= rl2;
+      const uint4 cS = nb.sblk_c[b.sblk0 + S];
+      if (cS.w > 0) scand = multi || gap2f(sL, cI, hI, cS, nb.sblk_h[b.sblk0 + S]) <= rl2;
     }
     unsigned sm = __ballot_sync(0xffffffffu, scand);
     while (sm && !overflow) {
-      const int J = (S0 + __ffs(sm) - 1) * 32 + lane;
+      const int J = b.blk0 + (S0 + __ffs(sm) - 1) * 32 + lane;
       sm &= sm - 1;
       bool cand = false;
       if (J > I && J < jend) {
@@ -589,103 +635,66 @@ __global__ void __launch_bounds__(BL_THREADS, BL_MINB) k_build_lists(SystemDev s
   const int padded = (count + 31) & ~31;
   if (!overflow)
     for (int k = count + lane; k < padded; k += 32) out[k] = -1;
+  const int tiles = overflow ? 0 : padded / 32;
   if (lane == 0) {
     if (overflow) atomicExch(&nb.status[0], 1);
-    nb.jcount[I] = overflow ? 0 : padded / 32;
+    nb.jcount[I] = tiles;
+  }
+  append_units(nb, I, tiles, multi, lane);
+  __syncwarp();  // the shared memory is written again for the next block
+}
+
+__global__ void __launch_bounds__(BL_THREADS, BL_MINB) k_build_lists(SystemDev s, NbListDev nb, double rlist2) {
+  __shared__ int cand_all[BL_THREADS / 32][BL_CAP];
+  __shared__ float4 ipos_all[BL_THREADS / 32][BLOCK];
+  if (!nb.ctl[CTL_REBUILD]) return;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (;;) {
+    int I = 0;
+    if (lane == 0) I = (int)atomicAdd(nb.ctl + CTL_CLAIM, 1u);
+    I = __shfl_sync(0xffffffffu, I, 0);
+    if (I >= nb.nblk_total) return;
+    build_block(s, nb, rlist2, I, cand_all[w], ipos_all[w]);
   }
 }
 
-// Padding that starts every box's tiles at a multiple of TILE_CHUNK (one block of threads, the
-// boxes in the order of their blocks): the pair kernel's warp assignments then never mix boxes,
-// and a box's partial sums are grouped as when it is alone.
-__global__ void k_box_pad(SystemDev s, NbListDev nb) {
-  if (!nb.ctl[1]) return;
-  const int per = (nb.nbox + (int)blockDim.x - 1) / (int)blockDim.x;
-  const int k0 = min(nb.nbox, (int)threadIdx.x * per), k1 = min(nb.nbox, k0 + per);
-  auto pad = [&](int b) {
-    const BoxDev &bx = s.box[b];
-    const int tot = nb.tile_off[bx.blk0 + bx.nblk] - nb.tile_off[bx.blk0];
-    return (TILE_CHUNK - tot % TILE_CHUNK) % TILE_CHUNK;
-  };
-  int acc = 0;
-  for (int k = k0; k < k1; k++) acc += pad(nb.box_order[k]);
-  int tot;
-  int ex = block_exclusive_scan(acc, &tot);
-  for (int k = k0; k < k1; k++) {
-    const int b = nb.box_order[k];
-    nb.box_shift[b] = ex;
-    ex += pad(b);
-  }
-  if (threadIdx.x == 0) nb.tile_start[nb.nblk_total] = nb.tile_off[nb.nblk_total] + tot;
-}
-
-// One warp per block: its first tile and its tiles' (block, index) entries, written by
-// consecutive lanes; a box's last block also writes the box's empty padding tiles.
-__global__ void k_tile_map(SystemDev s, NbListDev nb) {
-  if (!nb.ctl[1]) return;
-  const int I = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (I >= nb.nblk_total) return;
-  const int b = nb.blk_box[I];
-  const BoxDev &bx = s.box[b];
-  const int shift = nb.box_shift[b];
-  const int off = nb.tile_off[I] + shift, cnt = nb.jcount[I];
-  int end = off + cnt;
-  if (I == bx.blk0 + bx.nblk - 1) {
-    const int start = nb.tile_off[bx.blk0] + shift;
-    end = start + (end - start + TILE_CHUNK - 1) / TILE_CHUNK * TILE_CHUNK;
-  }
-  if (lane == 0) nb.tile_start[I] = off;
-  if (end > nb.tile_cap) {
-    if (lane == 0) atomicExch(&nb.status[1], 1);
-    return;
-  }
-  for (int k = lane; k < end - off; k += 32) {
-    nb.tile_blk[off + k] = k < cnt ? I : -1;
-    nb.tile_k[off + k] = k;
-  }
-}
-
-int scan_exclusive(const int *in, int *out, int n, int *tmp, cudaStream_t st, const unsigned *go) {
-  int nchunk = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
-  if (nchunk < 1) nchunk = 1;
-  k_scan_reduce<<<nchunk, 1024, 0, st>>>(in, n, tmp, go);
-  k_scan_chunks<<<1, 1024, 0, st>>>(tmp, nchunk, go);
-  k_scan_apply<<<nchunk, 1024, 0, st>>>(in, n, tmp, out, go);
-  return 0;
+// One CTA per box up to SORT_SMALL atoms, and up to SORT_MANY when the boxes alone fill the chip.
+constexpr int SORT_SMALL = 3072, SORT_MANY = 32768;
+bool sort_by_box(const SystemDev &s, const NbListDev &nb) {
+  return nb.max_box_atoms <= SORT_SMALL || (s.nbox >= nb.n_sm / 2 && nb.max_box_atoms <= SORT_MANY);
 }
 
 }  // namespace
 
-// First half of a build: displacement check, sort into slots and the slot records of this step's
-// positions (the PME kernels need no more than these).
+// First half of a build: displacement check and this step's slot records, then the sort into
+// slots of the boxes that rebuild (the PME kernels need no more than these).  Every kernel after
+// the displacement check exits at once unless ctl[CTL_REBUILD] asks for a rebuild.
 int nblist_sort(const SystemDev &s, NbListDev &nb, cudaStream_t st) {
   const int T = 256;
   int na = s.natoms;
   if (na <= 0) return 0;
-  // every kernel after the displacement check exits at once unless ctl[1] asks for a rebuild
-  // (inside a CUDA graph such a launch costs about a microsecond)
-  k_disp_check<<<(na + T - 1) / T, T, 0, st>>>(s, nb);
-  k_zero_bins<<<(nb.nkeys + T) / T, T, 0, st>>>(nb.bin_count, nb.nkeys, nb.ctl);
-  k_bin<<<(na + T - 1) / T, T, 0, st>>>(s, nb.key, nb.rank, nb.bin_count, nb.ctl, nb.box_rb);
-  scan_exclusive(nb.bin_count, nb.bin_start, nb.nkeys, nb.scan_tmp, st, nb.ctl);
-  k_scatter<<<(na + T - 1) / T, T, 0, st>>>(s, nb.key, nb.rank, nb.bin_start, nb.slot_orig, nb.ctl, nb.box_rb);
-  k_sort_bins<<<(nb.nkeys + T - 1) / T, T, 0, st>>>(s, nb.bin_box, nb.bin_start, nb.bin_count,
-                                                   nb.nkeys, nb.slot_orig, nb.ctl);
-  k_pack<<<(nb.nslot + T - 1) / T, T, 0, st>>>(s, nb, nb.want_fp64);
+  k_update<<<(na + T - 1) / T, T, 0, st>>>(s, nb);
+  if (sort_by_box(s, nb)) {
+    k_sort_box<<<s.nbox, SORT_THREADS, 0, st>>>(s, nb);
+    return 0;
+  }
+  const dim3 grid((nb.max_box_atoms + SORT_THREADS - 1) / SORT_THREADS, s.nbox);
+  k_sort_bin<<<grid, SORT_THREADS, 0, st>>>(s, nb);
+  k_sort_scatter<<<grid, SORT_THREADS, 0, st>>>(s, nb);
+  k_sort_place<<<grid, SORT_THREADS, 0, st>>>(s, nb);
   return 0;
 }
 
-// Second half: cluster boxes, the cluster j-lists and the tile map of the pair kernel.
+// Second half: the extents of the blocks (large boxes), the cluster j-lists and the units of the pair kernel.
 int nblist_lists(const SystemDev &s, NbListDev &nb, double list_cutoff, cudaStream_t st) {
-  const int T = 256;
   if (s.natoms <= 0) return 0;
-  const int wthreads = nb.nblk_total * 32;
-  k_block_bbox<<<(nb.nslot + T - 1) / T, T, 0, st>>>(nb);
-  k_superblock_bbox<<<(nb.nsblk * 32 + T - 1) / T, T, 0, st>>>(nb);
-  k_build_lists<<<(wthreads + BL_THREADS - 1) / BL_THREADS, BL_THREADS, 0, st>>>(s, nb, list_cutoff * list_cutoff);
-  scan_exclusive(nb.jcount, nb.tile_off, nb.nblk_total, nb.scan_tmp, st, nb.ctl);
-  k_box_pad<<<1, 1024, 0, st>>>(s, nb);
-  k_tile_map<<<(wthreads + T - 1) / T, T, 0, st>>>(s, nb);
+  if (!sort_by_box(s, nb)) {
+    const dim3 grid((nb.max_box_atoms + SORT_THREADS - 1) / SORT_THREADS, s.nbox);
+    k_sort_extents<<<grid, SORT_THREADS, 0, st>>>(s, nb);
+  }
+  // as many blocks as fit at once (blocks are claimed), so that the exit without a rebuild is short
+  const int warps = BL_THREADS / 32, need = (nb.nblk_total + warps - 1) / warps;
+  k_build_lists<<<need < nb.n_sm * BL_MINB ? need : nb.n_sm * BL_MINB, BL_THREADS, 0, st>>>(s, nb, list_cutoff * list_cutoff);
   return 0;
 }
 

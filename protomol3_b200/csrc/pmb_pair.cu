@@ -47,7 +47,6 @@ namespace {
 #endif
 constexpr int PAIR_THREADS = PAIR_BLOCK_THREADS;
 constexpr int PAIR_WARPS = PAIR_THREADS / 32;
-constexpr int CHUNK = TILE_CHUNK;  // consecutive tiles per warp assignment
 
 // switch / potential selectors (template parameters)
 constexpr int SWR = -1;   // read the switching function kind at run time
@@ -296,10 +295,6 @@ __device__ __forceinline__ float le_mask(float a, float b) {
 
 // Asynchronous global -> shared copies (cp.async, L1-allocating) used to prefetch the next tile's
 // j-list entries and slot records while the current tile computes.
-__device__ __forceinline__ void cp_async4(void *dst, const void *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
-}
 __device__ __forceinline__ void cp_async16(void *dst, const void *src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
                : "memory");
@@ -433,11 +428,11 @@ struct WarpCtx {
   int pad_;
 };
 
-// Bytes of one warp's prefetch region: the j-list entries of a chunk of tiles, and two buffers of
+// Bytes of one warp's prefetch region: the j-list entries of a unit, and two buffers of
 // slot records (position, metadata) and raw j-list words for the tile in flight and the next.
 template <bool MIXED>
 constexpr size_t warp_pref_bytes() {
-  return 2 * 32 * (MIXED ? sizeof(uint4) : sizeof(double4)) + 2 * 32 * sizeof(int4) + CHUNK * 32 * sizeof(int) +
+  return 2 * 32 * (MIXED ? sizeof(uint4) : sizeof(double4)) + 2 * 32 * sizeof(int4) + UNIT_TILES * 32 * sizeof(int) +
          2 * 32 * sizeof(int);
 }
 
@@ -445,7 +440,7 @@ template <bool MIXED, int LSW, int CM, int CSW, bool VIR, bool MULTI>
 __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !VIR && !MULTI) ? PAIR_MINB : (!MIXED && !VIR && !MULTI) ? PAIR_MINB_FP64 : 2)
     k_pair(SystemDev s, NbListDev nb, PairParams p,
            ParamsT<typename std::conditional<MIXED, float, double>::type> pt, const double *ljd,
-           const double *lat, int blk_lo, int blk_hi, int wslot) {
+           const double *lat, int unit_kinds, int wslot) {
   using T = typename std::conditional<MIXED, float, double>::type;
   using T2 = typename std::conditional<MIXED, float2, double2>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -471,21 +466,21 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !VIR && !MULTI) ? PAIR
   float4 *qb = qa + FAST_ENTRIES;
   int2 *qt = reinterpret_cast<int2 *>(reinterpret_cast<float4 *>(wstage) + 2 * FAST_ENTRIES) + qe;
   const int gwarp = blockIdx.x * PAIR_WARPS + wib, nwarps = gridDim.x * PAIR_WARPS;
-  // this launch's tiles: those of blocks [blk_lo, blk_hi)
-  int t_lo = nb.tile_start[blk_lo], t_hi = nb.tile_start[blk_hi];
-  if (t_hi > nb.tile_cap) t_hi = nb.tile_cap;
-  if (t_lo > t_hi) t_lo = t_hi;
+  // this launch's units: those of boxes without lattice images come first, then those with
+  const int n_front = min((int)nb.ctl[CTL_UNITS], nb.unit_cap), n_back = min((int)nb.ctl[CTL_UNITS + 1], nb.unit_cap - n_front);
+  const int u_lo = unit_kinds & 1 ? 0 : n_front, u_hi = unit_kinds & 2 ? n_front + n_back : n_front;
 
-  int curI = -1, curBox = -1;
-  // energies (and virials) per lane: summed in the arithmetic type over a chunk of tiles, then
+  int curBox = -1;
+  // energies (and virials) per lane: summed in the arithmetic type over CLOSE_TILES tiles, then
   // added in fixed point to this lane's slots in shared memory; summed over the warp and added to
   // the box accumulators when the box changes
   T el_acc = T(0), ec_acc = T(0), v_acc[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
   constexpr int NE = VIR ? 8 : 2;
+  // [NE + 3][32]: the energies and virial, then the i-forces of the current cluster
   long long *wsum = reinterpret_cast<long long *>(
-      smem_raw + ljbytes + PAIR_WARPS * (warp_stage_bytes<MIXED>() + sizeof(WarpCtx))) + wib * NE * 32;
+      smem_raw + ljbytes + PAIR_WARPS * (warp_stage_bytes<MIXED>() + sizeof(WarpCtx))) + wib * (NE + 3) * 32;
 #pragma unroll
-  for (int c = 0; c < NE; c++) wsum[c * 32 + lane] = 0;
+  for (int c = 0; c < NE + 3; c++) wsum[c * 32 + lane] = 0;
   int4 im = make_int4(-1, -1, 0, 0);   // orig, mol, type, box of this lane's i-atom
   T xi = 0, yi = 0, zi = 0, qi = 0;     // i-atom position (relative for the mixed path)
   const BoxDev *bx = nullptr;
@@ -499,8 +494,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !VIR && !MULTI) ? PAIR
   // eight scattered atoms (pair_fold moves them to original order afterwards)
   const long long nsl = nb.nslot;
   // i-forces of the current cluster per lane: the scalar path's in fi_acc, the packed path's
-  // (+f, the i-force is -fi) in a2p.fi; combined over the lane groups and added by slot when the
-  // cluster changes.  The packed path's energies and virial also accumulate in a2p over a chunk.
+  // (+f, the i-force is -fi) in a2p.fi; the packed path's energies and virial are in a2p too.
   T fi_acc[3] = {T(0), T(0), T(0)};
   Acc2 a2p;
 #pragma unroll
@@ -508,32 +502,36 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !VIR && !MULTI) ? PAIR
   a2p.elj = a2p.ec = sp2(0.f);
 #pragma unroll
   for (int c = 0; c < 6; c++) a2p.vir[c] = sp2(0.f);
-  auto flush_fi = [&]() {  // warp-uniform
+  // (FP64: one rounding for the warp, below what the 32 of its lanes would add up to)
+  auto add_fixed = [&](int c, T v) {
+    if constexpr (MIXED) {
+      wsum[c * 32 + lane] += f2fix(v, (T)ENERGY_SCALE);
+    } else {
+      const double w = warp_sum(v);
+      if (lane == 0) wsum[c * 32] += f2fix(w, ENERGY_SCALE);
+    }
+  };
+  // closes the floating-point sums of this lane: every CLOSE_TILES tiles of a list (counted from
+  // the list's start) they are added in fixed point to this lane's words in shared memory, so the
+  // sums do not depend on how a list is cut into units
+  auto close_sums = [&]() {
     T f[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       f[c] = fi_acc[c];
       if constexpr (MIXED) f[c] -= a2p.fi[c].x + a2p.fi[c].y;
-    }
-#pragma unroll
-    for (int o = BLOCK; o < 32; o <<= 1)
-#pragma unroll
-      for (int c = 0; c < 3; c++) f[c] += __shfl_xor_sync(0xffffffffu, f[c], o);
-    if (curI >= 0 && gb == 0 && im.x >= 0) {
-      long long *fs = nb.fslot + (long long)curI * BLOCK + li;
-      const long long v0 = f2fix(f[0], (T)FORCE_SCALE), v1 = f2fix(f[1], (T)FORCE_SCALE),
-                      v2 = f2fix(f[2], (T)FORCE_SCALE);
-      if (v0) red_add(fs, v0);
-      if (v1) red_add(fs + nsl, v1);
-      if (v2) red_add(fs + 2 * nsl, v2);
-    }
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
       fi_acc[c] = T(0);
       a2p.fi[c] = sp2(0.f);
     }
-  };
-  auto spill_e = [&]() {
+    if constexpr (!MIXED) {  // one rounding for the cluster's lane groups instead of four
+#pragma unroll
+      for (int o = BLOCK; o < 32; o <<= 1)
+#pragma unroll
+        for (int c = 0; c < 3; c++) f[c] += __shfl_xor_sync(0xffffffffu, f[c], o);
+    }
+    if (MIXED || gb == 0)
+#pragma unroll
+      for (int c = 0; c < 3; c++) wsum[(NE + c) * 32 + lane] += f2fix(f[c], (T)FORCE_SCALE);
     if constexpr (MIXED) {
       el_acc += a2p.elj.x + a2p.elj.y;
       ec_acc += a2p.ec.x + a2p.ec.y;
@@ -546,19 +544,31 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !VIR && !MULTI) ? PAIR
         }
       }
     }
-    wsum[lane] += f2fix(el_acc, (T)ENERGY_SCALE);
-    wsum[32 + lane] += f2fix(ec_acc, (T)ENERGY_SCALE);
+    add_fixed(0, el_acc);
+    add_fixed(1, ec_acc);
     el_acc = ec_acc = T(0);
     if constexpr (VIR) {
 #pragma unroll
       for (int c = 0; c < 6; c++) {
-        wsum[(2 + c) * 32 + lane] += f2fix(v_acc[c], (T)ENERGY_SCALE);
+        add_fixed(2 + c, v_acc[c]);
         v_acc[c] = T(0);
       }
     }
   };
+  // adds the cluster's i-forces by slot: lane 8 c + li takes component c of atom li
+  auto flush_fi = [&](int I) {  // warp-uniform
+    __syncwarp();
+    static_assert(BLOCK == 8, "24 lanes for the components of 8 atoms");
+    if (lane < 3 * BLOCK) {
+      const long long *w = wsum + (NE + gb / BLOCK) * 32 + li;
+      const long long v = w[0] + w[BLOCK] + w[2 * BLOCK] + w[3 * BLOCK];
+      if (v) red_add(nb.fslot + (gb / BLOCK) * nsl + (long long)I * BLOCK + li, v);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < 3; c++) wsum[(NE + c) * 32 + lane] = 0;
+  };
   auto flush_e = [&]() {  // warp-uniform
-    spill_e();
     const long long el = warp_sum_ll(wsum[lane]), ec = warp_sum_ll(wsum[32 + lane]);
     long long vs[6] = {0, 0, 0, 0, 0, 0};
     if constexpr (VIR)
@@ -582,22 +592,19 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !VIR && !MULTI) ? PAIR
   // stage one slot (or padding) as this lane's j-atom
   // (padding slots of a box's last cluster, orig < 0, become sentinels as well: they carry no
   // charge but an LJ type, and must never meet a real atom)
-  // prefetch region: slot records [2][32], metadata [2][32], a chunk's j-list words [CHUNK][32],
+  // prefetch region: slot records [2][32], metadata [2][32], a unit's j-list words [UNIT_TILES][32],
   // raw j-list words of the buffered tiles [2][32]
   using RawP = typename std::conditional<MIXED, uint4, double4>::type;
   unsigned char *wpref = smem_raw + ljbytes +
-                         PAIR_WARPS * (warp_stage_bytes<MIXED>() + sizeof(WarpCtx) + NE * 32 * sizeof(long long)) +
+                         PAIR_WARPS * (warp_stage_bytes<MIXED>() + sizeof(WarpCtx) + (NE + 3) * 32 * sizeof(long long)) +
                          wib * warp_pref_bytes<MIXED>();
   RawP *rawP = reinterpret_cast<RawP *>(wpref);
   int4 *rawM = reinterpret_cast<int4 *>(rawP + 64);
   int *jbuf = reinterpret_cast<int *>(rawM + 64);
-  int *rawJ = jbuf + CHUNK * 32;
-  int tI = -1, tk = -1, tjb = 0;  // lane t < CHUNK: block, index and j-list offset of chunk tile t
-  // issues the copies of tile t's slot records into buffer b (warp-uniform; one commit group)
+  int *rawJ = jbuf + UNIT_TILES * 32;
+  // issues the copies of the slot records of the unit's tile t into buffer b (one commit group)
   auto prefetch = [&](int t, int b) {
-    const int It = __shfl_sync(0xffffffffu, tI, t), kt = __shfl_sync(0xffffffffu, tk, t);
-    int jr = -1;
-    if (It >= 0) jr = jbuf[t * 32 + lane];
+    const int jr = jbuf[t * 32 + lane];
     rawJ[b * 32 + lane] = jr;
     const int sl = jr < 0 ? -1 : (jr & ~JSAME);
     if (sl >= 0) {
@@ -634,107 +641,86 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !VIR && !MULTI) ? PAIR
     }
   };
 
-  // Tiles go to warps in chunks of CHUNK consecutive tiles: chunk gwarp first, then the next
-  // unclaimed chunk from the launch's counter (ctl[6 + 2 wslot]), so warps that start late (SMs busy with the PME
-  // kernels beside this one) take fewer chunks.  The floating-point partial sums (i-forces,
-  // energies, virial) are closed at every chunk end, so the result does not depend on which warp
-  // took which chunk.  Per chunk the tile records and their j-list words are fetched once (one
-  // round trip each); each tile's slot records are copied one tile ahead into the other buffer,
-  // so only the first tile of a chunk waits for them.
-  unsigned *wq = nb.ctl + 6 + 2 * wslot;
-  const int nchunk = (t_hi - t_lo + CHUNK - 1) / CHUNK;
-  for (int ci = gwarp; ci < nchunk;) {
+  // Work goes to warps in units: at most UNIT_TILES consecutive tiles of one cluster's list, unit
+  // gwarp first, then the next unclaimed one from the launch's counter, so warps that start late
+  // (SMs busy with the PME kernels beside this one) take fewer.  The floating-point partial sums
+  // (i-forces, energies, virial) are closed every CLOSE_TILES tiles of the list, so the result
+  // depends neither on how the lists are cut into units nor on which warp takes which.  A unit's j-list words are fetched
+  // at once; each tile's slot records are copied one tile ahead into the other buffer, so only the
+  // first tile of a unit waits for them.
+  unsigned *wq = nb.ctl + CTL_PAIR + 2 * wslot;
+  for (int ci = u_lo + gwarp; ci < u_hi;) {
     int tnext = 0;
-    if (lane == 0) tnext = nwarps + (int)atomicAdd(wq, 1u);  // claimed now, read at chunk end
-    const int c0 = t_lo + ci * CHUNK;
-    const int nc = min(CHUNK, t_hi - c0);
-    tI = -1;
-    tk = -1;
-    tjb = 0;
-    if (lane < nc) {
-      const int I = nb.tile_blk[c0 + lane], k = nb.tile_k[c0 + lane];
-      // an inconsistent tile record is skipped (unreachable; keeps every access in bounds)
-      if (I >= 0 && I < nb.nblk_total && k >= 0) {
-        const int j0 = nb.jcap_off[I], j1 = nb.jcap_off[I + 1];
-        if (k * JCHUNK < j1 - j0) {
-          tI = I;
-          tk = k;
-          tjb = j0 + k * JCHUNK;
-        }
-      }
-    }
-    for (int t = 0; t < nc; t++) {
-      const int It = __shfl_sync(0xffffffffu, tI, t), kt = __shfl_sync(0xffffffffu, tk, t),
-                jb = __shfl_sync(0xffffffffu, tjb, t);
-      if (It >= 0) cp_async4(jbuf + t * 32 + lane, nb.jlist + jb + lane);
+    if (lane == 0) tnext = u_lo + nwarps + (int)atomicAdd(wq, 1u);  // claimed now, read at the unit's end
+    const int4 un = nb.units[ci < n_front ? ci : nb.unit_cap - 1 - (ci - n_front)];
+    const int I = un.x, k0 = un.y, nc = min(un.z, UNIT_TILES);
+    {
+      // the unit's j-list words, 16 bytes a lane (lists start at multiples of 128 bytes)
+      const int *src = nb.jlist + un.w;
+      for (int e = lane; e < nc * (JCHUNK / 4); e += 32) cp_async16(jbuf + 4 * e, src + 4 * e);
     }
     cp_async_commit();
+    const int sl = I * BLOCK + li;
+    im = nb.slot_meta[sl];
+    const int bidx = __shfl_sync(0xffffffffu, im.w, 0);
+    if (bidx != curBox) {
+      flush_e();
+      curBox = bidx;
+      bx = s.box + bidx;
+      __syncwarp();
+      if (lane == 0)
+        for (int c = 0; c < 3; c++) {
+          ctx->s[c] = bx->L[c] * (1.0 / 4294967296.0);
+          ctx->sf[c] = (float)(bx->L[c] * (1.0 / 4294967296.0));
+          ctx->L[c] = (float)bx->L[c];
+          ctx->Lr[c] = (float)bx->Lr[c];
+        }
+    }
+    if constexpr (MIXED) {
+      // coordinates relative to cluster atom 0 are minimal-image differences whenever
+      // L/2 > cutoff + cluster extent; otherwise (small boxes) every pair is wrapped again
+      const uint4 lo = nb.blk_lo[I], hi = nb.blk_hi[I];
+      const double rmax = sqrt(p.cut2) + 1e-3;
+      const double sx = bx->L[0] * (1.0 / 4294967296.0), sy = bx->L[1] * (1.0 / 4294967296.0),
+                   sz = bx->L[2] * (1.0 / 4294967296.0);
+      wrap = bx->multi_image || (double)(hi.x - lo.x) * sx + rmax >= 0.5 * bx->L[0] ||
+             (double)(hi.y - lo.y) * sy + rmax >= 0.5 * bx->L[1] ||
+             (double)(hi.z - lo.z) * sz + rmax >= 0.5 * bx->L[2];
+      const uint4 f = nb.slot_fx[sl];
+      const unsigned rx0 = __shfl_sync(0xffffffffu, f.x, 0), ry0 = __shfl_sync(0xffffffffu, f.y, 0),
+                     rz0 = __shfl_sync(0xffffffffu, f.z, 0);
+      __syncwarp();
+      if (lane == 0) {
+        ctx->r0[0] = rx0;
+        ctx->r0[1] = ry0;
+        ctx->r0[2] = rz0;
+      }
+      __syncwarp();
+      if (im.x >= 0) {
+        xi = (float)((double)(int)(f.x - rx0) * sx);
+        yi = (float)((double)(int)(f.y - ry0) * sy);
+        zi = (float)((double)(int)(f.z - rz0) * sz);
+      } else {
+        xi = yi = zi = 1e6f;
+      }
+      qi = __uint_as_float(f.w);
+    } else {
+      const double4 q4 = nb.slot_pq[sl];
+      if (im.x >= 0) {
+        xi = q4.x; yi = q4.y; zi = q4.z;
+      } else {
+        xi = yi = zi = 1e6;
+      }
+      qi = q4.w;
+    }
     cp_async_wait<0>();
+    __syncwarp();  // the words copied by the other lanes
     prefetch(0, 0);
     for (int t = 0; t < nc; t++) {
       if (t + 1 < nc) prefetch(t + 1, (t + 1) & 1);
       else cp_async_commit();  // an empty group keeps the wait count below uniform
       cp_async_wait<1>();      // tile t's copies (all but the newest group) have landed
-      const int buf = t & 1;
-      const int I = __shfl_sync(0xffffffffu, tI, t), k = __shfl_sync(0xffffffffu, tk, t);
-      if (I < 0) continue;
-      if (I != curI) {
-        flush_fi();
-        curI = I;
-        const int sl = I * BLOCK + li;
-        im = nb.slot_meta[sl];
-        const int bidx = __shfl_sync(0xffffffffu, im.w, 0);
-        if (bidx != curBox) {
-          flush_e();
-          curBox = bidx;
-          bx = s.box + bidx;
-          __syncwarp();
-          if (lane == 0)
-            for (int c = 0; c < 3; c++) {
-              ctx->s[c] = bx->L[c] * (1.0 / 4294967296.0);
-              ctx->sf[c] = (float)(bx->L[c] * (1.0 / 4294967296.0));
-              ctx->L[c] = (float)bx->L[c];
-              ctx->Lr[c] = (float)bx->Lr[c];
-            }
-        }
-        if constexpr (MIXED) {
-          // coordinates relative to cluster atom 0 are minimal-image differences whenever
-          // L/2 > cutoff + cluster extent; otherwise (small boxes) every pair is wrapped again
-          const uint4 lo = nb.blk_lo[I], hi = nb.blk_hi[I];
-          const double rmax = sqrt(p.cut2) + 1e-3;
-          const double sx = bx->L[0] * (1.0 / 4294967296.0), sy = bx->L[1] * (1.0 / 4294967296.0),
-                       sz = bx->L[2] * (1.0 / 4294967296.0);
-          wrap = bx->multi_image || (double)(hi.x - lo.x) * sx + rmax >= 0.5 * bx->L[0] ||
-                 (double)(hi.y - lo.y) * sy + rmax >= 0.5 * bx->L[1] ||
-                 (double)(hi.z - lo.z) * sz + rmax >= 0.5 * bx->L[2];
-          const uint4 f = nb.slot_fx[sl];
-          const unsigned rx0 = __shfl_sync(0xffffffffu, f.x, 0), ry0 = __shfl_sync(0xffffffffu, f.y, 0),
-                         rz0 = __shfl_sync(0xffffffffu, f.z, 0);
-          __syncwarp();
-          if (lane == 0) {
-            ctx->r0[0] = rx0;
-            ctx->r0[1] = ry0;
-            ctx->r0[2] = rz0;
-          }
-          __syncwarp();
-          if (im.x >= 0) {
-            xi = (float)((double)(int)(f.x - rx0) * sx);
-            yi = (float)((double)(int)(f.y - ry0) * sy);
-            zi = (float)((double)(int)(f.z - rz0) * sz);
-          } else {
-            xi = yi = zi = 1e6f;
-          }
-          qi = __uint_as_float(f.w);
-        } else {
-          const double4 q4 = nb.slot_pq[sl];
-          if (im.x >= 0) {
-            xi = q4.x; yi = q4.y; zi = q4.z;
-          } else {
-            xi = yi = zi = 1e6;
-          }
-          qi = q4.w;
-        }
-      }
+      const int buf = t & 1, k = k0 + t;
       // 32 listed j-atoms, JSAME marking those that share a molecule with the cluster; the first
       // tile opens with the cluster's own atoms (lane group 0, pairs j > i only)
       const bool diag = (k == 0);
@@ -899,14 +885,13 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !VIR && !MULTI) ? PAIR
         red_add(f + nsl, v1);
         red_add(f + 2 * nsl, v2);
       }
+      if (t + 1 == nc || (k + 1) % CLOSE_TILES == 0) close_sums();
     }
-    spill_e();
-    flush_fi();
+    flush_fi(I);
     ci = __shfl_sync(0xffffffffu, tnext, 0);
   }
-  flush_fi();
   flush_e();
-  // the last warp to finish resets the chunk counter for the next launch (every warp has made
+  // the last warp to finish resets the unit counter for the next launch (every warp has made
   // its last claim before it counts itself here)
   if (lane == 0 && atomicAdd(wq + 1, 1u) == (unsigned)nwarps - 1u) {
     atomicExch(wq, 0u);
@@ -924,7 +909,7 @@ int launch_t(const SystemDev &s, const NbListDev &nb, const PairLaunch &pl, cuda
   const int ntt = pl.p.ntypes * pl.p.ntypes;
   size_t ljbytes = ((size_t)2 * ntt * sizeof(T2) + 15) & ~(size_t)15;
   size_t smem = ljbytes + PAIR_WARPS * (warp_stage_bytes<MIXED>() + sizeof(WarpCtx) +
-                                        (VIR ? 8 : 2) * 32 * sizeof(long long) + warp_pref_bytes<MIXED>());
+                                        (VIR ? 11 : 5) * 32 * sizeof(long long) + warp_pref_bytes<MIXED>());
   // per device: the SM count, the resident blocks and the shared-memory limit they were found for
   static int n_sm[PMB_MAX_DEVICES] = {}, occupancy[PMB_MAX_DEVICES] = {};
   static size_t conf_smem[PMB_MAX_DEVICES] = {};
@@ -941,13 +926,15 @@ int launch_t(const SystemDev &s, const NbListDev &nb, const PairLaunch &pl, cuda
     occupancy[slot] = occ;
     conf_smem[slot] = smem;
   }
-  // persistent: every resident CTA walks its share of the tiles (chunks claimed from a counter,
-  // so any grid size gives the same result)
+  // persistent: every resident CTA walks its share of the units (claimed from a counter, so any
+  // grid size gives the same result).  A grid of 2 to 8 times that, whose CTAs retire one after
+  // another and leave room for the PME stream, was no faster but for FP64 (-6% a step at 15,000
+  // atoms) and cost a lone pair kernel 5 to 20%, as did one CTA per SM fewer.
   const int occ = occupancy[slot];
   const int per_sm = pl.ctas_per_sm > 0 && pl.ctas_per_sm < occ ? pl.ctas_per_sm : occ;
   const int grid = n_sm[slot] * per_sm;
   using T = typename std::conditional<MIXED, float, double>::type;
-  kern<<<grid, PAIR_THREADS, smem, st>>>(s, nb, pl.p, params_t<T>(pl.p), pl.lj, pl.lattice, pl.blk_lo, pl.blk_hi,
+  kern<<<grid, PAIR_THREADS, smem, st>>>(s, nb, pl.p, params_t<T>(pl.p), pl.lj, pl.lattice, pl.unit_kinds,
                                          pl.wslot);
   return 0;
 }
@@ -1079,8 +1066,12 @@ __global__ void __launch_bounds__(AP_THREADS)
     fout[3 * i + 1] = fi[1];
     fout[3 * i + 2] = fi[2];
   }
-  box_accumulate(eacc, b, valid, E_LJ, elj, nullptr);
-  box_accumulate(eacc, b, valid, E_COUL, ec, VIR ? vir : nullptr);
+  BoxSums<false> lj(eacc, E_LJ);
+  lj.term(b, valid, elj, nullptr);
+  lj.flush();
+  BoxSums<VIR> coul(eacc, E_COUL);
+  coul.term(b, valid, ec, VIR ? vir : nullptr);
+  coul.flush();
 }
 
 }  // namespace

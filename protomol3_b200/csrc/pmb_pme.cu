@@ -932,37 +932,6 @@ __global__ void __launch_bounds__(WZ) k_fft_z_inv_warp(PmeDev pm) {
   }
 }
 
-// Exclusion correction in FP64 with the exact erf (NonbondedPMEwaldSystemForce.h:874-911).
-__global__ void k_correction(const SystemDev s, const int *pairs, const int *kind, int n,
-                             double alpha, double a2pi, double csf, int virial) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  bool valid = k < n;
-  double en = 0.0, vir[6] = {0, 0, 0, 0, 0, 0};
-  int box = -1;
-  if (valid) {
-    int a1 = pairs[2 * k], a2 = pairs[2 * k + 1];
-    box = s.atom_box[a1];
-    const BoxDev &b = s.box[box];
-    double rij[3];
-    double r2 = min_diff(b, s.pos + 3 * a1, s.pos + 3 * a2, rij);
-    double qq = s.charge[a1] * s.charge[a2];
-    if (kind[k] == 1) qq *= 1 - csf;
-    double r = sqrt(r2), rr = 1 / r, e = erf(alpha * r) * rr;
-    en = -qq * e;
-    double fs = qq * (a2pi * exp(-alpha * alpha * r2) - e) * rr * rr;
-    double fij[3] = {rij[0] * fs, rij[1] * fs, rij[2] * fs};
-    long long *f1 = s.facc + 3 * (long long)a1, *f2 = s.facc + 3 * (long long)a2;
-    for (int c = 0; c < 3; c++) {
-      long long v = f2fix(fij[c], FORCE_SCALE);
-      red_add(f1 + c, -v);
-      red_add(f2 + c, v);
-    }
-    vir[0] = fij[0] * rij[0]; vir[1] = fij[0] * rij[1]; vir[2] = fij[0] * rij[2];
-    vir[3] = fij[1] * rij[1]; vir[4] = fij[1] * rij[2]; vir[5] = fij[2] * rij[2];
-  }
-  box_accumulate(s.eacc, box, valid, E_COUL, en, virial ? vir : nullptr);
-}
-
 template <typename T>
 int recip_t(const SystemDev &s, const NbListDev &nb, const PmeDev &pm, cudaStream_t st,
             StageMark mark, void *mctx) {
@@ -1034,15 +1003,6 @@ int pme_recip_launch(const SystemDev &s, const NbListDev &nb, const PmeDev &pm, 
                      StageMark mark, void *mctx) {
   return pm.precision ? recip_t<float>(s, nb, pm, st, mark, mctx)
                       : recip_t<double>(s, nb, pm, st, mark, mctx);
-}
-
-int pme_correction_launch(const SystemDev &s, const PmeDev &pm, const int *excl_pairs,
-                          const int *excl_kind, int nexcl, double coulomb_scaling, cudaStream_t st) {
-  if (nexcl <= 0) return 0;
-  const int TB = 256;
-  k_correction<<<(nexcl + TB - 1) / TB, TB, 0, st>>>(s, excl_pairs, excl_kind, nexcl, pm.alpha,
-                                                     pm.a2pi, coulomb_scaling, pm.virial);
-  return 0;
 }
 
 }  // namespace pmb
