@@ -356,6 +356,9 @@ struct pmb_system {
     s.excl_partner = d_excl_partner;
     s.excl_kind = d_excl_kindc;
     s.facc = d_facc;
+    s.fslot = nb.fslot;      // (null without a list; kept while a list waits to be replaced)
+    s.slot_of = nb.slot_of;
+    s.nslot = nb.nslot;
     s.eacc = d_eacc;
     return s;
   }
@@ -415,6 +418,11 @@ int nblist_alloc(pmb_system *s, double rl) {
   cudaStreamSynchronize(s->stream);  // no kernel of the system may still read the old storage
   if (s->side) cudaStreamSynchronize(s->side);
   if (s->terms) cudaStreamSynchronize(s->terms);
+  if (s->nb.fslot && s->nb.slot_of) {
+    // the forces of the last evaluation outlive the list (an MD run's next kick)
+    pair_fold(s->dev(), s->nb, s->stream);
+    CK(cudaStreamSynchronize(s->stream));
+  }
   s->nb_gen++;
   s->nba.~Allocs();
   new (&s->nba) Allocs();
@@ -611,7 +619,8 @@ void mark(void *ctx, const char *name) {
   s->prof->push_back({name, e});
 }
 
-// Enqueues every force of the set on the system stream; accumulators must be zero.
+// Enqueues every force of the set on the system stream; accumulators must be zero.  updated: the
+// list's displacement check and slot records of these positions are made (integrate_kick_drift).
 // Captured kernels keep the priority of the stream they were captured on: without the flag a graph
 // runs at the priority of the stream it is launched into, and the PME kernels queue behind every
 // block of the pair kernel.
@@ -641,7 +650,7 @@ double list_radius(pmb_system *s, pmb_force *const *fs, int n) {
   return need ? std::max(rl, 1.0) + s->skin + 1e-3 : 0.0;
 }
 
-int enqueue_forces(pmb_system *s, pmb_force *const *fs, int n, int virial) {
+int enqueue_forces(pmb_system *s, pmb_force *const *fs, int n, int virial, bool updated = false) {
   SystemDev sd = s->dev();
   cudaStream_t st = s->stream;
   std::vector<PairJob> jobs = pair_jobs(s, fs, n, virial);
@@ -704,7 +713,7 @@ int enqueue_forces(pmb_system *s, pmb_force *const *fs, int n, int virial) {
       CK(cudaMemsetAsync(s->nb.ctl + CTL_FORCED, 1, 1, st));
       s->nb_build_rl = rlist;
     }
-    nblist_sort(sd, s->nb, st);
+    nblist_sort(sd, s->nb, updated, st);
     if (split) {
       CK(cudaEventRecord(s->ev_slots, st));
       CK(cudaStreamWaitEvent(s->side, s->ev_slots, 0));
@@ -756,8 +765,6 @@ int enqueue_forces(pmb_system *s, pmb_force *const *fs, int n, int virial) {
     CK(cudaEventRecord(s->ev_terms, sterms));
     CK(cudaStreamWaitEvent(st, s->ev_terms, 0));
   }
-  // slot-ordered pair forces -> facc (a plain read-modify-write: after the join)
-  if (!jobs.empty()) pair_fold(sd, s->nb, st);
   CK(cudaGetLastError());
   return PMB_OK;
 }
@@ -837,17 +844,16 @@ int eval_graph_launch(pmb_system *s, pmb_force *const *fs, int n, int virial, bo
         CK(cudaMemcpyAsync(s->d_fin, hf, sizeof(double) * nf, cudaMemcpyHostToDevice, s->copy));
         CK(cudaEventRecord(s->ev_fin, s->copy));
       }
-      SystemDev sd = s->dev();
+      const SystemDev sd = s->dev();
       zero_accumulators(sd, st);
       int rc = enqueue_forces(s, fs, n, virial);
       if (rc) return rc;
       if (direct) {  // the caller's forces, uploaded beside the force kernels, are the base
         CK(cudaStreamWaitEvent(st, s->ev_fin, hf ? 0 : cudaEventWaitExternal));
-        forces_to_double(sd, s->d_fout, st, s->d_fin);
+        results_to_double(sd, s->d_fout, s->d_fin, s->d_eout, st);
       } else {
-        forces_to_double(sd, s->d_fout, st);
+        results_to_double(sd, s->d_fout, nullptr, s->d_eout, st);
       }
-      energies_to_double(sd, nullptr, s->d_eout, st);
       rc = enqueue_eval_copies(s, !direct);
       if (rc) return rc;
       if (hf) {
@@ -1506,12 +1512,10 @@ int pmb_evaluate_device(pmb_system *s, pmb_force *const *fs, int n, const double
     s->have_pos = true;
   }
   if (!s->have_pos) return fail(PMB_ERR_STATE, "no positions on the device yet: pass positions");
-  SystemDev sd = s->dev();
-  zero_accumulators(sd, st);
+  zero_accumulators(s->dev(), st);
   int rc = enqueue_forces(s, fs, n, virial);
   if (rc) return rc;
-  if (d_forces) forces_to_double(sd, d_forces, st);
-  if (d_energies) energies_to_double(sd, nullptr, d_energies, st);
+  results_to_double(s->dev(), d_forces, nullptr, d_energies, st);  // (the list may be new)
   CK(cudaGetLastError());
   return PMB_OK;
 }
@@ -1778,8 +1782,7 @@ int pmb_profile(pmb_system *s, const double *pos, pmb_force *const *fs, int n, i
   if (!s->have_pos) return fail(PMB_ERR_STATE, "no positions on the device yet: pass positions");
   const size_t flush_bytes = 256ull << 20;  // twice the 126 MB L2
   if (flush_l2 && !s->flush_buf) CK(cudaMalloc(&s->flush_buf, flush_bytes));
-  SystemDev sd = s->dev();
-  zero_accumulators(sd, st);
+  zero_accumulators(s->dev(), st);
   int rc = enqueue_forces(s, fs, n, 0);  // warm-up (also sizes the neighbour list)
   if (rc) return rc;
   CK(cudaStreamSynchronize(st));
@@ -1787,7 +1790,7 @@ int pmb_profile(pmb_system *s, const double *pos, pmb_force *const *fs, int n, i
   std::vector<double> acc;
   for (int r = 0; r < nrep; r++) {
     if (flush_l2) CK(cudaMemsetAsync(s->flush_buf, r & 0xff, flush_bytes, st));
-    zero_accumulators(sd, st);
+    zero_accumulators(s->dev(), st);
     std::vector<std::pair<std::string, cudaEvent_t>> ev;
     s->prof = &ev;
     mark(s, "start");
@@ -1838,7 +1841,8 @@ struct pmb_md {
   pmb_integrator_desc d{};
   IntegratorDev in{};
   Allocs a;
-  double *d_vel = nullptr, *d_kin = nullptr;
+  double *d_vel = nullptr, *d_kin = nullptr, *d_kin_parts = nullptr;
+  unsigned *d_kin_done = nullptr;
   long long *d_step = nullptr;
   unsigned long long *d_box_seed = nullptr;  // per box noise seed and step offset
   long long *d_box_step0 = nullptr;
@@ -1875,19 +1879,22 @@ namespace {
 int md_step_enqueue(pmb_md *m, double kick) {
   pmb_system *s = m->sys;
   SystemDev sd = s->dev();
+  // without SHAKE the drift leaves the step's final positions: the list's check joins it
+  const bool fused = !m->shake && list_radius(s, m->forces.data(), (int)m->forces.size()) > 0.0;
+  NbListDev *nb = fused ? &s->nb : nullptr;
   if (kick == 1.0 && m->rattle) {
     integrate_half_kick(sd, m->in, s->stream);
     if (constraints_apply(m->con, m->in, 1, s->stream)) return fail(PMB_ERR_CUDA, "RATTLE launch");
-    integrate_kick_drift(sd, m->in, 0.5, s->stream);
+    integrate_kick_drift(sd, m->in, 0.5, nb, s->stream);
   } else {
-    integrate_kick_drift(sd, m->in, kick, s->stream);
+    integrate_kick_drift(sd, m->in, kick, nb, s->stream);
   }
   if (m->shake && constraints_apply(m->con, m->in, 0, s->stream)) return fail(PMB_ERR_CUDA, "SHAKE launch");
-  return enqueue_forces(s, m->forces.data(), (int)m->forces.size(), m->virial ? 1 : 0);
+  return enqueue_forces(s, m->forces.data(), (int)m->forces.size(), m->virial ? 1 : 0, fused);
 }
 
-// Before a capture: the list storage the run's forces need exists, and a change of list radius
-// has been marked (a rebuild) outside the graph, so that the captured step neither allocates nor
+// Before a run's steps: the list storage its forces need exists, and a change of list radius
+// has been marked (a rebuild) outside the step, so that the captured step neither allocates nor
 // forces a rebuild on every replay.
 int md_prepare_list(pmb_md *m) {
   pmb_system *s = m->sys;
@@ -1953,11 +1960,13 @@ pmb_md *pmb_md_create(pmb_system *s, pmb_force *const *fs, int n, const pmb_inte
   const double INV_TIMEFACTOR = 0.02045482828087295, BOLTZMANN = 0.001987191;
   m->d_vel = m->a.get<double>(3 * (size_t)s->natoms);
   m->d_kin = m->a.get<double>(s->nbox);
+  m->d_kin_parts = m->a.get<double>(KIN_PARTS * (size_t)s->nbox);
+  m->d_kin_done = m->a.get<unsigned>(s->nbox);
   m->d_step = m->a.get<long long>(1);
   m->h_box_seed.resize(s->nbox);
   m->h_box_step0.assign(s->nbox, 0);
   for (int b = 0; b < s->nbox; b++) m->h_box_seed[b] = d->seed + (unsigned long long)b;
-  if (!m->d_vel || !m->d_kin || !m->d_step || upload(m->a, m->d_box_seed, m->h_box_seed) ||
+  if (!m->d_vel || !m->d_kin || !m->d_kin_parts || !m->d_kin_done || !m->d_step || upload(m->a, m->d_box_seed, m->h_box_seed) ||
       upload(m->a, m->d_box_step0, m->h_box_step0)) {
     delete m;
     return fail(PMB_ERR_CUDA, "allocation failed"), nullptr;
@@ -1966,6 +1975,12 @@ pmb_md *pmb_md_create(pmb_system *s, pmb_force *const *fs, int n, const pmb_inte
   m->in.h = d->timestep_fs * INV_TIMEFACTOR;
   m->in.gamma = d->gamma_ps / (1000 * INV_TIMEFACTOR);  // LangevinLeapfrogIntegrator.cpp:28
   m->in.kT = BOLTZMANN * d->temperature;
+  if (d->kind == PMB_LANGEVIN) {  // LangevinLeapfrogIntegrator.cpp:50-56
+    const double g = m->in.gamma, h = m->in.h;
+    m->in.vdt = std::exp(-0.5 * g * h);
+    m->in.fdt = (1.0 - m->in.vdt) / g;
+    m->in.ndt = std::sqrt((1.0 - std::exp(-g * h)) / (2.0 * g));
+  }
   m->in.seed = d->seed;
   m->in.box_seed = m->d_box_seed;
   m->in.box_step0 = m->d_box_step0;
@@ -2186,7 +2201,6 @@ int pmb_md_set_checkpoint(pmb_md *m, const double *pos, const double *vel, const
         (list_reference && !std::isfinite(list_reference[i])))
       return fail(PMB_ERR_NUMERIC, "non-finite state");
   const size_t bytes = sizeof(double) * 3 * (size_t)s->natoms;
-  SystemDev sd = s->dev();
   m->have_state = false;
   for (int attempt = 0; attempt < 3; attempt++) {
     int rc = PMB_OK;
@@ -2196,7 +2210,7 @@ int pmb_md_set_checkpoint(pmb_md *m, const double *pos, const double *vel, const
       CK(cudaMemcpyAsync(s->d_pos, list_reference, bytes, cudaMemcpyHostToDevice, s->stream));
       s->have_pos = true;
       if (s->nb_ready) CK(cudaMemsetAsync(s->nb.ctl + CTL_FORCED, 1, 1, s->stream));  // rebuild
-      zero_accumulators(sd, s->stream);
+      zero_accumulators(s->dev(), s->stream);
       rc = enqueue_forces(s, m->forces.data(), (int)m->forces.size(), m->virial ? 1 : 0);
       if (rc) return rc;
       rc = check_status(s);
@@ -2209,7 +2223,7 @@ int pmb_md_set_checkpoint(pmb_md *m, const double *pos, const double *vel, const
       // the Langevin noise counter: the restored run draws the streams the original would have
       CK(cudaMemcpyAsync(m->d_step, &step, sizeof(long long), cudaMemcpyHostToDevice, s->stream));
       constraints_init(m->con, m->in, s->stream);  // the new positions are SHAKE's last ones
-      zero_accumulators(sd, s->stream);
+      zero_accumulators(s->dev(), s->stream);
       rc = enqueue_forces(s, m->forces.data(), (int)m->forces.size(), m->virial ? 1 : 0);
       if (rc) return rc;
       rc = check_status(s);  // also waits for the step count's host copy
@@ -2261,9 +2275,8 @@ int pmb_md_run(pmb_md *m, int n) {
   pmb_system *s = m->sys;
   // the legacy default stream cannot be captured: replay eagerly there
   const bool graph_ok = s->stream != nullptr && s->stream != cudaStreamLegacy;
+  if (int prc = md_prepare_list(m)) return prc;
   if (m->use_graph && graph_ok) {
-    int prc = md_prepare_list(m);
-    if (prc) return prc;
     if (m->graph_gen != s->nb_gen) m->drop_graphs();
     m->graph_gen = s->nb_gen;
     if (!m->g_first) {
@@ -2359,8 +2372,10 @@ int pmb_md_energies(pmb_md *m, double *energies, double *kinetic) {
   if (!m) return fail(PMB_ERR_ARG, "null md");
   pmb_system *s = m->sys;
   SystemDev sd = s->dev();
-  energies_to_double(sd, nullptr, s->d_eout, s->stream);
-  kinetic_energy(sd, m->in, m->d_kin, s->stream);
+  energies_to_double(sd, s->d_eout, s->stream);
+  int max_box_atoms = 0;
+  for (const BoxDev &b : s->hbox) max_box_atoms = std::max(max_box_atoms, b.natoms);
+  kinetic_energy(sd, m->in, m->d_kin, m->d_kin_parts, m->d_kin_done, max_box_atoms, s->stream);
   CK(cudaMemcpyAsync(m->h_e.data(), s->d_eout, sizeof(double) * m->h_e.size(), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaMemcpyAsync(m->h_k.data(), m->d_kin, sizeof(double) * m->h_k.size(), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
@@ -2406,10 +2421,10 @@ extern "C" int pmb_cutoff_evaluate_static(pmb_force *f, const double *d_position
   for (const BoxDev &b : s->hbox) max_box_atoms = std::max(max_box_atoms, b.natoms);
   SystemDev sd = s->dev();
   sd.eacc = eacc;
-  sd.facc = nullptr;
+  sd.facc = sd.fslot = nullptr;
   CK(pair_allpairs_launch(sd, p, s->d_lj, d_positions, d_forces, eacc, max_box_atoms, s->stream));
   if (d_energies) {
-    energies_to_double(sd, nullptr, d_energies, s->stream);
+    energies_to_double(sd, d_energies, s->stream);
     CK(cudaGetLastError());
   }
   return PMB_OK;

@@ -73,8 +73,7 @@ struct NbListDev {
   uint4 *slot_fx;              // [nslot] fractional fixed-point x, y, z (2^32 per edge) + q bits
   double4 *slot_pq;            // [nslot] raw double position + q (FP64 path)
   int4 *slot_meta;             // [nslot] orig, molecule, type, box
-  long long *fslot;            // [3][nslot] pair forces by slot (component-major), fixed point;
-                               // folded into facc and cleared after the pair kernels
+  long long *fslot;            // [3][nslot] pair forces by slot (component-major), fixed point
   // sort
   int nkeys;
   int *key;                    // [natoms] sort bin within the atom's box
@@ -108,11 +107,16 @@ struct SystemDev {
   const double *charge;        // [natoms]
   const int *type, *molecule;  // [natoms]
   const int *excl_start, *excl_partner, *excl_kind;  // CSR by atom
+  // the forces of the last evaluation, fixed point: facc by atom plus fslot by slot (component-major
+  // [3][nslot], the pair kernel's part; slot_of null without a list), summed by who reads them
   long long *facc;             // [3 natoms]
+  long long *fslot;
+  const int *slot_of;          // [natoms]
+  int nslot;
   long long *eacc;             // [nbox * ACC_PER_BOX]
 };
 
-int nblist_sort(const SystemDev &s, NbListDev &nb, cudaStream_t st);
+int nblist_sort(const SystemDev &s, NbListDev &nb, bool updated, cudaStream_t st);
 int nblist_lists(const SystemDev &s, NbListDev &nb, double list_cutoff, cudaStream_t st);
 int fp32_peak_probe(double *tflops);
 
@@ -211,9 +215,10 @@ struct CorrectionDev {
 };
 // Exclusion corrections and bonded terms in one launch (either may be null).
 int atom_terms_launch(const SystemDev &s, const CorrectionDev *c, const BondedDev *b, cudaStream_t st);
-// out = base + the accumulated forces (base may be null)
-int forces_to_double(const SystemDev &s, double *out, cudaStream_t st, const double *base = nullptr);
-int energies_to_double(const SystemDev &s, const double *const_e, double *out, cudaStream_t st);
+// fout = base + the accumulated forces (base may be null), eout = the energies; either may be null
+int results_to_double(const SystemDev &s, double *fout, const double *base, double *eout, cudaStream_t st);
+int forces_to_double(const SystemDev &s, double *out, cudaStream_t st);
+int energies_to_double(const SystemDev &s, double *out, cudaStream_t st);
 int zero_accumulators(const SystemDev &s, cudaStream_t st);
 
 struct IntegratorDev {
@@ -226,6 +231,7 @@ struct IntegratorDev {
   // box and its box's step, so a box draws the same numbers alone and beside other boxes
   const unsigned long long *box_seed;  // [nbox]
   const long long *box_step0;          // [nbox]
+  double fdt, vdt, ndt;  // Langevin half kick factors (langevin_half_kick)
   const double *mass;  // [natoms]
   double *pos, *vel;
   long long *step;     // device step counter
@@ -264,8 +270,12 @@ constexpr int CON_ERR_BLOCK = 2 * (CON_MAX_SWEEPS + 1) + 2;
 constexpr int CON_WINDOW = 3;
 int constraints_init(const ConstraintDev &c, const IntegratorDev &in, cudaStream_t st);
 int constraints_apply(const ConstraintDev &c, const IntegratorDev &in, int rattle, cudaStream_t st);
-int integrate_kick_drift(const SystemDev &s, const IntegratorDev &in, double kick, cudaStream_t st);
+// kick and drift; with nb also the list's displacement check and slot records (update_atom)
+int integrate_kick_drift(const SystemDev &s, const IntegratorDev &in, double kick, NbListDev *nb, cudaStream_t st);
 int integrate_half_kick(const SystemDev &s, const IntegratorDev &in, cudaStream_t st);
-int kinetic_energy(const SystemDev &s, const IntegratorDev &in, double *out_per_box, cudaStream_t st);
+// parts [KIN_PARTS nbox] and done [nbox] (zero between launches): scratch
+constexpr int KIN_PARTS = 64;
+int kinetic_energy(const SystemDev &s, const IntegratorDev &in, double *out_per_box, double *parts, unsigned *done,
+                   int max_box_atoms, cudaStream_t st);
 
 }  // namespace pmb

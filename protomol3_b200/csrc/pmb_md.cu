@@ -9,7 +9,10 @@
 //   noise comes from a counter-based generator keyed by (the box's seed, the atom's index within
 //   its box, the box's step, component): every trajectory is reproducible bit for bit and
 //   independent of how boxes are batched.
+#include <algorithm>
+
 #include "pmb_internal.h"
+#include "pmb_update.cuh"
 
 namespace pmb {
 
@@ -136,22 +139,28 @@ __global__ void __launch_bounds__(ATOM_TERM_THREADS)
   sums.flush();
 }
 
-__global__ void k_forces_to_double(const SystemDev s, double *out, const double *base) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 3 * s.natoms) return;
-  const double f = (double)s.facc[i] * (1.0 / FORCE_SCALE);
-  out[i] = base ? base[i] + f : f;
+// The slot of atom i's pair forces, or -1.
+__device__ __forceinline__ int force_slot(const SystemDev &s, int i) { return s.slot_of ? s.slot_of[i] : -1; }
+// Component c of the force on atom i in fixed point, sl = force_slot(s, i).
+__device__ __forceinline__ long long force_fixed(const SystemDev &s, int i, int c, int sl) {
+  const long long f = s.facc[3 * (long long)i + c];
+  return sl >= 0 ? f + s.fslot[(long long)c * s.nslot + sl] : f;
 }
 
-__global__ void k_energies_to_double(const SystemDev s, const double *cst, double *out) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= s.nbox * ACC_PER_BOX) return;
-  out[i] = (double)s.eacc[i] * (1.0 / ENERGY_SCALE) + (cst ? cst[i] : 0.0);
+__global__ void k_results_to_double(const SystemDev s, double *fout, const double *base, double *eout) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (eout && i < s.nbox * ACC_PER_BOX) eout[i] = (double)s.eacc[i] * (1.0 / ENERGY_SCALE);
+  if (!fout || i >= 3 * s.natoms) return;
+  const int a = i / 3;
+  const double f = (double)force_fixed(s, a, i - 3 * a, force_slot(s, a)) * (1.0 / FORCE_SCALE);
+  fout[i] = base ? base[i] + f : f;
 }
 
-__global__ void k_zero(long long *a, long long n) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) a[i] = 0;
+__global__ void k_zero(const SystemDev s) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < 3ll * s.natoms) s.facc[i] = 0;
+  if (s.fslot && i < 3ll * s.nslot) s.fslot[i] = 0;
+  if (i < s.nbox * ACC_PER_BOX) s.eacc[i] = 0;
 }
 
 // Counter-based generator: a 4x32 Philox-style bijective mixing round function (Salmon et al.,
@@ -198,90 +207,127 @@ __device__ __forceinline__ double langevin_half_kick(double v, double f, double 
   return __dadd_rn(__dadd_rn(__dmul_rn(v, vdt), __ddiv_rn(__dmul_rn(f, fdt), m)), __dmul_rn(__dmul_rn(r, sq), ndt));
 }
 
-// Leapfrog kick (coefficient 1 or 1/2) + drift; the force accumulator is consumed and cleared.
-__global__ void k_kick_drift(const SystemDev s, IntegratorDev in, double kick) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+// Leapfrog kick (coefficient 1 or 1/2) + drift; the forces are consumed and cleared.  All of an
+// atom's loads are issued before the first store (with the stores between them, the components
+// were three chains of latency in a row: 11.5 us at 98,304 atoms).  UPDATE: also the list's
+// displacement check and slot records, the new position being in registers.
+template <bool LANGEVIN, bool UPDATE>
+__global__ void __launch_bounds__(UPDATE_THREADS) k_kick_drift(const SystemDev s, IntegratorDev in, NbListDev nb, double kick) {
+  const int i = blockIdx.x * UPDATE_THREADS + threadIdx.x;
   if (i < s.nbox * ACC_PER_BOX) s.eacc[i] = 0;
-  if (i >= s.natoms) return;
-  const double h = in.h, m = in.mass[i];
-  long long *fa = s.facc + 3 * (long long)i;
-  double *v = in.vel + 3 * (long long)i, *x = in.pos + 3 * (long long)i;
-  if (in.kind == 0) {
+  double x[3] = {0.0, 0.0, 0.0};
+  if (i < s.natoms) {
+    const double h = in.h, m = in.mass[i];
+    const int sl = force_slot(s, i);
+    double *vp = in.vel + 3 * (long long)i, *xp = in.pos + 3 * (long long)i;
+    double v[3], f[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      double f = (double)fa[c] * (1.0 / FORCE_SCALE);
-      fa[c] = 0;
-      // (F * h * 0.5) / m for the half kick, (F * h) / m for the full kick, as the reference
-      v[c] += kick == 1.0 ? f * h / m : f * h * 0.5 / m;
-      x[c] = __dadd_rn(x[c], __dmul_rn(v[c], h));  // rounded like the reference's x += v * h
+      v[c] = vp[c];
+      x[c] = xp[c];
+      f[c] = (double)force_fixed(s, i, c, sl) * (1.0 / FORCE_SCALE);
     }
-  } else {
-    // Langevin (StandardIntegrator::run, StandardIntegrator.cpp:27-37): per step a noisy half
-    // kick, drift, forces, noisy half kick.  The half kick closing step s-1 (noise stream 2s-1)
-    // is applied here together with the opening half kick of step s (stream 2s); run() ends
-    // with k_half_kick closing the last step.
-    const int b = s.atom_box[i], ia = i - s.box[b].atom0;
-    const long long step = *in.step + in.box_step0[b];
-    const double g = in.gamma;
-    const double fdt = (1.0 - exp(-0.5 * g * h)) / g, vdt = exp(-0.5 * g * h);
-    const double ndt = sqrt((1.0 - exp(-g * h)) / (2.0 * g));
-    const double sq = sqrt(2.0 * in.kT * g / m);
-    double ra[3], rb[3];
-    gauss3(in.box_seed[b], ia, 2 * step, ra);
-    if (kick == 1.0) gauss3(in.box_seed[b], ia, 2 * step - 1, rb);
+    if constexpr (!LANGEVIN) {
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        // (F * h * 0.5) / m for the half kick, (F * h) / m for the full kick, as the reference
+        v[c] += kick == 1.0 ? f[c] * h / m : f[c] * h * 0.5 / m;
+        x[c] = __dadd_rn(x[c], __dmul_rn(v[c], h));  // rounded like the reference's x += v * h
+      }
+    } else {
+      // Langevin (StandardIntegrator::run, StandardIntegrator.cpp:27-37): per step a noisy half
+      // kick, drift, forces, noisy half kick.  The half kick closing step s-1 (noise stream 2s-1)
+      // is applied here together with the opening half kick of step s (stream 2s); run() ends
+      // with k_half_kick closing the last step.
+      const int b = s.atom_box[i], ia = i - s.box[b].atom0;
+      const long long step = *in.step + in.box_step0[b];
+      const double sq = sqrt(2.0 * in.kT * in.gamma / m);
+      double ra[3], rb[3];
+      gauss3(in.box_seed[b], ia, 2 * step, ra);
+      if (kick == 1.0) gauss3(in.box_seed[b], ia, 2 * step - 1, rb);
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        if (kick == 1.0) v[c] = langevin_half_kick(v[c], f[c], rb[c], in.vdt, in.fdt, m, sq, in.ndt);
+        v[c] = langevin_half_kick(v[c], f[c], ra[c], in.vdt, in.fdt, m, sq, in.ndt);
+        x[c] = __dadd_rn(x[c], __dmul_rn(v[c], h));
+      }
+    }
+    long long *fa = s.facc + 3 * (long long)i;
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      double f = (double)fa[c] * (1.0 / FORCE_SCALE);
+      vp[c] = v[c];
+      xp[c] = x[c];
       fa[c] = 0;
-      if (kick == 1.0) v[c] = langevin_half_kick(v[c], f, rb[c], vdt, fdt, m, sq, ndt);
-      v[c] = langevin_half_kick(v[c], f, ra[c], vdt, fdt, m, sq, ndt);
-      x[c] = __dadd_rn(x[c], __dmul_rn(v[c], h));
+      if (sl >= 0) s.fslot[(long long)c * s.nslot + sl] = 0;
     }
   }
+  if constexpr (UPDATE) update_atom(s, nb, i, x, LANGEVIN ? in.step : nullptr);
 }
 
 __global__ void k_half_kick(const SystemDev s, IntegratorDev in) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= s.natoms) return;
   const double h = in.h, m = in.mass[i];
-  const long long *fa = s.facc + 3 * (long long)i;
-  double *v = in.vel + 3 * (long long)i;
+  const int sl = force_slot(s, i);
+  double *vp = in.vel + 3 * (long long)i;
+  double v[3], f[3];
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    v[c] = vp[c];
+    f[c] = (double)force_fixed(s, i, c, sl) * (1.0 / FORCE_SCALE);
+  }
   if (in.kind == 0) {
-    for (int c = 0; c < 3; c++) v[c] += ((double)fa[c] * (1.0 / FORCE_SCALE)) * h * 0.5 / m;
+#pragma unroll
+    for (int c = 0; c < 3; c++) v[c] += f[c] * h * 0.5 / m;
   } else {
     const int b = s.atom_box[i], ia = i - s.box[b].atom0;
     const long long step = *in.step + in.box_step0[b];
-    const double g = in.gamma;
-    const double fdt = (1.0 - exp(-0.5 * g * h)) / g, vdt = exp(-0.5 * g * h);
-    const double ndt = sqrt((1.0 - exp(-g * h)) / (2.0 * g));
-    const double sq = sqrt(2.0 * in.kT * g / m);
+    const double sq = sqrt(2.0 * in.kT * in.gamma / m);
     double rp[3];
     gauss3(in.box_seed[b], ia, 2 * step - 1, rp);  // closes the last completed step
-    for (int c = 0; c < 3; c++)
-      v[c] = langevin_half_kick(v[c], (double)fa[c] * (1.0 / FORCE_SCALE), rp[c], vdt, fdt, m, sq, ndt);
+#pragma unroll
+    for (int c = 0; c < 3; c++) v[c] = langevin_half_kick(v[c], f[c], rp[c], in.vdt, in.fdt, m, sq, in.ndt);
   }
+#pragma unroll
+  for (int c = 0; c < 3; c++) vp[c] = v[c];
 }
 
 __global__ void k_step_inc(long long *step) { *step += 1; }
 
-__global__ void k_kinetic(const SystemDev s, IntegratorDev in, double *out) {
-  // one block per box, fixed-order reduction
-  int b = blockIdx.x;
-  const BoxDev &bx = s.box[b];
+// Kinetic energy per box: at most KIN_PARTS blocks, each over a fixed run of the box's atoms in a
+// fixed order, then the last of them adds the parts in order (one block took 126 us at 98,304 atoms).
+constexpr int KIN_ATOMS = 2048;  // atoms of a part, more in boxes over KIN_PARTS times that
+__global__ void __launch_bounds__(256) k_kinetic(const SystemDev s, IntegratorDev in, double *out, double *parts, unsigned *done) {
+  const int b = blockIdx.y, n = s.box[b].natoms;
+  const int per = max(KIN_ATOMS, (n + KIN_PARTS - 1) / KIN_PARTS), np = (n + per - 1) / per;
+  const int part = blockIdx.x;
+  if (part >= np) return;
+  const int i0 = s.box[b].atom0, end = i0 + min(n, (part + 1) * per);
   double acc = 0.0;
-  for (int i = bx.atom0 + threadIdx.x; i < bx.atom0 + bx.natoms; i += blockDim.x) {
+#pragma unroll 4
+  for (int i = i0 + part * per + threadIdx.x; i < end; i += 256) {
     const double *v = in.vel + 3 * (long long)i;
     acc += 0.5 * in.mass[i] * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
   }
-  __shared__ double red[32];
+  __shared__ double red[8];
   acc = warp_sum(acc);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
   __syncthreads();
-  if (threadIdx.x < 32) {
-    double r = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
-    r = warp_sum(r);
-    if (threadIdx.x == 0) out[b] = r;
+  if (threadIdx.x != 0) return;
+  double r = 0.0;
+  for (int k = 0; k < 8; k++) r += red[k];
+  if (np == 1) {
+    out[b] = r;
+    return;
   }
+  parts[b * KIN_PARTS + part] = r;
+  __threadfence();
+  if (atomicAdd(done + b, 1u) != (unsigned)np - 1u) return;
+  __threadfence();
+  done[b] = 0u;
+  r = 0.0;
+  for (int k = 0; k < np; k++) r += __ldcg(parts + b * KIN_PARTS + k);
+  out[b] = r;
 }
 
 // FP32 FMA issue-rate probe: 8 independent dependency chains per thread keep the FMA pipes
@@ -771,31 +817,36 @@ int atom_terms_launch(const SystemDev &s, const CorrectionDev *c, const BondedDe
   return 0;
 }
 
-int forces_to_double(const SystemDev &s, double *out, cudaStream_t st, const double *base) {
-  const int T = 256, n = 3 * s.natoms;
-  if (n > 0) k_forces_to_double<<<(n + T - 1) / T, T, 0, st>>>(s, out, base);
+int results_to_double(const SystemDev &s, double *fout, const double *base, double *eout, cudaStream_t st) {
+  const int T = 256, n = std::max(fout ? 3 * s.natoms : 0, eout ? s.nbox * ACC_PER_BOX : 0);
+  if (n > 0) k_results_to_double<<<(n + T - 1) / T, T, 0, st>>>(s, fout, base, eout);
   return 0;
 }
-
-int energies_to_double(const SystemDev &s, const double *cst, double *out, cudaStream_t st) {
-  const int T = 128, n = s.nbox * ACC_PER_BOX;
-  k_energies_to_double<<<(n + T - 1) / T, T, 0, st>>>(s, cst, out);
-  return 0;
+int forces_to_double(const SystemDev &s, double *out, cudaStream_t st) {
+  return results_to_double(s, out, nullptr, nullptr, st);
+}
+int energies_to_double(const SystemDev &s, double *out, cudaStream_t st) {
+  return results_to_double(s, nullptr, nullptr, out, st);
 }
 
 int zero_accumulators(const SystemDev &s, cudaStream_t st) {
   const int T = 256;
-  long long n = 3LL * s.natoms;
-  if (n > 0) k_zero<<<(unsigned)((n + T - 1) / T), T, 0, st>>>(s.facc, n);
-  long long ne = (long long)s.nbox * ACC_PER_BOX;
-  k_zero<<<(unsigned)((ne + T - 1) / T), T, 0, st>>>(s.eacc, ne);
+  const long long n = std::max(3ll * s.natoms, std::max(s.fslot ? 3ll * s.nslot : 0ll, (long long)s.nbox * ACC_PER_BOX));
+  if (n > 0) k_zero<<<(unsigned)((n + T - 1) / T), T, 0, st>>>(s);
   return 0;
 }
 
-int integrate_kick_drift(const SystemDev &s, const IntegratorDev &in, double kick, cudaStream_t st) {
-  const int T = 256;
-  int n = s.natoms > s.nbox * ACC_PER_BOX ? s.natoms : s.nbox * ACC_PER_BOX;
-  k_kick_drift<<<(n + T - 1) / T, T, 0, st>>>(s, in, kick);
+int integrate_kick_drift(const SystemDev &s, const IntegratorDev &in, double kick, NbListDev *nb, cudaStream_t st) {
+  const int T = UPDATE_THREADS;
+  // (the energy words are cleared by threads past the last atom where the atoms are fewer)
+  const int grid = (std::max(s.natoms, s.nbox * ACC_PER_BOX) + T - 1) / T;
+  if (nb) {
+    if (in.kind == 1) k_kick_drift<true, true><<<grid, T, 0, st>>>(s, in, *nb, kick);
+    else k_kick_drift<false, true><<<grid, T, 0, st>>>(s, in, *nb, kick);
+    return 0;
+  }
+  if (in.kind == 1) k_kick_drift<true, false><<<grid, T, 0, st>>>(s, in, NbListDev{}, kick);
+  else k_kick_drift<false, false><<<grid, T, 0, st>>>(s, in, NbListDev{}, kick);
   if (in.kind == 1) k_step_inc<<<1, 1, 0, st>>>(in.step);
   return 0;
 }
@@ -806,8 +857,10 @@ int integrate_half_kick(const SystemDev &s, const IntegratorDev &in, cudaStream_
   return 0;
 }
 
-int kinetic_energy(const SystemDev &s, const IntegratorDev &in, double *out, cudaStream_t st) {
-  k_kinetic<<<s.nbox, 256, 0, st>>>(s, in, out);
+int kinetic_energy(const SystemDev &s, const IntegratorDev &in, double *out, double *parts, unsigned *done,
+                   int max_box_atoms, cudaStream_t st) {
+  const int np = std::max(1, std::min(KIN_PARTS, (max_box_atoms + KIN_ATOMS - 1) / KIN_ATOMS));
+  k_kinetic<<<dim3(np, s.nbox), 256, 0, st>>>(s, in, out, parts, done);
   return 0;
 }
 

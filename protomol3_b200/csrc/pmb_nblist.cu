@@ -8,6 +8,7 @@
 // cutoff of I's bounding box.  The pair kernel then sees (I, 32 j-atoms) tiles; the pair set it
 // evaluates is exactly the reference's: every unordered pair once, minimal image, r^2 <= rc^2.
 #include "pmb_internal.h"
+#include "pmb_update.cuh"
 
 namespace pmb {
 
@@ -49,15 +50,6 @@ __device__ __forceinline__ unsigned hilbert3(unsigned x, unsigned y, unsigned z,
   return h;
 }
 
-__device__ __forceinline__ unsigned frac_fixed(double x, double Lr) {
-  double u = x * Lr;
-  u -= floor(u);
-  double s = u * 4294967296.0;
-  if (!(s >= 0.0)) s = 0.0;                 // also catches NaN
-  if (s >= 4294967295.0) s = 4294967295.0;
-  return (unsigned)s;
-}
-
 // ---------------------------------------------------------------- scans
 __device__ int block_exclusive_scan(int v, int *total) {
   __shared__ int warp_tot[32];
@@ -88,131 +80,13 @@ __device__ int block_exclusive_scan(int v, int *total) {
 }
 
 // ---------------------------------------------------------------- binning and sort
-// Rebuild decision, box by box: max |x - x_ref|^2 over each box's atoms (box_d2), then the last
-// block sets box_rb[b] for every box that moved more than half the skin and ctl[CTL_REBUILD] when
-// any did (no host round trip).
-// It reads every position of every evaluation, so it also raises status[2] for a non-finite
-// one (the host reports PMB_ERR_NUMERIC; every later kernel maps such a position to an in-range
-// cell and grid index, so nothing reads out of bounds meanwhile), and, for a system whose boxes
-// stand in for vacuum (ctl[CTL_VACUUM]), status[3] once the atoms of a box spread over half an edge
-// (the minimal image would no longer be the plain difference).
-__device__ __forceinline__ int ford(float f) {  // order-preserving int image of a float
-  const int i = __float_as_int(f);
-  return i >= 0 ? i : i ^ 0x7fffffff;
-}
-__device__ __forceinline__ float fuord(int o) { return __int_as_float(o >= 0 ? o : o ^ 0x7fffffff); }
-
-//
-// The same pass writes this step's coordinates into the atom's slot record (the slot it got at
-// its box's last build; a box that is rebuilt packs its records again afterwards), so a step
-// without a rebuild has no pass of its own for that.
-__global__ void k_update(SystemDev s, NbListDev nb) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  float d2 = 0.f;
-  int box = -1;
-  const bool vacuum = nb.ctl[CTL_VACUUM] != 0u;
-  if (i < s.natoms) {
-    box = s.atom_box[i];
-    const double x = s.pos[3 * i], y = s.pos[3 * i + 1], z = s.pos[3 * i + 2];
-    const int sl = nb.slot_of[i];
-    if (sl >= 0) {
-      const BoxDev &b = s.box[box];
-      // x, y, z of the record; the charge in its last word stays
-      uint4 *f = nb.slot_fx + sl;
-      *reinterpret_cast<uint2 *>(f) = make_uint2(frac_fixed(x, b.Lr[0]), frac_fixed(y, b.Lr[1]));
-      f->z = frac_fixed(z, b.Lr[2]);
-      if (nb.want_fp64) {
-        double4 *q = nb.slot_pq + sl;
-        *reinterpret_cast<double2 *>(q) = make_double2(x, y);
-        q->z = z;
-      }
-    }
-    if (!(isfinite(x) && isfinite(y) && isfinite(z))) atomicExch(&nb.status[2], 1);
-    if (vacuum) {
-      int *e = nb.vext + 6 * s.atom_box[i];
-      const double p[3] = {x, y, z};
+__global__ void __launch_bounds__(UPDATE_THREADS) k_update(SystemDev s, NbListDev nb) {
+  const int i = blockIdx.x * UPDATE_THREADS + threadIdx.x;
+  double x[3] = {0.0, 0.0, 0.0};
+  if (i < s.natoms)
 #pragma unroll
-      for (int d = 0; d < 3; d++) {
-        const int o = ford((float)p[d]);
-        atomicMin(e + d, o);
-        atomicMax(e + 3 + d, o);
-      }
-      __threadfence();
-    }
-    double dx = x - nb.xref[3 * i], dy = y - nb.xref[3 * i + 1], dz = z - nb.xref[3 * i + 2];
-    double r2 = dx * dx + dy * dy + dz * dz;
-    d2 = r2 < 3.0e38 ? (float)r2 : 3.0e38f;
-    if (!(d2 >= 0.f)) d2 = 3.0e38f;  // NaN positions force a rebuild
-  }
-  // per-box maxima (float bits of non-negative values order as unsigned): a warp whose atoms
-  // belong to one box takes its maximum first, and the block adds one atomic per run of such
-  // warps of the same box
-  __shared__ int wbox[32];
-  __shared__ float wmax[32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const unsigned act = __ballot_sync(0xffffffffu, box >= 0);
-  int wb = -1;  // the warp's box when all its atoms share one, else -1 (atomics already added)
-  float m = 0.f;
-  if (act) {
-    const int b0 = __shfl_sync(0xffffffffu, box, __ffs(act) - 1);
-    if (__all_sync(0xffffffffu, box < 0 || box == b0)) {
-      m = d2;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-      wb = b0;
-    } else if (box >= 0) {
-      atomicMax(&nb.box_d2[box], __float_as_uint(d2));
-    }
-  }
-  if (lane == 0) {
-    wbox[w] = wb;
-    wmax[w] = m;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const int nw = (int)(blockDim.x >> 5);
-    for (int k = 0; k < nw;) {
-      const int b = wbox[k];
-      float mm = wmax[k];
-      int k2 = k + 1;
-      for (; k2 < nw && wbox[k2] == b; k2++) mm = fmaxf(mm, wmax[k2]);
-      if (b >= 0) atomicMax(&nb.box_d2[b], __float_as_uint(mm));
-      k = k2;
-    }
-  }
-  __threadfence();
-  __syncthreads();
-  __shared__ bool last;
-  if (threadIdx.x == 0) last = atomicAdd(&nb.ctl[CTL_BLOCKS], 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  const bool forced = nb.ctl[CTL_FORCED] != 0u;
-  int any = 0;
-  for (int b = threadIdx.x; b < s.nbox; b += blockDim.x) {
-    const float mx = __uint_as_float(atomicExch(&nb.box_d2[b], 0u));  // read and reset
-    const unsigned rb = (forced || mx > nb.half_skin2) ? 1u : 0u;
-    nb.box_rb[b] = rb;
-    any |= (int)rb;
-    if (vacuum)
-      for (int d = 0; d < 3; d++) {
-        // read and reset for the next evaluation
-        const float lo = fuord(atomicExch(nb.vext + 6 * b + d, 0x7fffffff));
-        const float hi = fuord(atomicExch(nb.vext + 6 * b + 3 + d, (int)0x80000000));
-        if (!((double)hi - (double)lo < 0.5 * s.box[b].L[d])) atomicExch(&nb.status[3], 1);
-      }
-  }
-  any = __syncthreads_or(any);
-  if (threadIdx.x == 0) {
-    nb.ctl[CTL_REBUILD] = any ? 1u : 0u;
-    if (any) {
-      ++*reinterpret_cast<unsigned long long *>(nb.ctl + CTL_BUILDS);
-      // the build starts its list of pair units anew
-      nb.ctl[CTL_CLAIM] = nb.ctl[CTL_UNITS] = nb.ctl[CTL_UNITS + 1] = nb.ctl[CTL_TILES] = 0u;
-    }
-    nb.ctl[CTL_BLOCKS] = 0u;
-    nb.ctl[CTL_FORCED] = 0u;
-  }
+    for (int c = 0; c < 3; c++) x[c] = s.pos[3 * i + c];
+  update_atom(s, nb, i, x, nullptr);
 }
 
 // ---- the sort into slots, a deterministic counting sort: histogram of the atoms over the
@@ -666,14 +540,14 @@ bool sort_by_box(const SystemDev &s, const NbListDev &nb) {
 
 }  // namespace
 
-// First half of a build: displacement check and this step's slot records, then the sort into
+// First half of a build: displacement check and this step's slot records (unless the kernel that
+// moved the atoms made them), then the sort into
 // slots of the boxes that rebuild (the PME kernels need no more than these).  Every kernel after
 // the displacement check exits at once unless ctl[CTL_REBUILD] asks for a rebuild.
-int nblist_sort(const SystemDev &s, NbListDev &nb, cudaStream_t st) {
-  const int T = 256;
-  int na = s.natoms;
+int nblist_sort(const SystemDev &s, NbListDev &nb, bool updated, cudaStream_t st) {
+  const int na = s.natoms;
   if (na <= 0) return 0;
-  k_update<<<(na + T - 1) / T, T, 0, st>>>(s, nb);
+  if (!updated) k_update<<<(na + UPDATE_THREADS - 1) / UPDATE_THREADS, UPDATE_THREADS, 0, st>>>(s, nb);
   if (sort_by_box(s, nb)) {
     k_sort_box<<<s.nbox, SORT_THREADS, 0, st>>>(s, nb);
     return 0;

@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !VIR && !MULTI) ? PAIR
 
   // forces accumulate by slot, one component-major array per axis: the j-atoms of a tile come
   // in runs of consecutive slots, so a lane group's atomics touch two sectors per axis rather than
-  // eight scattered atoms (pair_fold moves them to original order afterwards)
+  // eight scattered atoms (readers add them to the by-atom forces)
   const long long nsl = nb.nslot;
   // i-forces of the current cluster per lane: the scalar path's in fi_acc, the packed path's
   // (+f, the i-force is -fi) in a2p.fi; the packed path's energies and virial are in a2p too.
@@ -959,8 +959,9 @@ int launch_v(const SystemDev &s, const NbListDev &nb, const PairLaunch &pl, cuda
 
 }  // namespace
 
-// Adds the slot-ordered pair forces to the original-order accumulator and clears them (one thread
-// per slot; each atom owns one slot, so the read-modify-write needs no atomics).
+// Adds the slot-ordered pair forces to the original-order accumulator and clears them, before the
+// list's storage is replaced (one thread per slot; each atom owns one slot, so the read-modify-write
+// needs no atomics).  Otherwise whoever reads the forces adds the two.
 __global__ void k_pair_fold(SystemDev s, NbListDev nb) {
   const int sl = blockIdx.x * blockDim.x + threadIdx.x;
   if (sl >= nb.nslot) return;
