@@ -245,6 +245,9 @@ constexpr int PAIR2_STEPS_UNROLLED = PAIR2_UNROLL;
 #ifndef PAIR_MINB
 #define PAIR_MINB 5  // resident blocks per SM of the mixed kernels
 #endif
+#ifndef PAIR_MINB_VIR
+#define PAIR_MINB_VIR 4  // with the virial
+#endif
 #ifndef PAIR_MINB_FP64
 #define PAIR_MINB_FP64 5  // resident blocks per SM of the FP64 kernels (no virial, one image): 96 registers
 #endif
@@ -328,14 +331,14 @@ __device__ __forceinline__ void sw_apply2(const SwitchT<float> &w, float2 r2, fl
 }
 
 struct Acc2 {
-  float2 fi[3], fj[3], elj, ec, vir[6];
+  float2 fi[3], fj[3], elj, ec;
 };
 
 // HALF steps of one lane over its lane group's j-pairs; fi collects +f (the i-force is -fi).
 // sa: this lane's first entry of the packed staging positions (z, charges at + FAST_ENTRIES);
 // sty: its first entry of the packed types.  ALL: the LJ and Coulomb cutoffs both cover the pair
 // cutoff (the common case), so the pair mask is the only one (chosen per tile, not per step).
-template <int LSW, int CM, int CSW, bool VIR, bool ALL>
+template <int LSW, int CM, int CSW, bool ALL>
 __device__ __forceinline__ void tile_pairs2(const ParamsT<float> &p, const float2 *__restrict__ ljab,
                                             int tio, const float4 *sa, const int2 *sty, int nxt,
                                             float xi, float yi, float zi, float qi, Acc2 &a) {
@@ -394,11 +397,6 @@ __device__ __forceinline__ void tile_pairs2(const ParamsT<float> &p, const float
       fs = add2(fs, f);
     }
     const float2 fx = mul2(dx, fs), fy = mul2(dy, fs), fz = mul2(dz, fs);
-    if constexpr (VIR) {
-      a.vir[0] = fma2(fx, dx, a.vir[0]); a.vir[1] = fma2(fx, dy, a.vir[1]);
-      a.vir[2] = fma2(fx, dz, a.vir[2]); a.vir[3] = fma2(fy, dy, a.vir[3]);
-      a.vir[4] = fma2(fy, dz, a.vir[4]); a.vir[5] = fma2(fz, dz, a.vir[5]);
-    }
     a.fi[0] = add2(a.fi[0], fx); a.fi[1] = add2(a.fi[1], fy); a.fi[2] = add2(a.fi[2], fz);
     a.fj[0] = add2(a.fj[0], fx); a.fj[1] = add2(a.fj[1], fy); a.fj[2] = add2(a.fj[2], fz);
     // rotate both j-force accumulators inside the lane group
@@ -437,7 +435,7 @@ constexpr size_t warp_pref_bytes() {
 }
 
 template <bool MIXED, int LSW, int CM, int CSW, bool VIR, bool MULTI>
-__global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !VIR && !MULTI) ? PAIR_MINB : (!MIXED && !VIR && !MULTI) ? PAIR_MINB_FP64 : 2)
+__global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !MULTI) ? (VIR ? PAIR_MINB_VIR : PAIR_MINB) : (!MIXED && !VIR && !MULTI) ? PAIR_MINB_FP64 : 2)
     k_pair(SystemDev s, NbListDev nb, PairParams p,
            ParamsT<typename std::conditional<MIXED, float, double>::type> pt, const double *ljd,
            const double *lat, int unit_kinds, int wslot) {
@@ -474,7 +472,17 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !VIR && !MULTI) ? PAIR
   // energies (and virials) per lane: summed in the arithmetic type over CLOSE_TILES tiles, then
   // added in fixed point to this lane's slots in shared memory; summed over the warp and added to
   // the box accumulators when the box changes
-  T el_acc = T(0), ec_acc = T(0), v_acc[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
+  T el_acc = T(0), ec_acc = T(0);
+  // Virial sum f (x) d over the pairs of a tile whose coordinates need no wrap, d = r_j - r_i: the
+  // same as sum F_j (x) r_j + sum F_i (x) r_i with the tile's summed forces, six FP64 products
+  // per atom and tile for six FP32 ones per pair, and 128 registers for 162 (4 CTAs per SM for 3).
+  // LJ C2 + Coulomb C1 of 36,000 atoms: 134 -> 88 us, with an instance of its own.  Wrapped tiles
+  // sum per pair.
+  double v_acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  auto add_virial = [&](T fx, T fy, T fz, T x, T y, T z) {
+    v_acc[0] += (double)fx * (double)x; v_acc[1] += (double)fx * (double)y; v_acc[2] += (double)fx * (double)z;
+    v_acc[3] += (double)fy * (double)y; v_acc[4] += (double)fy * (double)z; v_acc[5] += (double)fz * (double)z;
+  };
   constexpr int NE = VIR ? 8 : 2;
   // [NE + 3][32]: the energies and virial, then the i-forces of the current cluster
   long long *wsum = reinterpret_cast<long long *>(
@@ -500,12 +508,10 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !VIR && !MULTI) ? PAIR
 #pragma unroll
   for (int c = 0; c < 3; c++) a2p.fi[c] = a2p.fj[c] = sp2(0.f);
   a2p.elj = a2p.ec = sp2(0.f);
-#pragma unroll
-  for (int c = 0; c < 6; c++) a2p.vir[c] = sp2(0.f);
   // (FP64: one rounding for the warp, below what the 32 of its lanes would add up to)
-  auto add_fixed = [&](int c, T v) {
+  auto add_fixed = [&](int c, auto v) {
     if constexpr (MIXED) {
-      wsum[c * 32 + lane] += f2fix(v, (T)ENERGY_SCALE);
+      wsum[c * 32 + lane] += f2fix(v, decltype(v)(ENERGY_SCALE));
     } else {
       const double w = warp_sum(v);
       if (lane == 0) wsum[c * 32] += f2fix(w, ENERGY_SCALE);
@@ -523,6 +529,8 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !VIR && !MULTI) ? PAIR
       fi_acc[c] = T(0);
       a2p.fi[c] = sp2(0.f);
     }
+    if constexpr (VIR && MIXED)
+      if (!wrap) add_virial(f[0], f[1], f[2], xi, yi, zi);
     if constexpr (!MIXED) {  // one rounding for the cluster's lane groups instead of four
 #pragma unroll
       for (int o = BLOCK; o < 32; o <<= 1)
@@ -536,13 +544,6 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !VIR && !MULTI) ? PAIR
       el_acc += a2p.elj.x + a2p.elj.y;
       ec_acc += a2p.ec.x + a2p.ec.y;
       a2p.elj = a2p.ec = sp2(0.f);
-      if constexpr (VIR) {
-#pragma unroll
-        for (int c = 0; c < 6; c++) {
-          v_acc[c] += a2p.vir[c].x + a2p.vir[c].y;
-          a2p.vir[c] = sp2(0.f);
-        }
-      }
     }
     add_fixed(0, el_acc);
     add_fixed(1, ec_acc);
@@ -551,7 +552,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !VIR && !MULTI) ? PAIR
 #pragma unroll
       for (int c = 0; c < 6; c++) {
         add_fixed(2 + c, v_acc[c]);
-        v_acc[c] = T(0);
+        v_acc[c] = 0.0;
       }
     }
   };
@@ -753,10 +754,10 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !VIR && !MULTI) ? PAIR
 #pragma unroll
           for (int c = 0; c < 3; c++) a2p.fj[c] = sp2(0.f);
           if (pt.lj_all && pt.coul_all)
-            tile_pairs2<LSW, CM, CSW, VIR, true>(pt, reinterpret_cast<const float2 *>(ljab), tio, qa, qt, nxt, xi,
+            tile_pairs2<LSW, CM, CSW, true>(pt, reinterpret_cast<const float2 *>(ljab), tio, qa, qt, nxt, xi,
                                                  yi, zi, qi, a2p);
           else
-            tile_pairs2<LSW, CM, CSW, VIR, false>(pt, reinterpret_cast<const float2 *>(ljab), tio, qa, qt, nxt,
+            tile_pairs2<LSW, CM, CSW, false>(pt, reinterpret_cast<const float2 *>(ljab), tio, qa, qt, nxt,
                                                   xi, yi, zi, qi, a2p);
           // after HALF rotations: .y holds this lane's j-atom, .x that of the lane HALF away
 #pragma unroll
@@ -812,7 +813,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !VIR && !MULTI) ? PAIR
             else ab = T2{T(0), T(0)};
             T fs = pair_force<MIXED, LSW, CM, CSW>(pt, in, ex, r2, qi * T(dj.p.w), ab, a);
             T fx = dx * fs, fy = dy * fs, fz = dz * fs;
-            if constexpr (VIR) {
+            if constexpr (VIR && WRAP) {
               a.vir[0] += fx * dx; a.vir[1] += fx * dy; a.vir[2] += fx * dz;
               a.vir[3] += fy * dy; a.vir[4] += fy * dz; a.vir[5] += fz * dz;
             }
@@ -871,8 +872,13 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !VIR && !MULTI) ? PAIR
         el_acc += a.elj;
         ec_acc += a.ec;
         if constexpr (VIR)
-          for (int c = 0; c < 6; c++) v_acc[c] += a.vir[c];
+          if (wrap)
+#pragma unroll
+            for (int c = 0; c < 6; c++) v_acc[c] += a.vir[c];
       }
+      // (an own atom's j-side force joins its i-side force below)
+      if constexpr (VIR && MIXED)
+        if (!wrap && !(diag && gb == 0)) add_virial(tfj[0], tfj[1], tfj[2], mine.p.x, mine.p.y, mine.p.z);
 
       if (diag && gb == 0) {  // own atom li: its j-side force joins its i-side force
 #pragma unroll
@@ -943,9 +949,10 @@ template <bool MIXED, bool VIR>
 int launch_v(const SystemDev &s, const NbListDev &nb, const PairLaunch &pl, cudaStream_t st) {
   const PairParams &p = pl.p;
   const int lk = p.do_lj ? p.lj_sw.kind : NONE, ck = p.coul_sw.kind;
-  // specialised force sets: LJ C2 + Ewald real (cutoff), LJ C2 + Coulomb C2, LJ C2 alone,
+  // specialised force sets: LJ C2 + Ewald real (cutoff), LJ C2 + Coulomb C1 or C2, LJ C2 alone,
   // Ewald real alone
   if (lk == SW_C2 && p.coul_mode == 2 && ck == SW_CUTOFF) return launch_t<MIXED, SW_C2, 2, SW_CUTOFF, VIR>(s, nb, pl, st);
+  if (lk == SW_C2 && p.coul_mode == 1 && ck == SW_C1) return launch_t<MIXED, SW_C2, 1, SW_C1, VIR>(s, nb, pl, st);
   if (lk == SW_C2 && p.coul_mode == 1 && ck == SW_C2) return launch_t<MIXED, SW_C2, 1, SW_C2, VIR>(s, nb, pl, st);
   if (lk == SW_C2 && p.coul_mode == 0) return launch_t<MIXED, SW_C2, 0, SW_CUTOFF, VIR>(s, nb, pl, st);
   if (lk == NONE && p.coul_mode == 2 && ck == SW_CUTOFF) return launch_t<MIXED, NONE, 2, SW_CUTOFF, VIR>(s, nb, pl, st);
