@@ -1335,6 +1335,17 @@ pmb_force *pmb_force_create(pmb_system *s, const pmb_force_desc *d) {
     const int lcap = pme_line_capacity();
     int zbuf = 1, lbuf = 1;
     std::vector<double> theta;
+    // the plane kernel takes every plan whose planes fit shared memory
+    std::vector<int2> pwork;
+    std::vector<int> pradix, perm;
+    size_t psmem = 0;
+    double plane_points = 0.0;
+    for (int bi = 0; bi < nbox; bi++) {
+      const int nx = d->box_grids ? d->box_grids[3 * bi] : d->grid[0], ny = d->box_grids ? d->box_grids[3 * bi + 1] : d->grid[1];
+      if (nx > 0 && ny > 0) psmem = std::max(psmem, pme_plane_smem(nx, ny, s->precision));
+      plane_points += (double)nx * ny / nbox;
+    }
+    const bool planes = psmem <= (size_t)PLANE_SMEM_MAX;
     double th0[8];
     bspline_h(P, 0.0, th0);
     for (int bi = 0; bi < nbox; bi++) {
@@ -1358,6 +1369,26 @@ pmb_force *pmb_force_create(pmb_system *s, const pmb_force_desc *d) {
         pl.rad0[k] = (int)radix.size();
         pl.nrad[k] = (int)rad.size();
         radix.insert(radix.end(), rad.begin(), rad.end());
+        // the index at each position of the plane kernel's transformed line: position
+        // k0 n / R0 + k1 n / (R0 R1) + .. holds index k0 + R0 k1 + ..
+        perm.resize(tw.size());
+        for (int j = 0; j < n; j++) perm[pl.tw0[k] + j] = j;
+        std::vector<int> pr;
+        if (planes && k < 2 && pme_plane_radices(n, pr)) {
+          pl.prad0[k] = (int)pradix.size();
+          pl.npr[k] = (int)pr.size();
+          pradix.insert(pradix.end(), pr.begin(), pr.end());
+          for (int pos = 0; pos < n; pos++) {
+            int rest = pos, m = n, idx = 0, mul = 1;
+            for (int R : pr) {
+              m /= R;
+              idx += mul * (rest / m);
+              rest %= m;
+              mul *= R;
+            }
+            perm[pl.tw0[k] + pos] = idx;
+          }
+        }
         // influence factor B(m) exp(-pi^2 m^2/alpha^2) (Grid.h:523-571, dftmod :588-600)
         pl.inf0[k] = (int)infl.size();
         double fac = M_PI * M_PI / (f->alpha * f->alpha);
@@ -1393,6 +1424,10 @@ pmb_force *pmb_force_create(pmb_system *s, const pmb_force_desc *d) {
                 cols = std::max(1, std::min(PME_XCOLS, lcap / pl.n[0]));
       lbuf = std::max(lbuf, std::max(rows * pl.n[1], cols * pl.n[0]));
       for (int kz = 0; kz <= pl.n[2] / 2; kz++) {
+        if (planes) {
+          pwork.push_back(make_int2(bi, kz));
+          continue;
+        }
         for (int x0 = 0; x0 < pl.n[0]; x0 += rows) ywork.push_back(make_int4(bi, kz, x0, std::min(rows, pl.n[0] - x0)));
         for (int y0 = 0; y0 < pl.n[1]; y0 += cols) xwork.push_back(make_int4(bi, kz, y0, std::min(cols, pl.n[1] - y0)));
       }
@@ -1403,8 +1438,9 @@ pmb_force *pmb_force_create(pmb_system *s, const pmb_force_desc *d) {
         const double *bx = infl.data() + pl.inf0[0], *by = infl.data() + pl.inf0[1],
                      *bz = infl.data() + pl.inf0[2];
         for (int kz = 0; kz < nh; kz++)
-          for (int i = 0; i < nx; i++)
-            for (int j = 0; j < ny; j++) {
+          for (int pi = 0; pi < nx; pi++)
+            for (int pj = 0; pj < ny; pj++) {
+              const int i = planes ? perm[pl.tw0[0] + pi] : pi, j = planes ? perm[pl.tw0[1] + pj] : pj;
               double th = 0.0;
               if (i || j || kz) {
                 const int i0 = i <= nx / 2 ? i : i - nx, j0 = j <= ny / 2 ? j : j - ny;
@@ -1448,6 +1484,18 @@ pmb_force *pmb_force_create(pmb_system *s, const pmb_force_desc *d) {
     rc |= upload(f->a, dz, zwork);
     rc |= upload(f->a, dy, ywork);
     rc |= upload(f->a, dx, xwork);
+    int2 *dpw;
+    int *dpr, *dperm;
+    rc |= upload(f->a, dpw, pwork);
+    rc |= upload(f->a, dpr, pradix);
+    rc |= upload(f->a, dperm, perm);
+    pm.pwork = dpw;
+    pm.npwork = (int)pwork.size();
+    pm.pradix = dpr;
+    pm.perm = dperm;
+    pm.psmem = psmem;
+    // threads for about one butterfly each in a stage of radix 4 or 5, up to PLANE_MAX_THREADS
+    pm.pthreads = std::max(64, std::min(PLANE_MAX_THREADS, ((int)(plane_points / 4) + 63) / 64 * 64));
     pm.plan = dplan;
     pm.twiddle = dtw;
     pm.twiddlef = dtwf;

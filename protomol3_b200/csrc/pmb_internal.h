@@ -154,6 +154,7 @@ struct PmeBoxPlan {
   int tw0[3];         // offsets of twiddle tables (complex elements)
   int inf0[3];        // offsets of influence tables
   int rad0[3], nrad[3];
+  int prad0[2], npr[2];  // radices of the plane kernel's x and y transforms
   double hr[3];       // n / L
   double mr[3];       // 1 / L
   double piVr, fac;   // 1/(pi V), pi^2 / alpha^2
@@ -177,6 +178,12 @@ struct PmeDev {
   int nywork;
   const int4 *xwork;          // x-line work items: box, kz, y0, columns
   int nxwork;
+  const int2 *pwork;          // planes of the plane kernel: box, kz (npwork 0: it is not used)
+  int npwork, pthreads;
+  size_t psmem;
+  const int *pradix;          // its radices
+  const int *perm;            // index at each position of its transformed lines (offsets tw0); theta
+                              // is in that order then
   int zbuf, lbuf;             // complex elements per ping-pong buffer of the z / line kernels
   int wz, wy, wx;             // R > 0: every box's z (y, x) lines have 32 R points and the inverse
                               // z pass (the y passes, the x pass) run the warp-shuffle transforms;
@@ -193,6 +200,11 @@ typedef void (*StageMark)(void *ctx, const char *stage);
 int pme_recip_launch(const SystemDev &s, const NbListDev &nb, const PmeDev &pm, cudaStream_t st,
                      StageMark mark = nullptr, void *mark_ctx = nullptr);
 int pme_line_capacity();
+// Plane kernel: most threads, most shared memory, the stages of a line, a plane's shared memory.
+constexpr int PLANE_MAX_THREADS = 512;
+constexpr int PLANE_SMEM_MAX = 227 * 1024;
+bool pme_plane_radices(int n, std::vector<int> &radices);
+size_t pme_plane_smem(int nx, int ny, int precision);
 // Exact Ewald reciprocal sum of one box (pmb_ewald.cu): S, C [nk] and the box's forces in fout.
 int ewald_recip_launch(const double *pos, const double *charge, int atom0, int n, const double3 *kv,
                        const double *a, int nk, double *S, double *Cc, double *fout, cudaStream_t st);

@@ -9,15 +9,15 @@
 //                 threads per slot, one x-plane of the stencil each)
 //   k_fft_z_fwd   z-lines of the fixed-point grid (cleared as it is read), two real lines packed
 //                 per complex FFT, half spectrum written as [kz][x][y]
-//   k_fft_y       y-lines of the half spectrum (groups of up to 16 rows of one kz plane)
-//   k_fft_x_infl  x-lines (groups of up to 16 columns): forward FFT, influence function multiply
-//                 with energy and virial partials added to the box accumulators, inverse FFT
-//   k_fft_y       inverse y-lines
+//   k_fft_plane   per kz plane, in shared memory: y- and x-lines forward, influence function
+//                 multiply with energy and virial partials added to the box accumulators, x- and
+//                 y-lines inverse (planes too large for that: k_fft_y, k_fft_x_infl, k_fft_y)
 //   k_fft_z_inv   inverse z transform back to the real potential grid [x][y][z]
 //   k_gather      one thread per atom slot, 64-point stencil, fixed-point force atomics
 // The transforms are unnormalised, as the reference's ZFFT/FFTW calls; r2c/c2r replace the
 // reference's full complex transform of a real grid (identical result: the spectrum is Hermitian
 // and the influence function even in m).
+#include <functional>
 #include <type_traits>
 
 #include "pmb_internal.h"
@@ -880,6 +880,328 @@ __global__ void __launch_bounds__(WX, 3) k_fft_x_warp(const SystemDev s, PmeDev 
   }
 }
 
+// ------------------------------------------------------------ plane transform (y, x, x, y)
+// Composite DFTs in registers: R = R1 R2 points, index n = R2 n1 + n2 -> k = k1 + R1 k2.
+// cos and sin of 2 pi k / N for the inner factors (N, k constant after unrolling).
+__device__ __forceinline__ double2 unit_root(int N, int k) {
+  switch (N * 16 + k) {
+    case 97: return make_double2(0.50000000000000011, 0.8660254037844386);
+    case 98: return make_double2(-0.49999999999999978, 0.86602540378443871);
+    case 100: return make_double2(-0.50000000000000044, -0.86602540378443837);
+    case 101: return make_double2(0.50000000000000011, -0.8660254037844386);
+    case 129: return make_double2(0.70710678118654757, 0.70710678118654746);
+    case 131: return make_double2(-0.70710678118654746, 0.70710678118654757);
+    case 133: return make_double2(-0.70710678118654768, -0.70710678118654746);
+    case 135: return make_double2(0.70710678118654735, -0.70710678118654768);
+    case 145: return make_double2(0.76604444311897801, 0.64278760968653925);
+    case 146: return make_double2(0.17364817766693041, 0.98480775301220802);
+    case 147: return make_double2(-0.49999999999999978, 0.86602540378443871);
+    case 148: return make_double2(-0.93969262078590832, 0.34202014332566888);
+    case 149: return make_double2(-0.93969262078590843, -0.34202014332566866);
+    case 150: return make_double2(-0.50000000000000044, -0.86602540378443837);
+    case 151: return make_double2(0.17364817766692997, -0.98480775301220813);
+    case 152: return make_double2(0.76604444311897779, -0.64278760968653958);
+    case 161: return make_double2(0.80901699437494745, 0.58778525229247314);
+    case 162: return make_double2(0.30901699437494745, 0.95105651629515353);
+    case 163: return make_double2(-0.30901699437494734, 0.95105651629515364);
+    case 164: return make_double2(-0.80901699437494734, 0.58778525229247325);
+    case 166: return make_double2(-0.80901699437494756, -0.58778525229247303);
+    case 167: return make_double2(-0.30901699437494756, -0.95105651629515353);
+    case 168: return make_double2(0.30901699437494723, -0.95105651629515364);
+    case 169: return make_double2(0.80901699437494734, -0.58778525229247336);
+    case 193: return make_double2(0.86602540378443871, 0.49999999999999994);
+    case 194: return make_double2(0.50000000000000011, 0.8660254037844386);
+    case 196: return make_double2(-0.49999999999999978, 0.86602540378443871);
+    case 197: return make_double2(-0.86602540378443871, 0.49999999999999994);
+    case 199: return make_double2(-0.86602540378443882, -0.49999999999999972);
+    case 200: return make_double2(-0.50000000000000044, -0.86602540378443837);
+    case 202: return make_double2(0.50000000000000011, -0.8660254037844386);
+    case 203: return make_double2(0.86602540378443837, -0.50000000000000044);
+    default: return make_double2(0.0, 0.0);
+  }
+}
+// a exp(SIGN 2 pi i k / N)
+template <int SIGN, typename T2>
+__device__ __forceinline__ T2 mul_root(T2 a, int N, int k) {
+  using S = decltype(a.x);
+  if (k == 0) return a;
+  if (2 * k == N) return cmk(-a.x, -a.y);
+  if (4 * k == N) return cis(a, SIGN);
+  if (4 * k == 3 * N) return cis(a, -SIGN);
+  const double2 w = unit_root(N, k);
+  const S c = (S)w.x, s = (S)(SIGN * w.y);
+  return cmk(a.x * c - a.y * s, a.x * s + a.y * c);
+}
+template <int R1, int R2, int SIGN, typename T2>
+__device__ __forceinline__ void dft_composite(T2 *v) {
+  T2 a[R1 * R2];
+#pragma unroll
+  for (int n2 = 0; n2 < R2; n2++) {
+    T2 t[R1];
+#pragma unroll
+    for (int n1 = 0; n1 < R1; n1++) t[n1] = v[R2 * n1 + n2];
+    dft_small<R1>(t, SIGN);
+#pragma unroll
+    for (int k1 = 0; k1 < R1; k1++) a[k1 * R2 + n2] = mul_root<SIGN>(t[k1], R1 * R2, n2 * k1);
+  }
+#pragma unroll
+  for (int k1 = 0; k1 < R1; k1++) {
+    dft_small<R2>(a + k1 * R2, SIGN);
+#pragma unroll
+    for (int k2 = 0; k2 < R2; k2++) v[k1 + R1 * k2] = a[k1 * R2 + k2];
+  }
+}
+template <int R, int SIGN, typename T2>
+__device__ __forceinline__ void dft_reg(T2 *v) {
+  if constexpr (R <= 5) dft_small_any<R>(v, SIGN);
+  else if constexpr (R == 6) dft_composite<2, 3, SIGN>(v);
+  else if constexpr (R == 8) dft_composite<2, 4, SIGN>(v);
+  else if constexpr (R == 9) dft_composite<3, 3, SIGN>(v);
+  else if constexpr (R == 10) dft_composite<2, 5, SIGN>(v);
+  else dft_composite<3, 4, SIGN>(v);
+}
+
+// One in-place stage of a length-n transform on sub-blocks of m = R mq points, butterfly (b, j):
+// the R points b m + j + r mq.  Forward (decimation in frequency): DFT, then the factors W_m^(j k)
+// on output k; inverse: the conjugate factors on input k, then the DFT.  After the forward stages
+// R0, R1, .. output k = k0 + R0 k1 + .. sits at k0 n / R0 + k1 n / (R0 R1) + ..; the inverse stages
+// in reverse order take it from there.  tw: W_n^k; ts = n / m.
+template <int R, int SIGN, typename T2>
+__device__ __forceinline__ void stage_math(T2 *v, const T2 *tw, int j, int ts) {
+  if constexpr (SIGN < 0) {
+    dft_reg<R, SIGN>(v);
+#pragma unroll
+    for (int k = 1; k < R; k++) v[k] = cmul(v[k], tw[j * k * ts]);
+  } else {
+#pragma unroll
+    for (int k = 1; k < R; k++) {
+      const T2 w = tw[j * k * ts];
+      v[k] = cmk(v[k].x * w.x + v[k].y * w.y, v[k].y * w.x - v[k].x * w.y);
+    }
+    dft_reg<R, SIGN>(v);
+  }
+}
+
+// What one plane's transform works on.
+template <typename T2>
+struct PlaneCtx {
+  T2 *buf;        // [nx][ld]
+  const T2 *twx, *twy;
+  T2 *C;          // the plane in memory, [nx][ny]
+  int nx, ny, ld;
+};
+
+// Rows (y).  The outermost stage (m = ny) reads (forward) or writes (inverse) the plane in memory
+// instead of the buffer, consecutive threads along the row; the others run consecutive threads
+// down the rows (the odd row stride keeps them on different banks).
+template <int R, int SIGN, bool OUTER, typename T2>
+__device__ __forceinline__ void row_stage(const PlaneCtx<T2> &p, int m) {
+  const int mq = m / R, ts = p.ny / m, total = p.nx * (p.ny / R);
+  const float rq = rcpf(mq), rnx = rcpf(p.nx);
+  for (int e = threadIdx.x; e < total; e += blockDim.x) {
+    int row, b, j;
+    if constexpr (OUTER) {
+      row = divf(e, rq);
+      j = e - row * mq;
+      b = 0;
+    } else {
+      const int q = divf(e, rnx);
+      row = e - q * p.nx;
+      b = divf(q, rq);
+      j = q - b * mq;
+    }
+    T2 *L = p.buf + row * p.ld + b * m + j;
+    T2 *G = p.C + (long long)row * p.ny + j;
+    T2 v[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) v[r] = OUTER && SIGN < 0 ? G[r * mq] : L[r * mq];
+    stage_math<R, SIGN>(v, p.twy, j, ts);
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      if (OUTER && SIGN > 0) G[r * mq] = v[r];
+      else L[r * mq] = v[r];
+    }
+  }
+}
+// Columns (x), consecutive threads along a row.
+template <int R, int SIGN, typename T2>
+__device__ __forceinline__ void col_stage(const PlaneCtx<T2> &p, int m) {
+  const int mq = m / R, ts = p.nx / m, total = p.ny * (p.nx / R);
+  const float rq = rcpf(mq), rny = rcpf(p.ny);
+  for (int e = threadIdx.x; e < total; e += blockDim.x) {
+    const int q = divf(e, rny), c = e - q * p.ny, b = divf(q, rq), j = q - b * mq;
+    T2 *L = p.buf + (b * m + j) * p.ld + c;
+    const int st = mq * p.ld;
+    T2 v[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) v[r] = L[r * st];
+    stage_math<R, SIGN>(v, p.twx, j, ts);
+#pragma unroll
+    for (int r = 0; r < R; r++) L[r * st] = v[r];
+  }
+}
+// Energy and virial sums of the influence function (as k_fft_x_infl).
+struct InflSums {
+  double en = 0, xx = 0, xy = 0, xz = 0, yy = 0, yz = 0, zz = 0;
+};
+// The columns' last forward stage, the influence function and their first inverse stage, in
+// registers (m = R: no factors).  th: the plane's influence function in the order of the buffer;
+// mx, my: the reciprocal vectors' components by buffer position (virial).
+template <int R, bool VIR, typename T, typename T2>
+__device__ __forceinline__ void col_infl(const PlaneCtx<T2> &p, const T *th, double wz, const double *mx, const double *my,
+                                         double mk, double fac, InflSums &s) {
+  const int total = p.ny * (p.nx / R);
+  const float rny = rcpf(p.ny);
+  for (int e = threadIdx.x; e < total; e += blockDim.x) {
+    const int b = divf(e, rny), c = e - b * p.ny;
+    T2 *L = p.buf + b * R * p.ld + c;
+    T2 v[R];
+    T t[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) t[r] = th[(b * R + r) * p.ny + c];
+#pragma unroll
+    for (int r = 0; r < R; r++) v[r] = L[r * p.ld];
+    dft_reg<R, -1>(v);
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      const double ee = wz * ((double)v[r].x * (double)v[r].x + (double)v[r].y * (double)v[r].y) * (double)t[r];
+      s.en += ee;
+      if constexpr (VIR)
+        if (t[r] != T(0)) {
+          const double mi = mx[b * R + r], mj = my[c];
+          const double vv = 2.0 * (1.0 / (mi * mi + mj * mj + mk * mk) + fac);
+          s.xx += ee * (1.0 - vv * mi * mi); s.xy -= ee * (vv * mi * mj); s.xz -= ee * (vv * mi * mk);
+          s.yy += ee * (1.0 - vv * mj * mj); s.yz -= ee * (vv * mj * mk); s.zz += ee * (1.0 - vv * mk * mk);
+        }
+      v[r] = cmk(v[r].x * t[r], v[r].y * t[r]);
+    }
+    dft_reg<R, +1>(v);
+#pragma unroll
+    for (int r = 0; r < R; r++) L[r * p.ld] = v[r];
+  }
+}
+
+#define PLANE_RADIX(R, CALL) \
+  switch (R) {               \
+    case 2: CALL(2); break;  \
+    case 3: CALL(3); break;  \
+    case 4: CALL(4); break;  \
+    case 5: CALL(5); break;  \
+    case 6: CALL(6); break;  \
+    case 8: CALL(8); break;  \
+    case 9: CALL(9); break;  \
+    case 10: CALL(10); break; \
+    default: CALL(12); break; \
+  }
+
+// One kz plane of the half spectrum per CTA, in shared memory between its two passes over memory:
+// forward y and x transforms, influence function with energy and virial (Grid.h:236-341), inverse x
+// and y.  Two or three register stages a direction (96 = 8 x 12), so about seven barriers; the
+// three kernels before it had four or five each way and moved the spectrum through memory six
+// times.  Few CTAs (49 at 96^3) of long latency, which suits running beside the pair kernel: alone
+// 20 -> 13 us at 72^3, 36 -> 31 us at 125^3, 12 -> 8 us at 20^3, and two launches fewer.
+template <typename T, bool VIR>
+__global__ void __launch_bounds__(PLANE_MAX_THREADS) k_fft_plane(const SystemDev s, PmeDev pm) {
+  using T2 = typename C2<T>::t;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int2 wk = pm.pwork[blockIdx.x];  // box, kz
+  const PmeBoxPlan &pl = pm.plan[wk.x];
+  const int nx = pl.n[0], ny = pl.n[1], nz = pl.n[2], kz = wk.y;
+  double *red = reinterpret_cast<double *>(smem_raw);  // 32 doubles
+  double *mx = red + 32, *my = mx + (VIR ? nx : 0);
+  T2 *twx = reinterpret_cast<T2 *>(my + (VIR ? ny + (nx + ny) % 2 : 0)), *twy = twx + nx;
+  PlaneCtx<T2> p;
+  p.buf = twy + ny;
+  p.twx = twx;
+  p.twy = twy;
+  p.C = reinterpret_cast<T2 *>(pm.cgrid) + pl.cgrid0 + (long long)kz * nx * ny;
+  p.nx = nx;
+  p.ny = ny;
+  p.ld = ny | 1;
+  for (int k = threadIdx.x; k < nx + ny; k += blockDim.x) {
+    const int at = k < nx ? pl.tw0[0] + k : pl.tw0[1] + k - nx;
+    if constexpr (sizeof(T) == 4) twx[k] = pm.twiddlef[at];
+    else twx[k] = pm.twiddle[at];
+    if constexpr (VIR) {  // components of the vector at buffer position k
+      const int d = k < nx ? 0 : 1, n = pl.n[d], i = pm.perm[at];
+      mx[k] = (i <= n / 2 ? i : i - n) * pl.mr[d];
+    }
+  }
+  __syncthreads();
+  const int *rx = pm.pradix + pl.prad0[0], *ry = pm.pradix + pl.prad0[1];
+  const int sx = pl.npr[0], sy = pl.npr[1];
+  int m = ny;
+#define ROW_FIRST(R) row_stage<R, -1, true>(p, m)
+  PLANE_RADIX(ry[0], ROW_FIRST)
+  m /= ry[0];
+  __syncthreads();
+  for (int q = 1; q < sy; q++) {
+#define ROW_FWD(R) row_stage<R, -1, false>(p, m)
+    PLANE_RADIX(ry[q], ROW_FWD)
+    m /= ry[q];
+    __syncthreads();
+  }
+  m = nx;
+  for (int q = 0; q + 1 < sx; q++) {
+#define COL_FWD(R) col_stage<R, -1>(p, m)
+    PLANE_RADIX(rx[q], COL_FWD)
+    m /= rx[q];
+    __syncthreads();
+  }
+  InflSums sum;
+  {
+    const T *th = reinterpret_cast<const T *>(pm.theta) + pl.cgrid0 + (long long)kz * nx * ny;
+    const double wz = (kz > 0 && ((2 * kz != nz) || (nz & 1))) ? 2.0 : 1.0;
+#define COL_INFL(R) col_infl<R, VIR, T>(p, th, wz, mx, my, kz * pl.mr[2], pl.fac, sum)
+    PLANE_RADIX(rx[sx - 1], COL_INFL)
+  }
+  __syncthreads();
+  for (int q = sx - 2; q >= 0; q--) {  // (m = rx[sx - 1] here)
+    m *= rx[q];
+#define COL_INV(R) col_stage<R, +1>(p, m)
+    PLANE_RADIX(rx[q], COL_INV)
+    __syncthreads();
+  }
+  m = 1;
+  for (int q = sy - 1; q > 0; q--) {
+    m *= ry[q];
+#define ROW_INV(R) row_stage<R, +1, false>(p, m)
+    PLANE_RADIX(ry[q], ROW_INV)
+    __syncthreads();
+  }
+#define ROW_LAST(R) row_stage<R, +1, true>(p, ny)
+  PLANE_RADIX(ry[0], ROW_LAST)
+#undef ROW_FIRST
+#undef ROW_FWD
+#undef COL_FWD
+#undef COL_INFL
+#undef COL_INV
+#undef ROW_INV
+#undef ROW_LAST
+  // the CTA's energy (x 0.5, Grid.h:319-337) and virial partials in fixed point, as k_fft_x_infl
+  const double part[7] = {sum.en, sum.xx, sum.xy, sum.xz, sum.yy, sum.yz, sum.zz};
+  long long *eb = s.eacc + (long long)wk.x * ACC_PER_BOX;
+  const int slot[6][2] = {{0, 0}, {1, 3}, {2, 6}, {4, 4}, {5, 7}, {8, 8}};  // xx xy xz yy yz zz
+#pragma unroll
+  for (int c = 0; c < (VIR ? 7 : 1); c++) {
+    const double w = warp_sum(part[c]);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = w;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double r = 0.0;
+      for (int k = 0; k < (int)(blockDim.x >> 5); k++) r += red[k];
+      const long long q = f2fix(r * 0.5, ENERGY_SCALE);
+      if (c == 0) {
+        red_add(eb + E_COUL, q);
+      } else {
+        red_add(eb + E_VIR + slot[c - 1][0], q);
+        if (slot[c - 1][1] != slot[c - 1][0]) red_add(eb + E_VIR + slot[c - 1][1], q);
+      }
+    }
+  }
+}
+
 constexpr int WZ = 128;  // threads of the warp z kernel: up to 8 lines (4 pairs) per work item
 
 // z-lines with n_z = 32 R, c2r (as k_fft_z_inv): the z_inv work item's lines (x, y0 .. y0 + cnt)
@@ -960,26 +1282,36 @@ int recip_t(const SystemDev &s, const NbListDev &nb, const PmeDev &pm, cudaStrea
     cudaFuncSetAttribute(k_fft_x_infl<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, lcap);
     lconf[dev] = true;
   }
-  auto fft_y = [&](int sign) {
-    switch (pm.wy) {
-      case 1: k_fft_y_warp<T, 1><<<pm.nywork, WT, 0, st>>>(pm, sign); break;
-      case 2: k_fft_y_warp<T, 2><<<pm.nywork, WT, 0, st>>>(pm, sign); break;
-      case 3: k_fft_y_warp<T, 3><<<pm.nywork, WT, 0, st>>>(pm, sign); break;
-      case 4: k_fft_y_warp<T, 4><<<pm.nywork, WT, 0, st>>>(pm, sign); break;
-      case 5: k_fft_y_warp<T, 5><<<pm.nywork, WT, 0, st>>>(pm, sign); break;
-      default: k_fft_y<T><<<pm.nywork, LT, lsmem, st>>>(pm, sign);
+  if (pm.npwork > 0) {  // y, x, influence, x, y of each kz plane in one kernel
+    static bool pconf[2][PMB_MAX_DEVICES] = {};  // per device
+    auto kern = pm.virial ? k_fft_plane<T, true> : k_fft_plane<T, false>;
+    if (!pconf[pm.virial != 0][dev]) {
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PLANE_SMEM_MAX);
+      pconf[pm.virial != 0][dev] = true;
     }
-  };
-  fft_y(-1);
-  switch (pm.wx) {
-    case 1: k_fft_x_warp<T, 1><<<pm.nxwork, WX, 0, st>>>(s, pm); break;
-    case 2: k_fft_x_warp<T, 2><<<pm.nxwork, WX, 0, st>>>(s, pm); break;
-    case 3: k_fft_x_warp<T, 3><<<pm.nxwork, WX, 0, st>>>(s, pm); break;
-    case 4: k_fft_x_warp<T, 4><<<pm.nxwork, WX, 0, st>>>(s, pm); break;
-    case 5: k_fft_x_warp<T, 5><<<pm.nxwork, WX, 0, st>>>(s, pm); break;
-    default: k_fft_x_infl<T><<<pm.nxwork, LT, lsmem, st>>>(s, pm);
+    kern<<<pm.npwork, pm.pthreads, pm.psmem, st>>>(s, pm);
+  } else {
+    auto fft_y = [&](int sign) {
+      switch (pm.wy) {
+        case 1: k_fft_y_warp<T, 1><<<pm.nywork, WT, 0, st>>>(pm, sign); break;
+        case 2: k_fft_y_warp<T, 2><<<pm.nywork, WT, 0, st>>>(pm, sign); break;
+        case 3: k_fft_y_warp<T, 3><<<pm.nywork, WT, 0, st>>>(pm, sign); break;
+        case 4: k_fft_y_warp<T, 4><<<pm.nywork, WT, 0, st>>>(pm, sign); break;
+        case 5: k_fft_y_warp<T, 5><<<pm.nywork, WT, 0, st>>>(pm, sign); break;
+        default: k_fft_y<T><<<pm.nywork, LT, lsmem, st>>>(pm, sign);
+      }
+    };
+    fft_y(-1);
+    switch (pm.wx) {
+      case 1: k_fft_x_warp<T, 1><<<pm.nxwork, WX, 0, st>>>(s, pm); break;
+      case 2: k_fft_x_warp<T, 2><<<pm.nxwork, WX, 0, st>>>(s, pm); break;
+      case 3: k_fft_x_warp<T, 3><<<pm.nxwork, WX, 0, st>>>(s, pm); break;
+      case 4: k_fft_x_warp<T, 4><<<pm.nxwork, WX, 0, st>>>(s, pm); break;
+      case 5: k_fft_x_warp<T, 5><<<pm.nxwork, WX, 0, st>>>(s, pm); break;
+      default: k_fft_x_infl<T><<<pm.nxwork, LT, lsmem, st>>>(s, pm);
+    }
+    fft_y(+1);
   }
-  fft_y(+1);
   switch (pm.wz) {
     case 1: k_fft_z_inv_warp<T, 1><<<pm.nzwork, WZ, 0, st>>>(pm); break;
     case 2: k_fft_z_inv_warp<T, 2><<<pm.nzwork, WZ, 0, st>>>(pm); break;
@@ -998,6 +1330,37 @@ int recip_t(const SystemDev &s, const NbListDev &nb, const PmeDev &pm, cudaStrea
 }  // namespace
 
 int pme_line_capacity() { return LMAXE; }
+
+bool pme_plane_radices(int n, std::vector<int> &rad) {
+  // the fewest stages, then the smallest sum of radices
+  static const int R[] = {12, 10, 9, 8, 6, 5, 4, 3, 2};
+  std::vector<int> best, cur;
+  int best_sum = 0;
+  std::function<void(int, int, int)> search = [&](int m, int from, int sum) {
+    if (m == 1) {
+      if (!cur.empty() && (best.empty() || cur.size() < best.size() || (cur.size() == best.size() && sum < best_sum))) {
+        best = cur;
+        best_sum = sum;
+      }
+      return;
+    }
+    if (!best.empty() && cur.size() >= best.size()) return;
+    for (int k = from; k < 9; k++)
+      if (m % R[k] == 0) {
+        cur.push_back(R[k]);
+        search(m / R[k], k, sum + R[k]);
+        cur.pop_back();
+      }
+  };
+  search(n, 0, 0);
+  rad = best;
+  return !best.empty();
+}
+
+size_t pme_plane_smem(int nx, int ny, int precision) {
+  const size_t c = precision ? sizeof(float2) : sizeof(double2);
+  return sizeof(double) * (32 + nx + ny + (nx + ny) % 2) + c * ((size_t)nx + ny + (size_t)nx * (ny | 1));
+}
 
 int pme_recip_launch(const SystemDev &s, const NbListDev &nb, const PmeDev &pm, cudaStream_t st,
                      StageMark mark, void *mctx) {
