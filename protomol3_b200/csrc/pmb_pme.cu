@@ -5,15 +5,15 @@
 // NonbondedPMEwaldSystemForce.h (reciprocalTerm :812-864, correctionTerm :874-911).
 //
 // Pipeline per step (every kernel batched over the boxes of a system):
-//   k_spread      B-spline weights, 64 int64 fixed-point atomics per atom slot (order 4: four
-//                 threads per slot, one x-plane of the stencil each)
+//   k_spread      B-spline weights, order^3 int64 fixed-point atomics per atom slot (two to eight
+//                 threads per slot, one z-offset of the stencil each)
 //   k_fft_z_fwd   z-lines of the fixed-point grid (cleared as it is read), two real lines packed
 //                 per complex FFT, half spectrum written as [kz][x][y]
 //   k_fft_plane   per kz plane, in shared memory: y- and x-lines forward, influence function
 //                 multiply with energy and virial partials added to the box accumulators, x- and
 //                 y-lines inverse (planes too large for that: k_fft_y, k_fft_x_infl, k_fft_y)
 //   k_fft_z_inv   inverse z transform back to the real potential grid [x][y][z]
-//   k_gather      one thread per atom slot, 64-point stencil, fixed-point force atomics
+//   k_gather      the same threads per atom slot, fixed-point force atomics
 // The transforms are unnormalised, as the reference's ZFFT/FFTW calls; r2c/c2r replace the
 // reference's full complex transform of a real grid (identical result: the spectrum is Hermitian
 // and the influence function even in m).
@@ -25,8 +25,6 @@
 namespace pmb {
 
 namespace {
-
-constexpr int MAXP = 8;  // largest supported interpolation order
 
 template <typename T>
 struct C2;
@@ -226,75 +224,20 @@ __device__ __forceinline__ int wrap3(int x, int n) {
   return x >= n ? x - n : x;
 }
 
-// PC > 0: interpolation order fixed at compile time (weights stay in registers); PC = 0: run time.
-template <bool MIXED, int PC>
-__global__ void k_spread(NbListDev nb, PmeDev pm) {
-  using T = typename std::conditional<MIXED, float, double>::type;
-  int sl = blockIdx.x * blockDim.x + threadIdx.x;
-  if (sl >= nb.nslot) return;
-  int4 m = nb.slot_meta[sl];
-  if (m.x < 0) return;
-  const PmeBoxPlan &pl = pm.plan[m.w];
-  const int P = PC > 0 ? PC : pm.order;
-  T th[3][MAXP];
-  int base[3];
-  T q;
-  if constexpr (MIXED) {
-    uint4 f = nb.slot_fx[sl];
-    unsigned fx[3] = {f.x, f.y, f.z};
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      T w;
-      grid_coord<true>(fx[d], 0.0, 0.0, pl.n[d], P, base[d], w);
-      bspline<T>(P, w, th[d], nullptr);
-    }
-    q = __uint_as_float(f.w);
-  } else {
-    double4 pq = nb.slot_pq[sl];
-    double x[3] = {pq.x, pq.y, pq.z};
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      T w;
-      grid_coord<false>(0u, x[d], pl.hr[d], pl.n[d], P, base[d], w);
-      bspline<T>(P, w, th[d], nullptr);
-    }
-    q = pq.w;
-  }
-  const int nx = pl.n[0], ny = pl.n[1], nz = pl.n[2];
-  long long *g = pm.qgrid + pl.grid0;
-  #pragma unroll
-  for (int i = 0; i < P; i++) {
-    T a = q * th[0][i];
-    int i1 = wrap3(i + base[0], nx);
-    #pragma unroll
-    for (int j = 0; j < P; j++) {
-      T ab = a * th[1][j];
-      int j1 = wrap3(j + base[1], ny);
-      long long *row = g + ((long long)i1 * ny + j1) * nz;
-      #pragma unroll
-      for (int k = 0; k < P; k++) {
-        int k1 = wrap3(k + base[2], nz);
-        long long v = f2fix(ab * th[2][k], (T)GRID_SCALE);
-        if (v) red_add(row + k1, v);
-      }
-    }
-  }
-}
-
-// B-spline weights and grid bases of one slot for order 4 (the common case).
-template <bool MIXED, bool DERIV>
-__device__ __forceinline__ void weights4(const PmeBoxPlan &pl, uint4 f, double4 pq,
-                                         typename std::conditional<MIXED, float, double>::type th[3][4],
-                                         typename std::conditional<MIXED, float, double>::type dth[3][4],
-                                         int base[3], typename std::conditional<MIXED, float, double>::type &q) {
+// B-spline weights and grid bases of one slot for order P (2, 4, 6 or 8).
+template <bool MIXED, int P, bool DERIV>
+__device__ __forceinline__ void slot_weights(const PmeBoxPlan &pl, uint4 f, double4 pq,
+                                             typename std::conditional<MIXED, float, double>::type th[3][P],
+                                             typename std::conditional<MIXED, float, double>::type dth[3][P],
+                                             int base[3], typename std::conditional<MIXED, float, double>::type &q) {
   using T = typename std::conditional<MIXED, float, double>::type;
   if constexpr (MIXED) {
     const unsigned fx[3] = {f.x, f.y, f.z};
 #pragma unroll
     for (int d = 0; d < 3; d++) {
       T w;
-      grid_coord<true>(fx[d], 0.0, 0.0, pl.n[d], 4, base[d], w);
-      bspline<T>(4, w, th[d], DERIV ? dth[d] : nullptr);
+      grid_coord<true>(fx[d], 0.0, 0.0, pl.n[d], P, base[d], w);
+      bspline<T>(P, w, th[d], DERIV ? dth[d] : nullptr);
     }
     q = __uint_as_float(f.w);
   } else {
@@ -302,30 +245,39 @@ __device__ __forceinline__ void weights4(const PmeBoxPlan &pl, uint4 f, double4 
 #pragma unroll
     for (int d = 0; d < 3; d++) {
       T w;
-      grid_coord<false>(0u, x[d], pl.hr[d], pl.n[d], 4, base[d], w);
-      bspline<T>(4, w, th[d], DERIV ? dth[d] : nullptr);
+      grid_coord<false>(0u, x[d], pl.hr[d], pl.n[d], P, base[d], w);
+      bspline<T>(P, w, th[d], DERIV ? dth[d] : nullptr);
     }
     q = pq.w;
   }
 }
 
-// v[p] for a run-time p in [0, 4) without indexing a register array (which would go to local
+// v[p] for a run-time p in [0, P) without indexing a register array (which would go to local
 // memory).
-template <typename T>
-__device__ __forceinline__ T pick4(const T v[4], int p) {
-  return p == 0 ? v[0] : (p == 1 ? v[1] : (p == 2 ? v[2] : v[3]));
+template <int P, typename T>
+__device__ __forceinline__ T pick(const T v[P], int p) {
+  T o = v[0];
+#pragma unroll
+  for (int k = 1; k < P; k++) o = p == k ? v[k] : o;
+  return o;
 }
 
-// Order 4 with four threads per atom slot: thread p adds the 16 points of z-offset p of the
-// stencil (the same values, in the same order of products, as the one-thread form), so that at
-// every step the slot's four threads add to four consecutive grid words (one or two 32-byte
-// sectors) rather than to four x-planes (four sectors).
-template <bool MIXED>
-__global__ void k_spread4(NbListDev nb, PmeDev pm) {
+// Threads of one atom slot: the order rounded up to a power of two.
+template <int P>
+constexpr int SLOT_THREADS = P <= 2 ? 2 : P <= 4 ? 4 : 8;
+
+// SLOT_THREADS threads per atom slot: thread p adds the P^2 points of z-offset p of the stencil,
+// so that at every step the slot's threads add to P consecutive grid words (one to three 32-byte
+// sectors).  Bound by the L2's atomics.  Orders above 4 ran one thread per slot, with the order
+// known at run time and the weights in local memory (19,200 atoms, order 6, FP64: 40 us, now 12; the
+// gather 43 us, now 17).
+template <bool MIXED, int P>
+__global__ void k_spread(NbListDev nb, PmeDev pm) {
   using T = typename std::conditional<MIXED, float, double>::type;
+  constexpr int W = SLOT_THREADS<P>;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int sl = (int)(t >> 2), p = (int)(t & 3);
-  if (sl >= nb.nslot) return;
+  const int sl = (int)(t / W), p = (int)(t % W);
+  if (sl >= nb.nslot || p >= P) return;
   // the slot's metadata and position are loaded together (one round trip)
   const int4 m = nb.slot_meta[sl];
   uint4 f4 = make_uint4(0, 0, 0, 0);
@@ -334,20 +286,20 @@ __global__ void k_spread4(NbListDev nb, PmeDev pm) {
   else p4 = nb.slot_pq[sl];
   if (m.x < 0) return;
   const PmeBoxPlan &pl = pm.plan[m.w];
-  T th[3][4];
+  T th[3][P];
   int base[3];
   T q;
-  weights4<MIXED, false>(pl, f4, p4, th, th, base, q);
+  slot_weights<MIXED, P, false>(pl, f4, p4, th, th, base, q);
   const int nx = pl.n[0], ny = pl.n[1], nz = pl.n[2];
   long long *g = pm.qgrid + pl.grid0;
-  const T c2 = pick4(th[2], p);
+  const T c2 = pick<P>(th[2], p);
   long long *col = g + wrap3(p + base[2], nz);
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
+  for (int i = 0; i < P; i++) {
     const T a = q * th[0][i];
     const int i1 = wrap3(i + base[0], nx);
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
+    for (int j = 0; j < P; j++) {
       const int j1 = wrap3(j + base[1], ny);
       const long long v = f2fix(a * th[1][j] * c2, (T)GRID_SCALE);
       if (v) red_add(col + ((long long)i1 * ny + j1) * nz, v);
@@ -355,78 +307,15 @@ __global__ void k_spread4(NbListDev nb, PmeDev pm) {
   }
 }
 
-template <bool MIXED, int PC>
+// The same threads read the stencil: thread p z-offset p, so that at every step the slot's threads
+// read P consecutive grid words; the partial forces are summed over the slot's lanes.  Every lane
+// takes part in the shuffles (slots out of range or padding, and lanes past the order, add zeros).
+template <bool MIXED, int P>
 __global__ void k_gather(const SystemDev s, NbListDev nb, PmeDev pm) {
   using T = typename std::conditional<MIXED, float, double>::type;
-  int sl = blockIdx.x * blockDim.x + threadIdx.x;
-  if (sl >= nb.nslot) return;
-  // the slot's metadata and position are loaded together (one round trip)
-  int4 m = nb.slot_meta[sl];
-  uint4 f4 = make_uint4(0, 0, 0, 0);
-  double4 pq = make_double4(0, 0, 0, 0);
-  if constexpr (MIXED) f4 = nb.slot_fx[sl];
-  else pq = nb.slot_pq[sl];
-  if (m.x < 0) return;
-  const PmeBoxPlan &pl = pm.plan[m.w];
-  const int P = PC > 0 ? PC : pm.order;
-  T th[3][MAXP], dth[3][MAXP];
-  int base[3];
-  T q;
-  if constexpr (MIXED) {
-    unsigned fx[3] = {f4.x, f4.y, f4.z};
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      T w;
-      grid_coord<true>(fx[d], 0.0, 0.0, pl.n[d], P, base[d], w);
-      bspline<T>(P, w, th[d], dth[d]);
-    }
-    q = __uint_as_float(f4.w);
-  } else {
-    double x[3] = {pq.x, pq.y, pq.z};
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      T w;
-      grid_coord<false>(0u, x[d], pl.hr[d], pl.n[d], P, base[d], w);
-      bspline<T>(P, w, th[d], dth[d]);
-    }
-    q = pq.w;
-  }
-  const int nx = pl.n[0], ny = pl.n[1], nz = pl.n[2];
-  const T *g = reinterpret_cast<const T *>(pm.rgrid) + pl.grid0;
-  T fx = 0, fy = 0, fz = 0;
-  #pragma unroll
-  for (int i = 0; i < P; i++) {
-    int i1 = wrap3(i + base[0], nx);
-    #pragma unroll
-    for (int j = 0; j < P; j++) {
-      int j1 = wrap3(j + base[1], ny);
-      T xij = dth[0][i] * th[1][j], yij = th[0][i] * dth[1][j], zij = th[0][i] * th[1][j];
-      const T *row = g + ((long long)i1 * ny + j1) * nz;
-      #pragma unroll
-      for (int k = 0; k < P; k++) {
-        int k1 = wrap3(k + base[2], nz);
-        T term = row[k1];
-        fx -= term * xij * th[2][k];
-        fy -= term * yij * th[2][k];
-        fz -= term * zij * dth[2][k];
-      }
-    }
-  }
-  long long *f = s.facc + 3 * (long long)m.x;
-  red_add(f, f2fix((double)(fx * T(pl.hr[0]) * q), FORCE_SCALE));
-  red_add(f + 1, f2fix((double)(fy * T(pl.hr[1]) * q), FORCE_SCALE));
-  red_add(f + 2, f2fix((double)(fz * T(pl.hr[2]) * q), FORCE_SCALE));
-}
-
-// Order 4 with four threads per atom slot: thread p reads z-offset p of the stencil, so that at
-// every step the slot's four threads read four consecutive grid words; the four partial forces
-// are summed over the slot's lanes.  Every lane takes part in the shuffles (slots out of range
-// or padding add zeros).
-template <bool MIXED>
-__global__ void k_gather4(const SystemDev s, NbListDev nb, PmeDev pm) {
-  using T = typename std::conditional<MIXED, float, double>::type;
+  constexpr int W = SLOT_THREADS<P>;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int sl = (int)(t >> 2), p = (int)(t & 3);
+  const int sl = (int)(t / W), p = (int)(t % W);
   const bool in = sl < nb.nslot;
   const int4 m = in ? nb.slot_meta[sl] : make_int4(-1, -1, 0, 0);
   uint4 f4 = make_uint4(0, 0, 0, 0);
@@ -438,18 +327,18 @@ __global__ void k_gather4(const SystemDev s, NbListDev nb, PmeDev pm) {
   const bool ok = m.x >= 0;
   T fx = 0, fy = 0, fz = 0, q = 0;
   const PmeBoxPlan *pl = ok ? pm.plan + m.w : nullptr;
-  if (ok) {
-    T th[3][4], dth[3][4];
+  if (ok && p < P) {
+    T th[3][P], dth[3][P];
     int base[3];
-    weights4<MIXED, true>(*pl, f4, pq, th, dth, base, q);
+    slot_weights<MIXED, P, true>(*pl, f4, pq, th, dth, base, q);
     const int nx = pl->n[0], ny = pl->n[1], nz = pl->n[2];
     const T *col = reinterpret_cast<const T *>(pm.rgrid) + pl->grid0 + wrap3(p + base[2], nz);
-    const T tz = pick4(th[2], p), dz = pick4(dth[2], p);
+    const T tz = pick<P>(th[2], p), dz = pick<P>(dth[2], p);
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
+    for (int i = 0; i < P; i++) {
       const int i1 = wrap3(i + base[0], nx);
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
+      for (int j = 0; j < P; j++) {
         const int j1 = wrap3(j + base[1], ny);
         const T xij = dth[0][i] * th[1][j], yij = th[0][i] * dth[1][j], zij = th[0][i] * th[1][j];
         const T term = col[((long long)i1 * ny + j1) * nz];
@@ -460,7 +349,7 @@ __global__ void k_gather4(const SystemDev s, NbListDev nb, PmeDev pm) {
     }
   }
 #pragma unroll
-  for (int o = 1; o < 4; o <<= 1) {
+  for (int o = 1; o < W; o <<= 1) {
     fx += __shfl_xor_sync(0xffffffffu, fx, o);
     fy += __shfl_xor_sync(0xffffffffu, fy, o);
     fz += __shfl_xor_sync(0xffffffffu, fz, o);
@@ -1260,9 +1149,13 @@ int recip_t(const SystemDev &s, const NbListDev &nb, const PmeDev &pm, cudaStrea
   using T2 = typename C2<T>::t;
   const int TB = 256;
   constexpr bool MIXED = sizeof(T) == 4;
-  const long long n4 = 4ll * nb.nslot;
-  if (pm.order == 4) k_spread4<MIXED><<<(unsigned)((n4 + TB - 1) / TB), TB, 0, st>>>(nb, pm);
-  else k_spread<MIXED, 0><<<(nb.nslot + TB - 1) / TB, TB, 0, st>>>(nb, pm);
+  auto slots = [&](int w) { return (unsigned)(((long long)w * nb.nslot + TB - 1) / TB); };
+  switch (pm.order) {  // (even, at most 8)
+    case 2: k_spread<MIXED, 2><<<slots(SLOT_THREADS<2>), TB, 0, st>>>(nb, pm); break;
+    case 4: k_spread<MIXED, 4><<<slots(SLOT_THREADS<4>), TB, 0, st>>>(nb, pm); break;
+    case 6: k_spread<MIXED, 6><<<slots(SLOT_THREADS<6>), TB, 0, st>>>(nb, pm); break;
+    default: k_spread<MIXED, 8><<<slots(SLOT_THREADS<8>), TB, 0, st>>>(nb, pm);
+  }
   if (mark) mark(mctx, "pme_spread");
   // shared memory sized to the largest work item of the plan (caps ZMAXE / LMAXE)
   const size_t zsmem = sizeof(T2) * (256 + 2 * (size_t)pm.zbuf);
@@ -1321,8 +1214,12 @@ int recip_t(const SystemDev &s, const NbListDev &nb, const PmeDev &pm, cudaStrea
     default: k_fft_z_inv<T><<<pm.nzwork, ZT, zsmem, st>>>(pm);
   }
   if (mark) mark(mctx, "pme_fft");
-  if (pm.order == 4) k_gather4<MIXED><<<(unsigned)((4ll * nb.nslot + TB - 1) / TB), TB, 0, st>>>(s, nb, pm);
-  else k_gather<MIXED, 0><<<(nb.nslot + TB - 1) / TB, TB, 0, st>>>(s, nb, pm);
+  switch (pm.order) {
+    case 2: k_gather<MIXED, 2><<<slots(SLOT_THREADS<2>), TB, 0, st>>>(s, nb, pm); break;
+    case 4: k_gather<MIXED, 4><<<slots(SLOT_THREADS<4>), TB, 0, st>>>(s, nb, pm); break;
+    case 6: k_gather<MIXED, 6><<<slots(SLOT_THREADS<6>), TB, 0, st>>>(s, nb, pm); break;
+    default: k_gather<MIXED, 8><<<slots(SLOT_THREADS<8>), TB, 0, st>>>(s, nb, pm);
+  }
   if (mark) mark(mctx, "pme_gather");
   return 0;
 }
