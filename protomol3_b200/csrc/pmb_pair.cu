@@ -23,9 +23,10 @@
 // instance with run-time switches.
 //
 // Two arithmetic paths share the structure:
-//   * FP64 ("plain"): raw double positions, the reference's minimal image (d - L rint(d/L) gives
-//     the same double as its single-wrap branches), IEEE division/sqrt/exp and the A&S erfc
-//     polynomial exactly as the reference evaluates them;
+//   * FP64 ("plain"): the reference's minimal image (d - L rint(d/L) gives the same double as its
+//     single-wrap branches), taken once per atom and tile relative to the cluster's first atom
+//     where the box is large enough for that and per pair otherwise, and the A&S erfc polynomial
+//     as the reference evaluates it;
 //   * mixed: positions as 32-bit fractional fixed point per box edge, so the minimal image is the
 //     wrap-around of an int32 difference and the pair vector keeps full FP32 precision however
 //     large the box; FP32 arithmetic with MUFU rsqrt/exp2/rcp.
@@ -161,8 +162,8 @@ __device__ __forceinline__ typename std::conditional<MIXED, float, double>::type
     rinv = rsqrt_ftz(r2s);
     rd2 = rinv * rinv;
   } else {
-    rd2 = 1.0 / r2s;
-    rinv = T(0);
+    rinv = rsqrt(r2s);
+    rd2 = rinv * rinv;
   }
   T fs = T(0);
   if constexpr (LSW != NONE) {
@@ -184,8 +185,7 @@ __device__ __forceinline__ typename std::conditional<MIXED, float, double>::type
     if (ex == 1) q *= T(p.coulomb_scaling);
     T e, f;
     if constexpr (CM == 1) {
-      if constexpr (MIXED) e = q * rinv;
-      else e = q * sqrt(rd2);
+      e = q * rinv;
       f = e * rd2;
     } else if constexpr (MIXED) {
       T r = r2s * rinv, ar = T(p.alpha) * r;
@@ -195,10 +195,10 @@ __device__ __forceinline__ typename std::conditional<MIXED, float, double>::type
       e = poly * g * rinv;
       f = (e + T(p.a2pi) * g) * rd2;
     } else {
-      T r = sqrt(r2s), rr = 1.0 / r, ar = p.alpha * r;
+      T r = r2s * rinv, ar = p.alpha * r;
       T g = q * exp(-ar * ar);
-      e = poly5(ar) * g * rr;
-      f = (e + p.a2pi * g) * rr * rr;
+      e = poly5(ar) * g * rinv;
+      f = (e + p.a2pi * g) * rd2;
     }
     sw_apply<CSW>(p.coul_sw, r2s, e, f);
     a.ec += e;
@@ -422,8 +422,9 @@ struct WarpCtx {
   double s[3];     // box edge / 2^32: fractional fixed point to A
   float sf[3];     // the same in FP32 (j-atom staging: one conversion and one product per axis)
   float L[3], Lr[3];
-  unsigned r0[3];  // fixed-point position of cluster atom 0 (mixed relative coordinates)
+  unsigned r0[3];  // position of cluster atom 0 (relative coordinates): fixed point (mixed),
   int pad_;
+  double p0[3];    // A (FP64)
 };
 
 // Bytes of one warp's prefetch region: the j-list entries of a unit, and two buffers of
@@ -435,7 +436,7 @@ constexpr size_t warp_pref_bytes() {
 }
 
 template <bool MIXED, int LSW, int CM, int CSW, bool VIR, bool MULTI>
-__global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !MULTI) ? (VIR ? PAIR_MINB_VIR : PAIR_MINB) : (!MIXED && !VIR && !MULTI) ? PAIR_MINB_FP64 : 2)
+__global__ void __launch_bounds__(PAIR_THREADS, MULTI ? 2 : VIR ? PAIR_MINB_VIR : MIXED ? PAIR_MINB : PAIR_MINB_FP64)
     k_pair(SystemDev s, NbListDev nb, PairParams p,
            ParamsT<typename std::conditional<MIXED, float, double>::type> pt, const double *ljd,
            const double *lat, int unit_kinds, int wslot) {
@@ -492,7 +493,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !MULTI) ? (VIR ? PAIR_
   int4 im = make_int4(-1, -1, 0, 0);   // orig, mol, type, box of this lane's i-atom
   T xi = 0, yi = 0, zi = 0, qi = 0;     // i-atom position (relative for the mixed path)
   const BoxDev *bx = nullptr;
-  bool wrap = !MIXED;
+  bool wrap = true;
   // per-warp constants of the current box and cluster, kept in shared memory rather than in
   // registers (they are read once per tile)
   WarpCtx *ctx = reinterpret_cast<WarpCtx *>(smem_raw + ljbytes + PAIR_WARPS * warp_stage_bytes<MIXED>()) + wib;
@@ -529,7 +530,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !MULTI) ? (VIR ? PAIR_
       fi_acc[c] = T(0);
       a2p.fi[c] = sp2(0.f);
     }
-    if constexpr (VIR && MIXED)
+    if constexpr (VIR)
       if (!wrap) add_virial(f[0], f[1], f[2], xi, yi, zi);
     if constexpr (!MIXED) {  // one rounding for the cluster's lane groups instead of four
 #pragma unroll
@@ -620,6 +621,11 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !MULTI) ? (VIR ? PAIR_
     }
     cp_async_commit();
   };
+  // FP64: minimal image of a coordinate relative to cluster atom 0, once per atom and tile
+  auto relative = [&](double x, int c) {
+    const double d = x - ctx->p0[c];
+    return d - bx->L[c] * rint(bx->Lr[c] * d);
+  };
   // stage this lane's j-atom of buffer b (or padding)
   auto stage_slot = [&](int sl, int b, JStage<MIXED> &js, int &orig) {
     const int4 m = sl >= 0 ? rawM[b * 32 + lane] : make_int4(-1, -1, 0, 0);
@@ -633,6 +639,11 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !MULTI) ? (VIR ? PAIR_
                            (float)(int)(f.z - ctx->r0[2]) * ctx->sf[2], __uint_as_float(f.w));
       } else {
         js.p = rawP[b * 32 + lane];
+        if (!wrap) {
+          js.p.x = relative(js.p.x, 0);
+          js.p.y = relative(js.p.y, 1);
+          js.p.z = relative(js.p.z, 2);
+        }
       }
     } else {
       orig = -1;
@@ -677,42 +688,54 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !MULTI) ? (VIR ? PAIR_
           ctx->Lr[c] = (float)bx->Lr[c];
         }
     }
-    if constexpr (MIXED) {
-      // coordinates relative to cluster atom 0 are minimal-image differences whenever
-      // L/2 > cutoff + cluster extent; otherwise (small boxes) every pair is wrapped again
+    {
+      // coordinates relative to cluster atom 0 are minimal-image differences whenever L/2 exceeds
+      // the cutoff and the cluster's extent at the last build with what two atoms may have moved
+      // since; otherwise (small boxes) every pair is wrapped again
       const uint4 lo = nb.blk_lo[I], hi = nb.blk_hi[I];
-      const double rmax = sqrt(p.cut2) + 1e-3;
+      const double rmax = sqrt(p.cut2) + 1e-3 + 2.0 * sqrt((double)nb.half_skin2);
       const double sx = bx->L[0] * (1.0 / 4294967296.0), sy = bx->L[1] * (1.0 / 4294967296.0),
                    sz = bx->L[2] * (1.0 / 4294967296.0);
       wrap = bx->multi_image || (double)(hi.x - lo.x) * sx + rmax >= 0.5 * bx->L[0] ||
              (double)(hi.y - lo.y) * sy + rmax >= 0.5 * bx->L[1] ||
              (double)(hi.z - lo.z) * sz + rmax >= 0.5 * bx->L[2];
-      const uint4 f = nb.slot_fx[sl];
-      const unsigned rx0 = __shfl_sync(0xffffffffu, f.x, 0), ry0 = __shfl_sync(0xffffffffu, f.y, 0),
-                     rz0 = __shfl_sync(0xffffffffu, f.z, 0);
-      __syncwarp();
-      if (lane == 0) {
-        ctx->r0[0] = rx0;
-        ctx->r0[1] = ry0;
-        ctx->r0[2] = rz0;
-      }
-      __syncwarp();
-      if (im.x >= 0) {
-        xi = (float)((double)(int)(f.x - rx0) * sx);
-        yi = (float)((double)(int)(f.y - ry0) * sy);
-        zi = (float)((double)(int)(f.z - rz0) * sz);
+      if constexpr (MIXED) {
+        const uint4 f = nb.slot_fx[sl];
+        const unsigned rx0 = __shfl_sync(0xffffffffu, f.x, 0), ry0 = __shfl_sync(0xffffffffu, f.y, 0),
+                       rz0 = __shfl_sync(0xffffffffu, f.z, 0);
+        __syncwarp();
+        if (lane == 0) {
+          ctx->r0[0] = rx0;
+          ctx->r0[1] = ry0;
+          ctx->r0[2] = rz0;
+        }
+        __syncwarp();
+        if (im.x >= 0) {
+          xi = (float)((double)(int)(f.x - rx0) * sx);
+          yi = (float)((double)(int)(f.y - ry0) * sy);
+          zi = (float)((double)(int)(f.z - rz0) * sz);
+        } else {
+          xi = yi = zi = 1e6f;
+        }
+        qi = __uint_as_float(f.w);
       } else {
-        xi = yi = zi = 1e6f;
+        const double4 q4 = nb.slot_pq[sl];
+        __syncwarp();
+        if (lane == 0) {
+          ctx->p0[0] = q4.x;
+          ctx->p0[1] = q4.y;
+          ctx->p0[2] = q4.z;
+        }
+        __syncwarp();
+        if (im.x >= 0) {
+          xi = wrap ? q4.x : relative(q4.x, 0);
+          yi = wrap ? q4.y : relative(q4.y, 1);
+          zi = wrap ? q4.z : relative(q4.z, 2);
+        } else {
+          xi = yi = zi = 1e6;
+        }
+        qi = q4.w;
       }
-      qi = __uint_as_float(f.w);
-    } else {
-      const double4 q4 = nb.slot_pq[sl];
-      if (im.x >= 0) {
-        xi = q4.x; yi = q4.y; zi = q4.z;
-      } else {
-        xi = yi = zi = 1e6;
-      }
-      qi = q4.w;
     }
     cp_async_wait<0>();
     __syncwarp();  // the words copied by the other lanes
@@ -789,7 +812,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !MULTI) ? (VIR ? PAIR_
             dj.p = sjp[gb | jl];
             dj.m = sjm[gb | jl];
             T dx = T(dj.p.x) - xi, dy = T(dj.p.y) - yi, dz = T(dj.p.z) - zi;
-            if constexpr (!MIXED) {
+            if constexpr (!MIXED && WRAP) {
               // the reference's minimal image: d - L rint(d / L) equals its single-wrap result
               dx -= bx->L[0] * rint(bx->Lr[0] * dx);
               dy -= bx->L[1] * rint(bx->Lr[1] * dy);
@@ -851,15 +874,10 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !MULTI) ? (VIR ? PAIR_
             fj[2] = __shfl_sync(0xffffffffu, fj[2], nxt);
           }
         };
-        bool unwrapped = false;
-        if constexpr (MIXED) {
-          if (!wrap) {
-            unwrapped = true;
-            if (diag) body(std::true_type{}, std::false_type{});
-            else body(std::false_type{}, std::false_type{});
-          }
-        }
-        if (!unwrapped) {
+        if (!wrap) {
+          if (diag) body(std::true_type{}, std::false_type{});
+          else body(std::false_type{}, std::false_type{});
+        } else {
           if (diag) body(std::true_type{}, std::true_type{});
           else body(std::false_type{}, std::true_type{});
         }
@@ -877,7 +895,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, (MIXED && !MULTI) ? (VIR ? PAIR_
             for (int c = 0; c < 6; c++) v_acc[c] += a.vir[c];
       }
       // (an own atom's j-side force joins its i-side force below)
-      if constexpr (VIR && MIXED)
+      if constexpr (VIR)
         if (!wrap && !(diag && gb == 0)) add_virial(tfj[0], tfj[1], tfj[2], mine.p.x, mine.p.y, mine.p.z);
 
       if (diag && gb == 0) {  // own atom li: its j-side force joins its i-side force
