@@ -449,6 +449,7 @@ int nblist_alloc(pmb_system *s, double rl) {
                                                                 std::pow(rl + 2.0, 3)) / (2 * JCHUNK));
   const double per_warp = tiles_est / (nb.n_sm * PAIR_WARPS_PER_SM * PAIR_UNITS_PER_WARP);
   nb.unit_tiles = std::max(CLOSE_TILES, std::min(UNIT_TILES, (int)(per_warp / CLOSE_TILES) * CLOSE_TILES));
+  nb.fills_chip = tiles_est / nb.unit_tiles >= nb.n_sm * PAIR_WARPS_PER_SM;
   long long units = 0;
   for (int bi = 0; bi < s->nbox; bi++) {
     const BoxDev &b = s->hbox[bi];
@@ -660,9 +661,9 @@ int enqueue_forces(pmb_system *s, pmb_force *const *fs, int n, int virial, bool 
   s->last_used_list = need_list;
   // PME, exclusion corrections and bonded terms run on the side stream beside the list build and
   // the pair kernel (every sum is an integer atomic, so the interleaving does not change a bit):
-  // both fork once this step's slot records are packed (beside the displacement check the terms
-  // held it up: 6 -> 12 us at 98,304 atoms), the PME chain and the terms each on a stream.  The
-  // stage profiler keeps everything in one stream to time each stage.
+  // the PME chain once this step's slot records are packed, the terms on a third stream after its
+  // z transforms (beside the displacement check or the spread they held those up: both live on
+  // atomics).  The stage profiler keeps everything in one stream to time each stage.
   bool others = false;
   for (int i = 0; i < n; i++) others |= fs[i]->kind == PMB_FORCE_PME || fs[i]->kind == PMB_FORCE_BONDED;
   bool split = !s->prof && !jobs.empty() && others && st != cudaStreamLegacy;
@@ -675,7 +676,7 @@ int enqueue_forces(pmb_system *s, pmb_force *const *fs, int n, int virial, bool 
   cudaStream_t so = split ? s->side : st, sterms = split ? s->terms : st;
   auto launch_recip = [&](pmb_force *f) {
     f->pm.virial = virial;
-    pme_recip_launch(sd, s->nb, f->pm, so, mark, s);
+    pme_recip_launch(sd, s->nb, f->pm, so, split ? s->ev_fork : nullptr, mark, s);
   };
   // exclusion corrections, bonded terms: no list needed; a PME force's corrections and a bonded
   // force share a launch, except under the stage profiler
@@ -717,9 +718,9 @@ int enqueue_forces(pmb_system *s, pmb_force *const *fs, int n, int virial, bool 
     if (split) {
       CK(cudaEventRecord(s->ev_slots, st));
       CK(cudaStreamWaitEvent(s->side, s->ev_slots, 0));
-      CK(cudaStreamWaitEvent(s->terms, s->ev_slots, 0));
       for (int i = 0; i < n; i++)
         if (fs[i]->kind == PMB_FORCE_PME && fs[i]->d.reciprocal) launch_recip(fs[i]);
+      CK(cudaStreamWaitEvent(s->terms, need_pme_slots ? s->ev_fork : s->ev_slots, 0));
       launch_all_atom_terms();
     }
     nblist_lists(sd, s->nb, rlist, st);
@@ -730,6 +731,10 @@ int enqueue_forces(pmb_system *s, pmb_force *const *fs, int n, int virial, bool 
       if (fs[i]->kind == PMB_FORCE_PME && fs[i]->d.reciprocal) launch_recip(fs[i]);
     launch_all_atom_terms();
   }
+  // Where the pair kernel's CTAs fill every SM until they end, it waits for the PME chain's first two
+  // kernels: the next one, of few CTAs, then starts beside it and not after it (27,000 atoms: 133 ->
+  // 121 us a step; FP64, 15,000: 123 -> 117).  A smaller system leaves room anyway.
+  if (split && need_pme_slots && s->nb.fills_chip) CK(cudaStreamWaitEvent(st, s->ev_fork, 0));
   for (size_t q = 0; q < jobs.size(); q++) {
     const PairJob &j = jobs[q];
     PairLaunch pl;
@@ -1227,10 +1232,10 @@ int pmb_system_list_tiles(pmb_system *s, long long *tiles) {
   if (!s || !tiles) return fail(PMB_ERR_ARG, "null argument");
   *tiles = 0;
   if (!s->nb_ready) return PMB_OK;
-  int v = 0;
-  CK(cudaMemcpyAsync(&v, s->nb.ctl + CTL_TILES, sizeof(v), cudaMemcpyDeviceToHost, s->stream));
+  std::vector<int> cnt(s->nb.nblk_total);
+  CK(cudaMemcpyAsync(cnt.data(), s->nb.jcount, sizeof(int) * cnt.size(), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
-  *tiles = v;
+  for (int c : cnt) *tiles += c;
   return PMB_OK;
 }
 
@@ -1494,8 +1499,11 @@ pmb_force *pmb_force_create(pmb_system *s, const pmb_force_desc *d) {
     pm.pradix = dpr;
     pm.perm = dperm;
     pm.psmem = psmem;
-    // threads for about one butterfly each in a stage of radix 4 or 5, up to PLANE_MAX_THREADS
-    pm.pthreads = std::max(64, std::min(PLANE_MAX_THREADS, ((int)(plane_points / 4) + 63) / 64 * 64));
+    // threads for about one butterfly each in a stage, of radix 4 or 5 where the planes are few and
+    // latency counts, of radix 8 where they fill the chip (256 boxes: 218 -> 138 us), up to
+    // PLANE_MAX_THREADS
+    const int stage = pwork.size() >= 1024 ? 8 : 4;
+    pm.pthreads = std::max(64, std::min(PLANE_MAX_THREADS, ((int)(plane_points / stage) + 63) / 64 * 64));
     pm.plan = dplan;
     pm.twiddle = dtw;
     pm.twiddlef = dtwf;

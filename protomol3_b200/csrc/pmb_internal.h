@@ -43,9 +43,8 @@ enum {
   CTL_BUILDS = 4,   // list builds so far (64 bits)
   CTL_PAIR = 6,     // the pair kernel's next unit and finished warps, two launches; zero between them
   CTL_VACUUM = 10,  // check the extent of vacuum boxes
-  CTL_CLAIM = 11,   // the list build's next block
+  CTL_CLAIM = 11,   // the list build's next group of blocks
   CTL_UNITS = 12,   // pair units of boxes without and with lattice images
-  CTL_TILES = 14,   // tiles of all lists
   CTL_WORDS = 16
 };
 struct NbListDev {
@@ -65,6 +64,7 @@ struct NbListDev {
                                // need lattice images from the end of the array, the others from
                                // the front (ctl[CTL_UNITS + 1] and ctl[CTL_UNITS] of them)
   int unit_cap;
+  bool fills_chip;             // about a unit or more for every warp the chip holds
   int unit_tiles;              // most tiles of a unit: CLOSE_TILES .. UNIT_TILES
   int *status;                 // [4]: list / tile overflow, non-finite position, vacuum extent
   // per slot
@@ -197,7 +197,8 @@ struct PmeDev {
 #endif
 // Optional stage marker (profiling): called on the host between kernel launches.
 typedef void (*StageMark)(void *ctx, const char *stage);
-int pme_recip_launch(const SystemDev &s, const NbListDev &nb, const PmeDev &pm, cudaStream_t st,
+// head: recorded on st once the z transforms are enqueued (null: not)
+int pme_recip_launch(const SystemDev &s, const NbListDev &nb, const PmeDev &pm, cudaStream_t st, cudaEvent_t head = nullptr,
                      StageMark mark = nullptr, void *mark_ctx = nullptr);
 int pme_line_capacity();
 // Plane kernel: most threads, most shared memory, the stages of a line, a plane's shared memory.

@@ -245,21 +245,21 @@ __device__ __forceinline__ void sort_extents(const NbListDev &nb, const BoxDev &
 }
 
 // Every phase in one launch, a CTA per box: small boxes, and systems of many.
-constexpr int SORT_THREADS = 512;
-__global__ void __launch_bounds__(SORT_THREADS) k_sort_box(SystemDev s, NbListDev nb) {
+constexpr int SORT_THREADS = 512, SORT_BOX_THREADS = 1024;
+__global__ void __launch_bounds__(SORT_BOX_THREADS) k_sort_box(SystemDev s, NbListDev nb) {
   if (!nb.ctl[CTL_REBUILD]) return;
   const int bi = blockIdx.x, t = threadIdx.x;
   if (!nb.box_rb[bi]) return;  // the box keeps its slots
   const BoxDev &b = s.box[bi];
-  sort_bin(s, nb, b, t, SORT_THREADS);
+  sort_bin(s, nb, b, t, SORT_BOX_THREADS);
   __syncthreads();
   sort_scan(nb, b);
   __syncthreads();
-  sort_scatter(nb, b, t, SORT_THREADS);
+  sort_scatter(nb, b, t, SORT_BOX_THREADS);
   __syncthreads();
-  sort_place(s, nb, b, bi, t, SORT_THREADS);
+  sort_place(s, nb, b, bi, t, SORT_BOX_THREADS);
   __syncthreads();
-  sort_extents(nb, b, t, SORT_THREADS);
+  sort_extents(nb, b, t, SORT_BOX_THREADS);
 }
 
 // One launch per phase over the whole chip (blockIdx.y: box): large boxes.  The last CTA of a box
@@ -315,44 +315,15 @@ __device__ __forceinline__ float gap2f(const float sL[3], const unsigned c1[3], 
 constexpr int BL_THREADS = BL_BLOCK_THREADS;
 constexpr int BL_CAP = 128;  // candidate blocks buffered per warp before their atoms are tested
 
-// Appends I's list to the pair kernel's work as units of at most nb.unit_tiles tiles (about equal
-// parts of the list, starting at multiples of CLOSE_TILES tiles); a block of a box that keeps its
-// list appends the units it has.  The units of boxes that need lattice images grow from the end
-// of the array.  Their order varies from build to build and changes no result: the pair kernel
-// closes its floating-point sums every CLOSE_TILES tiles of a list.
-__device__ __forceinline__ void append_units(NbListDev &nb, int I, int tiles, bool multi, int lane) {
-  const int nc = (tiles + CLOSE_TILES - 1) / CLOSE_TILES;
-  const int per = nb.unit_tiles / CLOSE_TILES, nu = (nc + per - 1) / per;
-  if (nu == 0) return;
-  int at = 0;
-  if (lane == 0) {
-    at = (int)atomicAdd(nb.ctl + CTL_UNITS + (multi ? 1 : 0), (unsigned)nu);
-    atomicAdd(nb.ctl + CTL_TILES, (unsigned)tiles);
-  }
-  at = __shfl_sync(0xffffffffu, at, 0);
-  for (int p = lane; p < nu; p += 32) {
-    const int k0 = (int)((long long)nc * p / nu) * CLOSE_TILES;
-    const int k1 = min(tiles, (int)((long long)nc * (p + 1) / nu) * CLOSE_TILES);
-    const int u = at + p;  // (within the array: it is sized for full lists)
-    nb.units[multi ? nb.unit_cap - 1 - u : u] = make_int4(I, k0, k1 - k0, nb.jcap_off[I] + k0 * JCHUNK);
-  }
-}
-
-// One warp per block I (claimed from a counter, in ascending order: the early blocks' lists are
-// the longest): its own slots, then the candidate blocks J > I of the same box by
+// One warp per block I: its own slots, then the candidate blocks J > I of the same box by
 // bounding-box gap (superblocks of 32 blocks first), compacted into a shared-memory list, then
 // the atoms of GROUPS listed blocks per pass within the list cutoff of I's box, compacted into
 // I's j-list (tiles of 32 entries).  The loads of the next pass are issued before the current
 // pass is tested.
-// One block's list; cl [BL_CAP] and ipos [BLOCK] are the warp's shared memory.
-__device__ __forceinline__ void build_block(const SystemDev &s, NbListDev &nb, double rlist2, int I, int *cl, float4 *ipos) {
+// One block's list; cl [BL_CAP] and ipos [BLOCK] are the warp's shared memory.  Returns its tiles.
+__device__ __forceinline__ int build_block(const SystemDev &s, NbListDev &nb, double rlist2, int I, const BoxDev &b, int *cl,
+                                           float4 *ipos) {
   const int lane = threadIdx.x & 31;
-  const int bi = nb.blk_box[I];
-  const BoxDev &b = s.box[bi];
-  if (!nb.box_rb[bi]) {  // the box keeps its list
-    append_units(nb, I, nb.jcount[I], b.multi_image != 0, lane);
-    return;
-  }
   const uint4 cIv = nb.blk_c[I], hIv = nb.blk_h[I];
   const float sL[3] = {(float)(b.L[0] * (1.0 / 4294967296.0)), (float)(b.L[1] * (1.0 / 4294967296.0)),
                        (float)(b.L[2] * (1.0 / 4294967296.0))};
@@ -514,21 +485,55 @@ __device__ __forceinline__ void build_block(const SystemDev &s, NbListDev &nb, d
     if (overflow) atomicExch(&nb.status[0], 1);
     nb.jcount[I] = tiles;
   }
-  append_units(nb, I, tiles, multi, lane);
-  __syncwarp();  // the shared memory is written again for the next block
+  return tiles;
 }
 
+// CTAs claim groups of consecutive blocks from a counter, one block per warp, in ascending order (the
+// early blocks' lists are the longest).  The group's lists then join the pair kernel's work as units
+// of at most nb.unit_tiles tiles (about equal parts of a list, starting at multiples of CLOSE_TILES
+// tiles); a block of a box that keeps its list appends the units it has.  The units of boxes that
+// need lattice images grow from the end of the array.  Their order varies from build to build and
+// changes no result: the pair kernel closes its floating-point sums every CLOSE_TILES tiles of a
+// list.  One claim and one append per group: with three atomics per block the counters' words were
+// the bound of an ensemble's build (810,000 atoms, a quarter of the boxes rebuilt: 590 us a step).
 __global__ void __launch_bounds__(BL_THREADS, BL_MINB) k_build_lists(SystemDev s, NbListDev nb, double rlist2) {
-  __shared__ int cand_all[BL_THREADS / 32][BL_CAP];
-  __shared__ float4 ipos_all[BL_THREADS / 32][BLOCK];
+  constexpr int NW = BL_THREADS / 32;
+  __shared__ int cand_all[NW][BL_CAP];
+  __shared__ float4 ipos_all[NW][BLOCK];
+  __shared__ int group, units[NW], base[2];
   if (!nb.ctl[CTL_REBUILD]) return;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, per = nb.unit_tiles / CLOSE_TILES;
   for (;;) {
-    int I = 0;
-    if (lane == 0) I = (int)atomicAdd(nb.ctl + CTL_CLAIM, 1u);
-    I = __shfl_sync(0xffffffffu, I, 0);
-    if (I >= nb.nblk_total) return;
-    build_block(s, nb, rlist2, I, cand_all[w], ipos_all[w]);
+    if (threadIdx.x == 0) group = (int)atomicAdd(nb.ctl + CTL_CLAIM, 1u);
+    __syncthreads();
+    if (group * NW >= nb.nblk_total) return;
+    const int I = group * NW + w;
+    int tiles = 0, multi = 0;
+    if (I < nb.nblk_total) {
+      const int bi = nb.blk_box[I];
+      const BoxDev &b = s.box[bi];
+      multi = b.multi_image != 0;
+      tiles = nb.box_rb[bi] ? build_block(s, nb, rlist2, I, b, cand_all[w], ipos_all[w]) : nb.jcount[I];
+    }
+    const int nc = (tiles + CLOSE_TILES - 1) / CLOSE_TILES, nu = (nc + per - 1) / per;
+    if (lane == 0) units[w] = 2 * nu + multi;
+    __syncthreads();
+    if (threadIdx.x < 2) {  // the group's units without and with lattice images
+      int n = 0;
+      for (int k = 0; k < NW; k++)
+        if ((units[k] & 1) == (int)threadIdx.x) n += units[k] >> 1;
+      base[threadIdx.x] = n ? (int)atomicAdd(nb.ctl + CTL_UNITS + threadIdx.x, (unsigned)n) : 0;
+    }
+    __syncthreads();
+    int at = base[multi];
+    for (int k = 0; k < w; k++)
+      if ((units[k] & 1) == multi) at += units[k] >> 1;
+    for (int p = lane; p < nu; p += 32) {
+      const int k0 = (int)((long long)nc * p / nu) * CLOSE_TILES;
+      const int k1 = min(tiles, (int)((long long)nc * (p + 1) / nu) * CLOSE_TILES);
+      const int u = at + p;  // (within the array: it is sized for full lists)
+      nb.units[multi ? nb.unit_cap - 1 - u : u] = make_int4(I, k0, k1 - k0, nb.jcap_off[I] + k0 * JCHUNK);
+    }
   }
 }
 
@@ -549,7 +554,7 @@ int nblist_sort(const SystemDev &s, NbListDev &nb, bool updated, cudaStream_t st
   if (na <= 0) return 0;
   if (!updated) k_update<<<(na + UPDATE_THREADS - 1) / UPDATE_THREADS, UPDATE_THREADS, 0, st>>>(s, nb);
   if (sort_by_box(s, nb)) {
-    k_sort_box<<<s.nbox, SORT_THREADS, 0, st>>>(s, nb);
+    k_sort_box<<<s.nbox, SORT_BOX_THREADS, 0, st>>>(s, nb);
     return 0;
   }
   const dim3 grid((nb.max_box_atoms + SORT_THREADS - 1) / SORT_THREADS, s.nbox);

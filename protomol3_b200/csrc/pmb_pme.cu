@@ -1144,7 +1144,7 @@ __global__ void __launch_bounds__(WZ) k_fft_z_inv_warp(PmeDev pm) {
 }
 
 template <typename T>
-int recip_t(const SystemDev &s, const NbListDev &nb, const PmeDev &pm, cudaStream_t st,
+int recip_t(const SystemDev &s, const NbListDev &nb, const PmeDev &pm, cudaStream_t st, cudaEvent_t head,
             StageMark mark, void *mctx) {
   using T2 = typename C2<T>::t;
   const int TB = 256;
@@ -1168,6 +1168,7 @@ int recip_t(const SystemDev &s, const NbListDev &nb, const PmeDev &pm, cudaStrea
     zconf[dev] = true;
   }
   k_fft_z_fwd<T><<<pm.nzwork, ZT, zsmem, st>>>(pm);
+  if (head) cudaEventRecord(head, st);
   const size_t lsmem = 32 * sizeof(double) + sizeof(T2) * (256 + 2 * (size_t)pm.lbuf);
   if (!lconf[dev]) {
     const int lcap = (int)(32 * sizeof(double) + sizeof(T2) * (256 + 2 * (size_t)LMAXE));
@@ -1259,10 +1260,10 @@ size_t pme_plane_smem(int nx, int ny, int precision) {
   return sizeof(double) * (32 + nx + ny + (nx + ny) % 2) + c * ((size_t)nx + ny + (size_t)nx * (ny | 1));
 }
 
-int pme_recip_launch(const SystemDev &s, const NbListDev &nb, const PmeDev &pm, cudaStream_t st,
+int pme_recip_launch(const SystemDev &s, const NbListDev &nb, const PmeDev &pm, cudaStream_t st, cudaEvent_t head,
                      StageMark mark, void *mctx) {
-  return pm.precision ? recip_t<float>(s, nb, pm, st, mark, mctx)
-                      : recip_t<double>(s, nb, pm, st, mark, mctx);
+  return pm.precision ? recip_t<float>(s, nb, pm, st, head, mark, mctx)
+                      : recip_t<double>(s, nb, pm, st, head, mark, mctx);
 }
 
 }  // namespace pmb

@@ -138,7 +138,7 @@ __device__ __forceinline__ void update_atom(const SystemDev &s, NbListDev &nb, i
     if (any) {
       ++*reinterpret_cast<unsigned long long *>(nb.ctl + CTL_BUILDS);
       // the build starts its list of pair units anew
-      nb.ctl[CTL_CLAIM] = nb.ctl[CTL_UNITS] = nb.ctl[CTL_UNITS + 1] = nb.ctl[CTL_TILES] = 0u;
+      nb.ctl[CTL_CLAIM] = nb.ctl[CTL_UNITS] = nb.ctl[CTL_UNITS + 1] = 0u;
     }
     nb.ctl[CTL_BLOCKS] = 0u;
     nb.ctl[CTL_FORCED] = 0u;
