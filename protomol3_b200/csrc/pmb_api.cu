@@ -2162,6 +2162,12 @@ int pmb_md_set_constraints(pmb_md *m, const pmb_constraint_desc *d) {
   c.ncons = nc;
   c.max_atoms = max_atoms;
   c.max_cons = max_cons;
+  c.water3 = local.size() == 3 * (size_t)ng && atoms.size() == 3 * (size_t)ng;
+  for (int g = 0; g < ng && c.water3; g++) {
+    const int2 *l = local.data() + 3 * (size_t)g;
+    c.water3 = group_con[g + 1] == 3 * (g + 1) && group_atom[g + 1] == 3 * (g + 1) && l[0].x == 0 && l[0].y == 1 &&
+               l[1].x == 0 && l[1].y == 2 && l[2].x == 1 && l[2].y == 2;
+  }
   c.group_con = d_gc;
   c.group_atom = d_ga;
   c.atoms = d_atoms;

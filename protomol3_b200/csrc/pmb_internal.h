@@ -257,6 +257,7 @@ constexpr double CON_ERR_SCALE = 1099511627776.0;  // 2^40: fixed point of the p
 struct ConstraintDev {
   int ngroup, ncons;
   int max_atoms, max_cons;  // largest group (selects the kernel: rigid waters have 3 and 3)
+  int water3;               // every group: three atoms, constraints 0-1, 0-2, 1-2 in that order
   const int *group_con;    // [ngroup + 1] constraint offsets of each group
   const int *group_atom;   // [ngroup + 1] offsets into atoms
   const int *atoms;        // group atoms (global indices), each group's first-use order

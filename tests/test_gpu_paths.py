@@ -1,0 +1,135 @@
+"""The kernels' dispatch rules at the sizes where they change: list sort, pair work, plane
+transform, stencil orders, virial, kinetic energy, state copies, against the CPU oracle (or numpy).
+
+Tolerances as tests/test_gpu_parity.py: FP64 1e-9 and mixed 1e-5 of the norm of the forces; virials
+ten times that of their largest component."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from protomol3_b200 import forces as F
+from protomol3_b200 import waterbox as W
+
+pytestmark = pytest.mark.gpu
+TOL = {"fp64": 1e-9, "mixed": 1e-5}
+
+
+def rel(a, b):
+    return float(np.linalg.norm(a - b) / np.linalg.norm(b))
+
+
+def shaken(n, seed):
+    """A water box with stretched bonds and bent angles."""
+    b = W.water_box(n, seed=seed)
+    b["pos"] = b["pos"] + np.random.default_rng(seed).normal(0.0, 0.02, b["pos"].shape)
+    return b
+
+
+def evaluate(boxes, fl, precision, virial=False):
+    topo = F.Topology(boxes, precision)
+    f, e = np.zeros((topo.n_atoms, 3)), F.ScalarStructure(topo.n_boxes, virial=virial)
+    F.evaluate_all(topo, fl, topo.positions(), f, e)
+    return f, e, topo
+
+
+# 1024 waters are the last box that one CTA sorts (3,072 atoms); 2 waters are less than a block
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("waters", [2, 3, 341, 1024, 1025])
+def test_list_sort_and_units(precision, waters):
+    b = shaken(waters, 31)
+    cut = min(8.0, 0.45 * b["box"][0])
+    f, e, topo = evaluate(b, [F.NonbondedCutoffSystemForce(lj=("C2", 0.8 * cut, cut), coulomb=("C1", 0.0, cut)),
+                              F.BondedSystemForce()], precision, virial=True)
+    fo, _, vo, _ = O.evaluate(O.System(b), b["pos"], cutoff=O.cutoff_params(lj=("C2", 0.8 * cut, cut), coul=("C1", 0.0, cut)),
+                              bonded=True, virial=True)
+    assert rel(f, fo) < TOL[precision]
+    np.testing.assert_allclose(e.virial().ravel(), vo, rtol=0, atol=10 * TOL[precision] * np.abs(vo).max() + 1e-7)
+    assert topo.list_tiles() >= -(-topo.n_atoms // 8)
+
+
+def test_large_boxes_of_one_system_sort_alike():
+    """Boxes above and below the one-CTA size in one system (a launch per phase) give each box's
+    own forces bit for bit."""
+    boxes = [shaken(n, 40 + n) for n in (1500, 40, 1025)]
+    fl = lambda: [F.NonbondedCutoffSystemForce(lj=("C2", 6.0, 7.0))]  # noqa: E731
+    f, _, _ = evaluate(boxes, fl(), "mixed")
+    at = 0
+    for b in boxes:
+        n = len(b["charge"])
+        alone, _, _ = evaluate(b, fl(), "mixed")
+        np.testing.assert_array_equal(f[at:at + n], alone)
+        at += n
+
+
+# every radix of the plane transform, one to three stages, odd rows, a virial; 128 x 125 FP64 does not
+# fit shared memory and takes the line kernels
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("grid", [(8, 9, 10), (12, 15, 16), (25, 27, 20), (10, 81, 24), (50, 6, 45), (125, 24, 8),
+                                  (128, 125, 9), (4, 5, 6), (72, 54, 12)])
+def test_plane_transform(precision, grid):
+    b = shaken(60, 7)
+    pme = F.NonbondedPMEwaldSystemForce(grid, 6.0, real=False, correction=False)
+    f, e, _ = evaluate(b, [pme], precision, virial=True)
+    fo, _, vo, _ = O.evaluate(O.System(b), b["pos"], pme=O.pme_params(grid, 6.0, real=0, recip=1, corr=0), virial=True)
+    assert rel(f, fo) < TOL[precision]
+    np.testing.assert_allclose(e.virial().ravel(), vo, rtol=0, atol=10 * TOL[precision] * np.abs(vo).max())
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("order", [2, 4, 6, 8])
+def test_stencil_orders(precision, order):
+    b = shaken(77, 5)
+    f, _, _ = evaluate(b, [F.NonbondedPMEwaldSystemForce((16, 18, 20), 6.0, order=order)], precision)
+    fo, _, _, _ = O.evaluate(O.System(b), b["pos"], pme=O.pme_params((16, 18, 20), 6.0, order=order))
+    assert rel(f, fo) < TOL[precision]
+
+
+# edges just above and below what lets a tile skip the image per pair (2 (cutoff + cluster extent + skin))
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("waters", [130, 260, 420, 700])
+def test_virial_with_and_without_wrapped_tiles(precision, waters):
+    b = shaken(waters, 19)
+    g = W.pme_grid_for(b["box"][0])
+    f, e, _ = evaluate(b, [F.NonbondedCutoffSystemForce(lj=("C2", 6.0, 7.5)), F.NonbondedPMEwaldSystemForce((g, g, g), 7.5)],
+                       precision, virial=True)
+    fo, _, vo, _ = O.evaluate(O.System(b), b["pos"], cutoff=O.cutoff_params(lj=("C2", 6.0, 7.5)),
+                              pme=O.pme_params((g, g, g), 7.5), virial=True)
+    assert rel(f, fo) < TOL[precision]
+    np.testing.assert_allclose(e.virial().ravel(), vo, rtol=0, atol=10 * TOL[precision] * np.abs(vo).max())
+
+
+# one part, exactly one, one atom more, several; summation order only: n ulp at most
+@pytest.mark.parametrize("waters", [1, 682, 683, 7300])
+def test_kinetic_energy_and_state(waters):
+    """The kinetic energy of boxes of one and several parts; 7,300 waters (65,700 doubles) also take
+    the staged state copy."""
+    b = W.water_box(waters, seed=2)
+    topo = F.Topology(b, "mixed")
+    md = F.Integrator(topo, [F.BondedSystemForce()])
+    md.set_state(b["pos"], b["vel"])
+    _, kin = md.energies()
+    want = 0.5 * (b["mass"][:, None] * b["vel"] ** 2).sum()
+    assert abs(kin[0] - want) <= 3 * waters * 2.3e-16 * want
+    for _ in range(2):  # the second copy reuses the staging
+        pos, vel = md.state()
+        np.testing.assert_array_equal(pos, b["pos"])
+        np.testing.assert_array_equal(vel, b["vel"])
+
+
+@pytest.mark.parametrize("kind", ["leapfrog", "langevin"])
+def test_forces_outlive_the_list(kind):
+    """A run whose list storage is replaced between two calls goes on with the same forces: equal to
+    an uninterrupted one but for the order of the sums (other clusters), 1e-12 relative per step in
+    FP64, which ten steps amplify by less than 1e2."""
+    b = shaken(300, 3)
+    out = []
+    for change in (False, True):
+        topo = F.Topology(b, "fp64")
+        md = F.Integrator(topo, [F.NonbondedCutoffSystemForce(lj=("C2", 6.0, 7.0)), F.BondedSystemForce()], kind=kind, seed=5)
+        md.set_state(b["pos"], b["vel"])
+        md.run(5)
+        if change:
+            topo.set_tuning(skin=0.5, sort_cell=1.9)
+        md.run(5)
+        out.append(np.concatenate(md.state()))
+    assert rel(out[1], out[0]) < 1e-10
