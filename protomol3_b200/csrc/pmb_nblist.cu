@@ -314,6 +314,7 @@ __device__ __forceinline__ float gap2f(const float sL[3], const unsigned c1[3], 
 #endif
 constexpr int BL_THREADS = BL_BLOCK_THREADS;
 constexpr int BL_CAP = 128;  // candidate blocks buffered per warp before their atoms are tested
+constexpr float PAD_NORM = 1e12f;  // |q|^2 of a block's padding atoms
 
 // One warp per block I: its own slots, then the candidate blocks J > I of the same box by
 // bounding-box gap (superblocks of 32 blocks first), compacted into a shared-memory list, then
@@ -338,11 +339,12 @@ __device__ __forceinline__ int build_block(const SystemDev &s, NbListDev &nb, do
   // molecules of the cluster's atoms (-2: padding): a listed j-atom of one of them is flagged
   // JSAME, so the pair kernel runs the exclusion test only on tiles holding such an atom; the
   // block's own slots open its list (the pair kernel takes j > i among them)
-  // and the block's atom positions (fixed point; padding atoms far away): a candidate atom is
-  // listed when it is within the list radius of one of them, the exact Verlet condition per
-  // pair (the bounding-box gap alone would list about a third more atoms)
-  // (in shared memory, FP32 relative to the block's first atom; padding atoms far away)
-  // stored as pairs of atoms {t, t + BLOCK/2}: x x' y y' | z z' (two-wide FP32 tests)
+  // and the block's atom positions q: a candidate atom p is listed when it is within the list
+  // radius of one of them, the exact Verlet condition per pair (the bounding-box gap alone would
+  // list about a third more atoms).  In shared memory, FP32 relative to the block's first atom, as
+  // -2 q and |q|^2 of pairs of atoms {t, t + BLOCK/2}: x x' y y' | z z' n n', so that a pair of
+  // atoms takes three two-wide products, |p - q|^2 <= r^2 as |q|^2 - 2 p.q <= r^2 - |p|^2 (rounding
+  // 1e-4 A^2 against the list radius' margin of 0.02 A^2); padding atoms have |q|^2 = 1e12.
   int imol[BLOCK];
   unsigned r0[3];
   {
@@ -355,17 +357,19 @@ __device__ __forceinline__ int build_block(const SystemDev &s, NbListDev &nb, do
     r0[0] = __shfl_sync(0xffffffffu, f.x, 0);
     r0[1] = __shfl_sync(0xffffffffu, f.y, 0);
     r0[2] = __shfl_sync(0xffffffffu, f.z, 0);
-    float px = 1e6f, py = 1e6f, pz = 1e6f;
+    float px = 0.f, py = 0.f, pz = 0.f, pn = PAD_NORM;
     if (m.x >= 0) {
       px = (float)(int)(f.x - r0[0]) * sL[0];
       py = (float)(int)(f.y - r0[1]) * sL[1];
       pz = (float)(int)(f.z - r0[2]) * sL[2];
+      pn = fmaf(pz, pz, fmaf(py, py, px * px));
     }
     const float qx = __shfl_down_sync(0xffffffffu, px, BLOCK / 2), qy = __shfl_down_sync(0xffffffffu, py, BLOCK / 2),
-                qz = __shfl_down_sync(0xffffffffu, pz, BLOCK / 2);
+                qz = __shfl_down_sync(0xffffffffu, pz, BLOCK / 2), qn = __shfl_down_sync(0xffffffffu, pn, BLOCK / 2);
+    __syncwarp();  // (the previous block's reads)
     if (lane < BLOCK / 2) {
-      ipos[2 * lane] = make_float4(px, qx, py, qy);
-      ipos[2 * lane + 1] = make_float4(pz, qz, 0.f, 0.f);
+      ipos[2 * lane] = make_float4(-2.f * px, -2.f * qx, -2.f * py, -2.f * qy);
+      ipos[2 * lane + 1] = make_float4(-2.f * pz, -2.f * qz, pn, qn);
     }
     __syncwarp();
   }
@@ -385,26 +389,27 @@ __device__ __forceinline__ int build_block(const SystemDev &s, NbListDev &nb, do
 #pragma unroll
       for (int t = 0; t < BLOCK / 2; t++) {
         const float4 a = ipos[2 * t], c = ipos[2 * t + 1];
-        const float qx[2] = {a.x, a.y}, qy[2] = {a.z, a.w}, qz[2] = {c.x, c.y};
+        const float qx[2] = {a.x, a.y}, qy[2] = {a.z, a.w}, qz[2] = {c.x, c.y}, qn[2] = {c.z, c.w};
 #pragma unroll
         for (int u = 0; u < 2; u++) {
-          float dx = px - qx[u], dy = py - qy[u], dz = pz - qz[u];
+          float dx = fmaf(0.5f, qx[u], px), dy = fmaf(0.5f, qy[u], py), dz = fmaf(0.5f, qz[u], pz);
           dx -= Lf[0] * rintf(dx * Lrf[0]);
           dy -= Lf[1] * rintf(dy * Lrf[1]);
           dz -= Lf[2] * rintf(dz * Lrf[2]);
-          near |= fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= rl2;
+          near |= (fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= rl2) & (qn[u] < PAD_NORM);
         }
       }
       return near;
     }
-    const float2 nx2 = make_float2(-px, -px), ny2 = make_float2(-py, -py), nz2 = make_float2(-pz, -pz);
+    const float2 px2 = make_float2(px, px), py2 = make_float2(py, py), pz2 = make_float2(pz, pz);
+    const float lim = rl2 - fmaf(pz, pz, fmaf(py, py, px * px));
 #pragma unroll
     for (int t = 0; t < BLOCK / 2; t++) {
       const float4 a = ipos[2 * t], c = ipos[2 * t + 1];
-      const float2 dx = __fadd2_rn(make_float2(a.x, a.y), nx2), dy = __fadd2_rn(make_float2(a.z, a.w), ny2),
-                   dz = __fadd2_rn(make_float2(c.x, c.y), nz2);
-      const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-      near |= (r2.x <= rl2) | (r2.y <= rl2);
+      const float2 d = __ffma2_rn(
+          make_float2(c.x, c.y), pz2,
+          __ffma2_rn(make_float2(a.z, a.w), py2, __ffma2_rn(make_float2(a.x, a.y), px2, make_float2(c.z, c.w))));
+      near |= (d.x <= lim) | (d.y <= lim);
     }
     return near;
   };
@@ -414,23 +419,26 @@ __device__ __forceinline__ int build_block(const SystemDev &s, NbListDev &nb, do
   // atoms of the listed candidate blocks, GROUPS blocks (32 slots) per pass
   auto atoms = [&]() {
     __syncwarp();
-    int sl = g < ncand ? cl[g] * BLOCK + li : -1;
-    int4 m = make_int4(-1, -1, 0, 0);
-    uint4 f = make_uint4(0, 0, 0, 0);
-    if (sl >= 0) {
-      m = nb.slot_meta[sl];
-      f = nb.slot_fx[sl];
-    }
-    for (int p = 0; p < ncand; p += GROUPS) {
-      const int q = p + GROUPS + g;
-      const int sl2 = q < ncand ? cl[q] * BLOCK + li : -1;
-      int4 m2 = make_int4(-1, -1, 0, 0);
-      uint4 f2 = make_uint4(0, 0, 0, 0);
-      if (sl2 >= 0) {
-        m2 = nb.slot_meta[sl2];
-        f2 = nb.slot_fx[sl2];
+    // (slots past the box's last atom are padding)
+    const int slot_end = b.blk0 * BLOCK + b.natoms;
+    auto fetch = [&](int q, int &sl, uint4 &f, int &mol) {
+      sl = q < ncand ? cl[q] * BLOCK + li : -1;
+      if (sl >= slot_end) sl = -1;
+      f = make_uint4(0, 0, 0, 0);
+      mol = -1;
+      if (sl >= 0) {
+        f = nb.slot_fx[sl];
+        mol = nb.slot_meta[sl].y;
       }
-      const bool take = m.x >= 0 && (multi || (gap2f(sL, cI, hI, f, make_uint4(0, 0, 0, 0)) <= rl2 && near_any(f)));
+    };
+    int sl, mol;
+    uint4 f;
+    fetch(g, sl, f, mol);
+    for (int p = 0; p < ncand; p += GROUPS) {
+      int sl2, mol2;
+      uint4 f2;
+      fetch(p + GROUPS + g, sl2, f2, mol2);
+      const bool take = sl >= 0 && (multi || near_any(f));
       const unsigned tm = __ballot_sync(0xffffffffu, take);
       const int n = __popc(tm);
       if (count + n > cap) {
@@ -440,12 +448,12 @@ __device__ __forceinline__ int build_block(const SystemDev &s, NbListDev &nb, do
       if (take) {
         bool same = false;
 #pragma unroll
-        for (int t = 0; t < BLOCK; t++) same |= m.y == imol[t];
+        for (int t = 0; t < BLOCK; t++) same |= mol == imol[t];
         out[count + __popc(tm & ((1u << lane) - 1u))] = same ? (sl | JSAME) : sl;
       }
       count += n;
       sl = sl2;
-      m = m2;
+      mol = mol2;
       f = f2;
     }
     ncand = 0;
