@@ -43,7 +43,7 @@ enum {
   CTL_BUILDS = 4,   // list builds so far (64 bits)
   CTL_PAIR = 6,     // the pair kernel's next unit and finished warps, two launches; zero between them
   CTL_VACUUM = 10,  // check the extent of vacuum boxes
-  CTL_CLAIM = 11,   // the list build's next group of blocks
+  CTL_CLAIM = 11,   // the list build's next claim
   CTL_UNITS = 12,   // pair units of boxes without and with lattice images
   CTL_WORDS = 16
 };
@@ -64,6 +64,7 @@ struct NbListDev {
                                // need lattice images from the end of the array, the others from
                                // the front (ctl[CTL_UNITS + 1] and ctl[CTL_UNITS] of them)
   int unit_cap;
+  int claim_blocks;            // consecutive blocks of a claim of the list build
   bool fills_chip;             // about a unit or more for every warp the chip holds
   int unit_tiles;              // most tiles of a unit: CLOSE_TILES .. UNIT_TILES
   int *status;                 // [4]: list / tile overflow, non-finite position, vacuum extent

@@ -7,6 +7,8 @@
 // and each block I gets a compacted list of atoms of blocks J > I that lie within the list
 // cutoff of I's bounding box.  The pair kernel then sees (I, 32 j-atoms) tiles; the pair set it
 // evaluates is exactly the reference's: every unordered pair once, minimal image, r^2 <= rc^2.
+#include <algorithm>
+
 #include "pmb_internal.h"
 #include "pmb_update.cuh"
 
@@ -496,54 +498,68 @@ __device__ __forceinline__ int build_block(const SystemDev &s, NbListDev &nb, do
   return tiles;
 }
 
-// CTAs claim groups of consecutive blocks from a counter, one block per warp, in ascending order (the
-// early blocks' lists are the longest).  The group's lists then join the pair kernel's work as units
-// of at most nb.unit_tiles tiles (about equal parts of a list, starting at multiples of CLOSE_TILES
-// tiles); a block of a box that keeps its list appends the units it has.  The units of boxes that
-// need lattice images grow from the end of the array.  Their order varies from build to build and
-// changes no result: the pair kernel closes its floating-point sums every CLOSE_TILES tiles of a
-// list.  One claim and one append per group: with three atomics per block the counters' words were
-// the bound of an ensemble's build (810,000 atoms, a quarter of the boxes rebuilt: 590 us a step).
+// Warps claim nb.claim_blocks consecutive blocks from a counter, in ascending order (the early
+// blocks' lists are the longest).  Their lists then join the pair kernel's work as units of at most
+// nb.unit_tiles tiles (about equal parts of a list, starting at multiples of CLOSE_TILES tiles); a
+// block of a box that keeps its list appends the units it has.  The units of boxes that need lattice
+// images grow from the end of the array.  Their order varies from build to build and changes no
+// result: the pair kernel closes its floating-point sums every CLOSE_TILES tiles of a list.
+// One claim and one append per several blocks in a large system: with three atomics per block the
+// counters' words were the bound of an ensemble's build (810,000 atoms, a quarter of the boxes
+// rebuilt: 590 us a step); one block per claim where there are few per warp, and no barrier between
+// warps (8 blocks to a CTA's claim: 13% of the warps' time).
 __global__ void __launch_bounds__(BL_THREADS, BL_MINB) k_build_lists(SystemDev s, NbListDev nb, double rlist2) {
-  constexpr int NW = BL_THREADS / 32;
-  __shared__ int cand_all[NW][BL_CAP];
-  __shared__ float4 ipos_all[NW][BLOCK];
-  __shared__ int group, units[NW], base[2];
+  __shared__ int cand_all[BL_THREADS / 32][BL_CAP];
+  __shared__ float4 ipos_all[BL_THREADS / 32][BLOCK];
   if (!nb.ctl[CTL_REBUILD]) return;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, per = nb.unit_tiles / CLOSE_TILES;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, G = nb.claim_blocks, per = nb.unit_tiles / CLOSE_TILES;
   for (;;) {
-    if (threadIdx.x == 0) group = (int)atomicAdd(nb.ctl + CTL_CLAIM, 1u);
-    __syncthreads();
-    if (group * NW >= nb.nblk_total) return;
-    const int I = group * NW + w;
-    int tiles = 0, multi = 0;
-    if (I < nb.nblk_total) {
-      const int bi = nb.blk_box[I];
+    int I0 = 0;
+    if (lane == 0) I0 = (int)atomicAdd(nb.ctl + CTL_CLAIM, 1u) * G;
+    I0 = __shfl_sync(0xffffffffu, I0, 0);
+    if (I0 >= nb.nblk_total) return;
+    const int n = min(G, nb.nblk_total - I0);
+    int tiles = 0, multi = 0;  // lane q: block I0 + q
+    for (int q = 0; q < n; q++) {
+      const int I = I0 + q, bi = nb.blk_box[I];
       const BoxDev &b = s.box[bi];
-      multi = b.multi_image != 0;
-      tiles = nb.box_rb[bi] ? build_block(s, nb, rlist2, I, b, cand_all[w], ipos_all[w]) : nb.jcount[I];
+      const int t = nb.box_rb[bi] ? build_block(s, nb, rlist2, I, b, cand_all[w], ipos_all[w]) : nb.jcount[I];
+      if (lane == q) {
+        tiles = t;
+        multi = b.multi_image != 0;
+      }
     }
     const int nc = (tiles + CLOSE_TILES - 1) / CLOSE_TILES, nu = (nc + per - 1) / per;
-    if (lane == 0) units[w] = 2 * nu + multi;
-    __syncthreads();
-    if (threadIdx.x < 2) {  // the group's units without and with lattice images
-      int n = 0;
-      for (int k = 0; k < NW; k++)
-        if ((units[k] & 1) == (int)threadIdx.x) n += units[k] >> 1;
-      base[threadIdx.x] = n ? (int)atomicAdd(nb.ctl + CTL_UNITS + threadIdx.x, (unsigned)n) : 0;
+    int at = 0;
+    const unsigned all = __ballot_sync(0xffffffffu, nu > 0), images = __ballot_sync(0xffffffffu, multi != 0);
+    for (int kind = 0; kind < 2; kind++) {  // units without and with lattice images
+      if (!(all & (kind ? images : ~images))) continue;
+      const int mine = multi == kind ? nu : 0;
+      int sum = mine;  // inclusive sum over the lanes
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += y;
+      }
+      int base = 0;
+      if (lane == 31) base = (int)atomicAdd(nb.ctl + CTL_UNITS + kind, (unsigned)sum);
+      base = __shfl_sync(0xffffffffu, base, 31);
+      if (multi == kind) at = base + sum - mine;
     }
-    __syncthreads();
-    int at = base[multi];
-    for (int k = 0; k < w; k++)
-      if ((units[k] & 1) == multi) at += units[k] >> 1;
-    for (int p = lane; p < nu; p += 32) {
-      const int k0 = (int)((long long)nc * p / nu) * CLOSE_TILES;
-      const int k1 = min(tiles, (int)((long long)nc * (p + 1) / nu) * CLOSE_TILES);
-      const int u = at + p;  // (within the array: it is sized for full lists)
-      nb.units[multi ? nb.unit_cap - 1 - u : u] = make_int4(I, k0, k1 - k0, nb.jcap_off[I] + k0 * JCHUNK);
+    for (int q = 0; q < n; q++) {
+      const int nuq = __shfl_sync(0xffffffffu, nu, q), ncq = __shfl_sync(0xffffffffu, nc, q),
+                tq = __shfl_sync(0xffffffffu, tiles, q), atq = __shfl_sync(0xffffffffu, at, q);
+      const bool mq = (images >> q) & 1u;
+      for (int p = lane; p < nuq; p += 32) {
+        const int k0 = (int)((long long)ncq * p / nuq) * CLOSE_TILES;
+        const int k1 = min(tq, (int)((long long)ncq * (p + 1) / nuq) * CLOSE_TILES);
+        const int u = atq + p;  // (within the array: it is sized for full lists)
+        nb.units[mq ? nb.unit_cap - 1 - u : u] = make_int4(I0 + q, k0, k1 - k0, nb.jcap_off[I0 + q] + k0 * JCHUNK);
+      }
     }
   }
 }
+constexpr int CLAIMS_PER_WARP = 4;  // at least, before a claim takes more than one block
 
 // One CTA per box up to SORT_SMALL atoms, and up to SORT_MANY when the boxes alone fill the chip.
 constexpr int SORT_SMALL = 3072, SORT_MANY = 32768;
@@ -581,6 +597,7 @@ int nblist_lists(const SystemDev &s, NbListDev &nb, double list_cutoff, cudaStre
   }
   // as many blocks as fit at once (blocks are claimed), so that the exit without a rebuild is short
   const int warps = BL_THREADS / 32, need = (nb.nblk_total + warps - 1) / warps;
+  nb.claim_blocks = std::max(1, std::min(8, nb.nblk_total / (nb.n_sm * BL_MINB * warps * CLAIMS_PER_WARP)));
   k_build_lists<<<need < nb.n_sm * BL_MINB ? need : nb.n_sm * BL_MINB, BL_THREADS, 0, st>>>(s, nb, list_cutoff * list_cutoff);
   return 0;
 }
