@@ -782,30 +782,6 @@ __device__ __forceinline__ double2 unit_root(int N, int k) {
     case 131: return make_double2(-0.70710678118654746, 0.70710678118654757);
     case 133: return make_double2(-0.70710678118654768, -0.70710678118654746);
     case 135: return make_double2(0.70710678118654735, -0.70710678118654768);
-    case 145: return make_double2(0.76604444311897801, 0.64278760968653925);
-    case 146: return make_double2(0.17364817766693041, 0.98480775301220802);
-    case 147: return make_double2(-0.49999999999999978, 0.86602540378443871);
-    case 148: return make_double2(-0.93969262078590832, 0.34202014332566888);
-    case 149: return make_double2(-0.93969262078590843, -0.34202014332566866);
-    case 150: return make_double2(-0.50000000000000044, -0.86602540378443837);
-    case 151: return make_double2(0.17364817766692997, -0.98480775301220813);
-    case 152: return make_double2(0.76604444311897779, -0.64278760968653958);
-    case 161: return make_double2(0.80901699437494745, 0.58778525229247314);
-    case 162: return make_double2(0.30901699437494745, 0.95105651629515353);
-    case 163: return make_double2(-0.30901699437494734, 0.95105651629515364);
-    case 164: return make_double2(-0.80901699437494734, 0.58778525229247325);
-    case 166: return make_double2(-0.80901699437494756, -0.58778525229247303);
-    case 167: return make_double2(-0.30901699437494756, -0.95105651629515353);
-    case 168: return make_double2(0.30901699437494723, -0.95105651629515364);
-    case 169: return make_double2(0.80901699437494734, -0.58778525229247336);
-    case 193: return make_double2(0.86602540378443871, 0.49999999999999994);
-    case 194: return make_double2(0.50000000000000011, 0.8660254037844386);
-    case 196: return make_double2(-0.49999999999999978, 0.86602540378443871);
-    case 197: return make_double2(-0.86602540378443871, 0.49999999999999994);
-    case 199: return make_double2(-0.86602540378443882, -0.49999999999999972);
-    case 200: return make_double2(-0.50000000000000044, -0.86602540378443837);
-    case 202: return make_double2(0.50000000000000011, -0.8660254037844386);
-    case 203: return make_double2(0.86602540378443837, -0.50000000000000044);
     default: return make_double2(0.0, 0.0);
   }
 }
@@ -844,10 +820,7 @@ template <int R, int SIGN, typename T2>
 __device__ __forceinline__ void dft_reg(T2 *v) {
   if constexpr (R <= 5) dft_small_any<R>(v, SIGN);
   else if constexpr (R == 6) dft_composite<2, 3, SIGN>(v);
-  else if constexpr (R == 8) dft_composite<2, 4, SIGN>(v);
-  else if constexpr (R == 9) dft_composite<3, 3, SIGN>(v);
-  else if constexpr (R == 10) dft_composite<2, 5, SIGN>(v);
-  else dft_composite<3, 4, SIGN>(v);
+  else dft_composite<2, 4, SIGN>(v);
 }
 
 // One in-place stage of a length-n transform on sub-blocks of m = R mq points, butterfly (b, j):
@@ -970,6 +943,8 @@ __device__ __forceinline__ void col_infl(const PlaneCtx<T2> &p, const T *th, dou
   }
 }
 
+// (Radices of 9, 10 and 12 save a stage of most lengths, but the code of the stages then outgrew the
+// instruction cache: fetches were the top stall, and a 98,304-atom run took 7308 us, now 7053.)
 #define PLANE_RADIX(R, CALL) \
   switch (R) {               \
     case 2: CALL(2); break;  \
@@ -977,15 +952,12 @@ __device__ __forceinline__ void col_infl(const PlaneCtx<T2> &p, const T *th, dou
     case 4: CALL(4); break;  \
     case 5: CALL(5); break;  \
     case 6: CALL(6); break;  \
-    case 8: CALL(8); break;  \
-    case 9: CALL(9); break;  \
-    case 10: CALL(10); break; \
-    default: CALL(12); break; \
+    default: CALL(8); break; \
   }
 
 // One kz plane of the half spectrum per CTA, in shared memory between its two passes over memory:
 // forward y and x transforms, influence function with energy and virial (Grid.h:236-341), inverse x
-// and y.  Two or three register stages a direction (96 = 8 x 12), so about seven barriers; the
+// and y.  Two or three register stages a direction (96 = 6 x 4 x 4), so about ten barriers; the
 // three kernels before it had four or five each way and moved the spectrum through memory six
 // times.  Few CTAs (49 at 96^3) of long latency, which suits running beside the pair kernel: alone
 // 20 -> 13 us at 72^3, 36 -> 31 us at 125^3, 12 -> 8 us at 20^3, and two launches fewer.
@@ -1231,7 +1203,7 @@ int pme_line_capacity() { return LMAXE; }
 
 bool pme_plane_radices(int n, std::vector<int> &rad) {
   // the fewest stages, then the smallest sum of radices
-  static const int R[] = {12, 10, 9, 8, 6, 5, 4, 3, 2};
+  static const int R[] = {8, 6, 5, 4, 3, 2};
   std::vector<int> best, cur;
   int best_sum = 0;
   std::function<void(int, int, int)> search = [&](int m, int from, int sum) {
@@ -1243,7 +1215,7 @@ bool pme_plane_radices(int n, std::vector<int> &rad) {
       return;
     }
     if (!best.empty() && cur.size() >= best.size()) return;
-    for (int k = from; k < 9; k++)
+    for (int k = from; k < 6; k++)
       if (m % R[k] == 0) {
         cur.push_back(R[k]);
         search(m / R[k], k, sum + R[k]);
