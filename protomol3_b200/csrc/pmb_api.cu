@@ -648,12 +648,16 @@ int ensure_side_stream(pmb_system *s) {
 // culling), or 0 when no force of the set uses the list (no pair term, no PME reciprocal term).
 double list_radius(pmb_system *s, pmb_force *const *fs, int n) {
   double rl = 0.0;
-  bool need = false;
+  bool pairs = false, slots = false;
   for (int i = 0; i < n; i++) {
     rl = std::max(rl, force_pair_cutoff(fs[i]));
-    need |= pair_jobs(s, fs + i, 1, 0).size() > 0 || (fs[i]->kind == PMB_FORCE_PME && fs[i]->d.reciprocal);
+    pairs |= pair_jobs(s, fs + i, 1, 0).size() > 0;
+    slots |= fs[i]->kind == PMB_FORCE_PME && fs[i]->d.reciprocal;
   }
-  return need ? std::max(rl, 1.0) + s->skin + 1e-3 : 0.0;
+  // (a radius no pair set has where only the slots are needed: their builds make no j-lists, so a
+  // pair set that follows on the same system must build anew)
+  if (!pairs) return slots ? 0.5 + s->skin + 1e-3 : 0.0;
+  return std::max(rl, 1.0) + s->skin + 1e-3;
 }
 
 int enqueue_forces(pmb_system *s, pmb_force *const *fs, int n, int virial, bool updated = false) {
@@ -728,7 +732,7 @@ int enqueue_forces(pmb_system *s, pmb_force *const *fs, int n, int virial, bool 
       CK(cudaStreamWaitEvent(s->terms, need_pme_slots ? s->ev_fork : s->ev_slots, 0));
       launch_all_atom_terms();
     }
-    nblist_lists(sd, s->nb, rlist, st);
+    if (!jobs.empty()) nblist_lists(sd, s->nb, rlist, st);
     mark(s, "nblist");
   }
   if (!split) {
