@@ -18,10 +18,7 @@
 #include <string>
 #include <vector>
 
-// PME transform work items per CTA (z-lines <= 16; rows / columns capped by the line buffer).
-#ifndef PME_ZLINES
-#define PME_ZLINES 8
-#endif
+// PME row / column work items per CTA (capped by the line buffer).
 #ifndef PME_YROWS
 #define PME_YROWS 4
 #endif
@@ -1357,7 +1354,8 @@ pmb_force *pmb_force_create(pmb_system *s, const pmb_force_desc *d) {
     std::vector<int4> ywork, xwork;
     long long g0 = 0, c0 = 0;
     const int lcap = pme_line_capacity();
-    int zbuf = 1, lbuf = 1;
+    size_t zsmem = 0;
+    int lbuf = 1;
     std::vector<double> theta;
     // the plane kernel takes every plan whose planes fit shared memory
     std::vector<int2> pwork;
@@ -1370,6 +1368,10 @@ pmb_force *pmb_force_create(pmb_system *s, const pmb_force_desc *d) {
       plane_points += (double)nx * ny / nbox;
     }
     const bool planes = psmem <= (size_t)PLANE_SMEM_MAX;
+    // z-lines a CTA: eight where sixteen would leave fewer than four CTAs an SM (216 waters: 25
+    // steps 975 us with eight, 989 with all 20 lines of a plane in one CTA; 96^3, just under the line:
+    // the same either way)
+    const int zlines = plane_points * nbox < 16.0 * 4 * 148 ? 8 : 16;
     double th0[8];
     bspline_h(P, 0.0, th0);
     for (int bi = 0; bi < nbox; bi++) {
@@ -1398,7 +1400,7 @@ pmb_force *pmb_force_create(pmb_system *s, const pmb_force_desc *d) {
         perm.resize(tw.size());
         for (int j = 0; j < n; j++) perm[pl.tw0[k] + j] = j;
         std::vector<int> pr;
-        if (planes && k < 2 && pme_plane_radices(n, pr)) {
+        if ((planes || k == 2) && pme_plane_radices(n, pr)) {
           pl.prad0[k] = (int)pradix.size();
           pl.npr[k] = (int)pr.size();
           pradix.insert(pradix.end(), pr.begin(), pr.end());
@@ -1410,7 +1412,7 @@ pmb_force *pmb_force_create(pmb_system *s, const pmb_force_desc *d) {
               rest %= m;
               mul *= R;
             }
-            perm[pl.tw0[k] + pos] = idx;
+            perm[pl.tw0[k] + (k == 2 ? idx : pos)] = k == 2 ? pos : idx;
           }
         }
         // influence factor B(m) exp(-pi^2 m^2/alpha^2) (Grid.h:523-571, dftmod :588-600)
@@ -1435,14 +1437,12 @@ pmb_force *pmb_force_create(pmb_system *s, const pmb_force_desc *d) {
       pl.fac = M_PI * M_PI / (f->alpha * f->alpha);
       g0 += (long long)pl.n[0] * pl.n[1] * pl.n[2];
       c0 += (long long)(pl.n[2] / 2 + 1) * pl.n[0] * pl.n[1];
-      // small work items (PME_ZLINES z-lines = PME_ZLINES / 2 packed complex lines, PME_YROWS
-      // y-lines, PME_XCOLS x-lines per CTA): many CTAs in flight hide the latency of the
-      // shared-memory stages
+      // small work items: many CTAs in flight hide the latency of the shared-memory stages
       for (int x = 0; x < pl.n[0]; x++)
-        for (int y0 = 0; y0 < pl.n[1]; y0 += PME_ZLINES) {
-          const int cnt = std::min(PME_ZLINES, pl.n[1] - y0);
+        for (int y0 = 0; y0 < pl.n[1]; y0 += zlines) {
+          const int cnt = std::min(zlines, pl.n[1] - y0);
           zwork.push_back(make_int4(bi, x, y0, cnt));
-          zbuf = std::max(zbuf, (cnt + 1) / 2 * pl.n[2]);
+          zsmem = std::max(zsmem, pme_z_smem(pl.n[2], zlines, s->precision));
         }
       const int rows = std::max(1, std::min(PME_YROWS, lcap / pl.n[1])),
                 cols = std::max(1, std::min(PME_XCOLS, lcap / pl.n[0]));
@@ -1534,7 +1534,8 @@ pmb_force *pmb_force_create(pmb_system *s, const pmb_force_desc *d) {
     pm.nywork = (int)ywork.size();
     pm.xwork = dx;
     pm.nxwork = (int)xwork.size();
-    pm.zbuf = zbuf;
+    pm.zsmem = zsmem;
+    pm.zpairs = zlines / 2;
     pm.lbuf = lbuf;
     // the warp-shuffle transforms take lines of 32 R points (R <= 5), the same R in every box
     auto warp_r = [&](int d) {
@@ -1549,7 +1550,6 @@ pmb_force *pmb_force_create(pmb_system *s, const pmb_force_desc *d) {
     // (one row per warp of a 4-warp block, one column per warp of an 8-warp block)
     pm.wy = PME_YROWS <= 4 ? warp_r(1) : 0;
     pm.wx = PME_XCOLS * 32 <= PME_WX_THREADS ? warp_r(0) : 0;
-    pm.wz = PME_ZLINES <= 8 ? warp_r(2) : 0;  // (two lines per warp of a 4-warp block)
     pm.qgrid = f->a.get<long long>(g0);
     pm.rgrid = s->precision ? (void *)f->a.get<float>(g0) : (void *)f->a.get<double>(g0);
     pm.cgrid = s->precision ? (void *)f->a.get<float2>(c0) : (void *)f->a.get<double2>(c0);

@@ -155,7 +155,7 @@ struct PmeBoxPlan {
   int tw0[3];         // offsets of twiddle tables (complex elements)
   int inf0[3];        // offsets of influence tables
   int rad0[3], nrad[3];
-  int prad0[2], npr[2];  // radices of the plane kernel's x and y transforms
+  int prad0[3], npr[3];  // radices of the register-stage transforms (x and y: plane kernel)
   double hr[3];       // n / L
   double mr[3];       // 1 / L
   double piVr, fac;   // 1/(pi V), pi^2 / alpha^2
@@ -183,12 +183,13 @@ struct PmeDev {
   int npwork, pthreads;
   size_t psmem;
   const int *pradix;          // its radices
-  const int *perm;            // index at each position of its transformed lines (offsets tw0); theta
-                              // is in that order then
-  int zbuf, lbuf;             // complex elements per ping-pong buffer of the z / line kernels
-  int wz, wy, wx;             // R > 0: every box's z (y, x) lines have 32 R points and the inverse
-                              // z pass (the y passes, the x pass) run the warp-shuffle transforms;
-                              // 0: the shared-memory ones
+  const int *perm;            // (offsets tw0) x and y: index at each position of the plane kernel's
+                              // transformed lines, theta is in that order then; z: position of index
+  int zpairs;                 // packed lines of a full work item of the z kernels
+  size_t zsmem;               // shared memory of the z kernels
+  int lbuf;                   // complex elements per ping-pong buffer of the line kernels
+  int wy, wx;                 // R > 0: every box's y (x) lines have 32 R points and the y passes (the
+                              // x pass) run the warp-shuffle transforms; 0: the shared-memory ones
   double alpha, a2pi;
   int virial;
 };
@@ -207,6 +208,16 @@ constexpr int PLANE_MAX_THREADS = 512;
 constexpr int PLANE_SMEM_MAX = 227 * 1024;
 bool pme_plane_radices(int n, std::vector<int> &radices);
 size_t pme_plane_smem(int nx, int ny, int precision);
+constexpr int Z_SMEM_MAX = 48 * 1024;  // z kernels: 16 lines of 256 points in FP64 take 37 KB
+// Stride of a packed line in the z kernels' buffer.  Consecutive threads take the same point of
+// consecutive lines: with 16 / pairs + 16 i eight-byte numbers (an odd count of sixteen-byte ones)
+// between lines a half (quarter) warp falls on different banks, whatever the stage.
+__host__ __device__ inline int z_line_stride(int nz, int pairs, bool f32) {
+  if (!f32) return nz | 1;
+  const int off = pairs > 8 ? 1 : pairs > 4 ? 2 : 4;
+  return nz + ((off - nz) & 15);
+}
+size_t pme_z_smem(int nz, int lines, int precision);
 // Exact Ewald reciprocal sum of one box (pmb_ewald.cu): S, C [nk] and the box's forces in fout.
 int ewald_recip_launch(const double *pos, const double *charge, int atom0, int n, const double3 *kv,
                        const double *a, int nk, double *S, double *Cc, double *fout, cudaStream_t st);

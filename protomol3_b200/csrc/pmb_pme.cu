@@ -362,91 +362,6 @@ __global__ void k_gather(const SystemDev s, NbListDev nb, PmeDev pm) {
   }
 }
 
-constexpr int ZT = 128;         // threads of the z-line kernels
-constexpr int ZMAXE = 8 * 256;  // 8 packed line pairs x nz <= 256, per ping-pong buffer
-
-template <typename T>
-__global__ void __launch_bounds__(ZT, 8) k_fft_z_fwd(PmeDev pm) {
-  using T2 = typename C2<T>::t;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int4 wk = pm.zwork[blockIdx.x];
-  const PmeBoxPlan &pl = pm.plan[wk.x];
-  const int nx = pl.n[0], ny = pl.n[1], nz = pl.n[2], x = wk.y, y0 = wk.z, cnt = wk.w;
-  const int npair = (cnt + 1) / 2;
-  T2 *tw = reinterpret_cast<T2 *>(smem_raw);
-  T2 *buf = tw + 256, *tmp = buf + pm.zbuf;
-  for (int k = threadIdx.x; k < nz; k += ZT) {
-    if constexpr (sizeof(T) == 4) tw[k] = pm.twiddlef[pl.tw0[2] + k];
-    else tw[k] = pm.twiddle[pl.tw0[2] + k];
-  }
-  long long *g = pm.qgrid + pl.grid0 + ((long long)x * ny + y0) * nz;
-  // the work item's lines are one contiguous run of cnt * nz grid values: read them all (no
-  // store in between, so the loads overlap), then clear the charge grid for the next step, each
-  // thread the values it read itself
-  const int nrun = cnt * nz;
-  const float rnz = rcpf(nz), rnp = rcpf(npair);
-#pragma unroll 4
-  for (int e = threadIdx.x; e < npair * 2 * nz; e += ZT) {
-    const long long q = e < nrun ? __ldcs(g + e) : 0ll;
-    const int line = divf(e, rnz), z = e - line * nz;
-    T *dst = reinterpret_cast<T *>(buf + (line >> 1) * nz + z);
-    dst[line & 1] = T((double)q * (1.0 / GRID_SCALE));
-  }
-  for (int e = threadIdx.x; e < nrun; e += ZT) g[e] = 0;
-  __syncthreads();
-  const T2 *res = fft_lines(buf, tmp, nz, npair, nz, 1, pm.radix + pl.rad0[2], pl.nrad[2], tw, -1);
-  const int nh = nz / 2 + 1;
-  T2 *C = reinterpret_cast<T2 *>(pm.cgrid) + pl.cgrid0;
-  for (int e = threadIdx.x; e < npair * nh; e += ZT) {
-    const int k = divf(e, rnp), pi = e - k * npair;
-    T2 zk = res[pi * nz + k], zn = res[pi * nz + (k == 0 ? 0 : nz - k)];
-    // X = (Z_k + conj(Z_{n-k})) / 2, Y = -i/2 (Z_k - conj(Z_{n-k}))
-    T2 X = cmk(T(0.5) * (zk.x + zn.x), T(0.5) * (zk.y - zn.y));
-    T2 Y = cmk(T(0.5) * (zk.y + zn.y), T(-0.5) * (zk.x - zn.x));
-    T2 *row = C + ((long long)k * nx + x) * ny + y0 + 2 * pi;
-    row[0] = X;
-    if (2 * pi + 1 < cnt) row[1] = Y;
-  }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(ZT, 8) k_fft_z_inv(PmeDev pm) {
-  using T2 = typename C2<T>::t;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int4 wk = pm.zwork[blockIdx.x];
-  const PmeBoxPlan &pl = pm.plan[wk.x];
-  const int nx = pl.n[0], ny = pl.n[1], nz = pl.n[2], x = wk.y, y0 = wk.z, cnt = wk.w;
-  const int npair = (cnt + 1) / 2, nh = nz / 2 + 1;
-  T2 *tw = reinterpret_cast<T2 *>(smem_raw);
-  T2 *buf = tw + 256, *tmp = buf + pm.zbuf;
-  for (int k = threadIdx.x; k < nz; k += ZT) {
-    if constexpr (sizeof(T) == 4) tw[k] = pm.twiddlef[pl.tw0[2] + k];
-    else tw[k] = pm.twiddle[pl.tw0[2] + k];
-  }
-  const T2 *C = reinterpret_cast<const T2 *>(pm.cgrid) + pl.cgrid0;
-  const float rnz = rcpf(nz), rnp = rcpf(npair);
-  for (int e = threadIdx.x; e < npair * nh; e += ZT) {
-    const int k = divf(e, rnp), pi = e - k * npair;
-    const T2 *row = C + ((long long)k * nx + x) * ny + y0 + 2 * pi;
-    T2 X = row[0];
-    T2 Y = (2 * pi + 1 < cnt) ? row[1] : cmk(T(0), T(0));
-    if (k == 0 || (2 * k == nz)) {
-      X.y = T(0);
-      Y.y = T(0);
-    }
-    buf[pi * nz + k] = cmk(X.x - Y.y, X.y + Y.x);
-    if (k > 0 && 2 * k != nz) buf[pi * nz + nz - k] = cmk(X.x + Y.y, Y.x - X.y);
-  }
-  __syncthreads();
-  const T2 *res = fft_lines(buf, tmp, nz, npair, nz, 1, pm.radix + pl.rad0[2], pl.nrad[2], tw, +1);
-  T *R = reinterpret_cast<T *>(pm.rgrid) + pl.grid0 + ((long long)x * ny + y0) * nz;
-  for (int e = threadIdx.x; e < cnt * nz; e += ZT) {
-    const int line = divf(e, rnz), z = e - line * nz;
-    T2 v = res[(line >> 1) * nz + z];
-    R[(long long)line * nz + z] = (line & 1) ? v.y : v.x;
-  }
-}
-
 template <int THREADS, typename T>
 __device__ __forceinline__ double block_sum(double v, double *red) {
   v = warp_sum(v);
@@ -1063,55 +978,151 @@ __global__ void __launch_bounds__(PLANE_MAX_THREADS) k_fft_plane(const SystemDev
   }
 }
 
-constexpr int WZ = 128;  // threads of the warp z kernel: up to 8 lines (4 pairs) per work item
+constexpr int ZT = 128;  // threads of the z-line kernels
 
-// z-lines with n_z = 32 R, c2r (as k_fft_z_inv): the z_inv work item's lines (x, y0 .. y0 + cnt)
-// as cnt / 2 packed pairs, one per warp, rebuilt from the half spectrum (read in rows of cnt
-// consecutive y through shared memory), written to the real potential grid [x][y][z].  (The r2c
-// forward pass keeps the shared-memory kernel: its warp form was no faster.)
-template <typename T, int R>
-__global__ void __launch_bounds__(WZ) k_fft_z_inv_warp(PmeDev pm) {
+// Shared memory of a z kernel: factors, positions, lines, radices (read before the first barrier with
+// the rest, so that no stage waits for memory).
+template <typename T2>
+struct ZLines {
+  PlaneCtx<T2> p;       // rows: the packed lines, of nz points
+  const int *pos;       // position of index k in a transformed line
+  const int *rad;
+};
+template <typename T, typename T2>
+__device__ __forceinline__ ZLines<T2> z_lines(const PmeDev &pm, const PmeBoxPlan &pl, int npair, unsigned char *smem) {
+  const int nz = pl.n[2];
+  ZLines<T2> z;
+  T2 *tw = reinterpret_cast<T2 *>(smem);
+  int *pos = reinterpret_cast<int *>(tw + nz + (nz & 1));
+  z.p.twx = nullptr;
+  z.p.twy = tw;
+  z.p.C = nullptr;
+  z.p.nx = npair;
+  z.p.ny = nz;
+  z.p.ld = z_line_stride(nz, pm.zpairs, sizeof(T) == 4);
+  z.p.buf = reinterpret_cast<T2 *>(pos + (nz + 3) / 4 * 4);
+  z.pos = pos;
+  __shared__ int rad[8];  // 2^a 3^b 5^c <= 256 in radices up to 8
+  if (threadIdx.x < pl.npr[2]) rad[threadIdx.x] = pm.pradix[pl.prad0[2] + threadIdx.x];
+  z.rad = rad;
+  for (int k = threadIdx.x; k < nz; k += ZT) {
+    if constexpr (sizeof(T) == 4) tw[k] = pm.twiddlef[pl.tw0[2] + k];
+    else tw[k] = pm.twiddle[pl.tw0[2] + k];
+    pos[k] = pm.perm[pl.tw0[2] + k];
+  }
+  return z;
+}
+
+// r2c: the work item's lines of the fixed-point charge grid, two real lines packed per complex line,
+// in the plane kernel's in-place register stages; the half spectrum leaves as [kz][x][y].  Latency
+// bound (load, two to four stages, store, with a barrier between each).  Against shared-memory stages
+// with a table lookup per point (both directions): 14.6 + 12.1 -> 12.6 + 9.7 us at 125^3, 186 + 168
+// -> 152 + 130 us for 256 boxes of 15 to 40 points; 9.2 + 16.9 -> 9.7 + 16.5 us at 96^3 beside the
+// pair kernel (there the inverse had a form of one line per warp).  A box of 216 waters pays 0.6 us
+// a step (38.5) for the larger code.
+template <typename T>
+__global__ void __launch_bounds__(ZT, sizeof(T) == 4 ? 8 : 4) k_fft_z_fwd(PmeDev pm) {
   using T2 = typename C2<T>::t;
-  constexpr int nz = 32 * R, nh = nz / 2 + 1, NP = WZ / 32;
-  __shared__ T2 zl[NP][nz];
-  __shared__ T2 in[nh * 2 * NP];  // [k][line]
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   const int4 wk = pm.zwork[blockIdx.x];
   const PmeBoxPlan &pl = pm.plan[wk.x];
-  const int nx = pl.n[0], ny = pl.n[1], x = wk.y, y0 = wk.z, cnt = wk.w;
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const T2 *C = reinterpret_cast<const T2 *>(pm.cgrid) + pl.cgrid0;
-  for (int e = threadIdx.x; e < nh * cnt; e += WZ) {
-    const int k = e / cnt, c = e - k * cnt;
-    in[k * 2 * NP + c] = C[((long long)k * nx + x) * ny + y0 + c];
+  const int nx = pl.n[0], ny = pl.n[1], nz = pl.n[2], x = wk.y, y0 = wk.z, cnt = wk.w;
+  const int npair = (cnt + 1) / 2;
+  const ZLines<T2> z = z_lines<T, T2>(pm, pl, npair, smem_raw);
+  long long *g = pm.qgrid + pl.grid0 + ((long long)x * ny + y0) * nz;
+  const float rnz = rcpf(nz), rnp = rcpf(npair);
+#pragma unroll 4
+  for (int e = threadIdx.x; e < npair * nz; e += ZT) {
+    const int pi = divf(e, rnz), k = e - pi * nz;
+    long long *ga = g + e + pi * nz;
+    const bool two = 2 * pi + 1 < cnt;
+    const long long qa = __ldcs(ga), qb = two ? __ldcs(ga + nz) : 0ll;
+    z.p.buf[pi * z.p.ld + k] = cmk(T((double)qa * (1.0 / GRID_SCALE)), T((double)qb * (1.0 / GRID_SCALE)));
   }
   __syncthreads();
-  if (2 * w >= cnt) return;  // warp-uniform; no block barrier below
-  const bool two = 2 * w + 1 < cnt;
-  for (int k = lane; k < nh; k += 32) {
-    T2 X = in[k * 2 * NP + 2 * w];
-    T2 Y = two ? in[k * 2 * NP + 2 * w + 1] : cmk(T(0), T(0));
-    if (k == 0 || 2 * k == nz) {
+  int m = nz;
+  for (int q = 0; q < pl.npr[2]; q++) {
+#define Z_FWD(R) row_stage<R, -1, false>(z.p, m)
+    PLANE_RADIX(z.rad[q], Z_FWD)
+#undef Z_FWD
+    m /= z.rad[q];
+    __syncthreads();
+  }
+  const int nh = nz / 2 + 1;
+  T2 *C = reinterpret_cast<T2 *>(pm.cgrid) + pl.cgrid0;
+  const bool vec = ((ny | cnt | pl.cgrid0) & 1) == 0;  // both lines of a pair at an aligned 16 bytes
+  for (int e = threadIdx.x; e < npair * nh; e += ZT) {
+    const int k = divf(e, rnp), pi = e - k * npair;
+    const T2 *L = z.p.buf + pi * z.p.ld;
+    const T2 zk = L[z.pos[k]], zn = L[z.pos[k == 0 ? 0 : nz - k]];
+    // X = (Z_k + conj(Z_{n-k})) / 2, Y = -i/2 (Z_k - conj(Z_{n-k}))
+    const T2 X = cmk(T(0.5) * (zk.x + zn.x), T(0.5) * (zk.y - zn.y));
+    const T2 Y = cmk(T(0.5) * (zk.y + zn.y), T(-0.5) * (zk.x - zn.x));
+    T2 *row = C + ((long long)k * nx + x) * ny + y0 + 2 * pi;
+    if constexpr (sizeof(T) == 4) {
+      if (vec) {
+        *reinterpret_cast<float4 *>(row) = make_float4(X.x, X.y, Y.x, Y.y);
+        continue;
+      }
+    }
+    row[0] = X;
+    if (2 * pi + 1 < cnt) row[1] = Y;
+  }
+  // the charge grid cleared for the next step
+  for (int e = threadIdx.x; e < cnt * nz; e += ZT) g[e] = 0;
+}
+
+// c2r: the packed lines rebuilt from the half spectrum, in the order that the inverse stages take.
+template <typename T>
+__global__ void __launch_bounds__(ZT, sizeof(T) == 4 ? 8 : 4) k_fft_z_inv(PmeDev pm) {
+  using T2 = typename C2<T>::t;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int4 wk = pm.zwork[blockIdx.x];
+  const PmeBoxPlan &pl = pm.plan[wk.x];
+  const int nx = pl.n[0], ny = pl.n[1], nz = pl.n[2], x = wk.y, y0 = wk.z, cnt = wk.w;
+  const int npair = (cnt + 1) / 2, nh = nz / 2 + 1;
+  const ZLines<T2> z = z_lines<T, T2>(pm, pl, npair, smem_raw);
+  const int *pos = pm.perm + pl.tw0[2];  // (not through shared memory: no barrier before the loads)
+  const T2 *C = reinterpret_cast<const T2 *>(pm.cgrid) + pl.cgrid0;
+  const float rnz = rcpf(nz), rnp = rcpf(npair);
+  const bool vec = ((ny | cnt | pl.cgrid0) & 1) == 0;  // both lines of a pair at an aligned 16 bytes
+#pragma unroll 2
+  for (int e = threadIdx.x; e < npair * nh; e += ZT) {
+    const int k = divf(e, rnp), pi = e - k * npair;
+    const T2 *row = C + ((long long)k * nx + x) * ny + y0 + 2 * pi;
+    T2 X, Y;
+    if (sizeof(T) == 4 && vec) {
+      const float4 v = *reinterpret_cast<const float4 *>(row);
+      X = cmk(T(v.x), T(v.y));
+      Y = cmk(T(v.z), T(v.w));
+    } else {
+      X = row[0];
+      Y = (2 * pi + 1 < cnt) ? row[1] : cmk(T(0), T(0));
+    }
+    if (k == 0 || (2 * k == nz)) {
       X.y = T(0);
       Y.y = T(0);
     }
     // Z_k = X_k + i Y_k and Z_{n-k} = conj(X_k) + i conj(Y_k)
-    zl[w][k] = cmk(X.x - Y.y, X.y + Y.x);
-    if (k > 0 && 2 * k != nz) zl[w][nz - k] = cmk(X.x + Y.y, Y.x - X.y);
+    T2 *L = z.p.buf + pi * z.p.ld;
+    L[pos[k]] = cmk(X.x - Y.y, X.y + Y.x);
+    if (k > 0 && 2 * k != nz) L[pos[nz - k]] = cmk(X.x + Y.y, Y.x - X.y);
   }
-  __syncwarp();
-  WarpTw<R, T2> tw;
-  if constexpr (sizeof(T) == 4) tw = warp_twiddles<R, T2>(pm.twiddlef + pl.tw0[2]);
-  else tw = warp_twiddles<R, T2>(pm.twiddle + pl.tw0[2]);
-  const int b = brev5(lane);
-  T2 v[R];
-#pragma unroll
-  for (int k = 0; k < R; k++) v[k] = zl[w][k + R * b];
-  warp_fft_inv<R>(v, tw);
-  T *Rg = reinterpret_cast<T *>(pm.rgrid) + pl.grid0 + ((long long)x * ny + y0 + 2 * w) * nz;
-#pragma unroll
-  for (int r = 0; r < R; r++) {
-    Rg[r * 32 + lane] = v[r].x;
-    if (two) Rg[nz + r * 32 + lane] = v[r].y;
+  __syncthreads();
+  int m = 1;
+  for (int q = pl.npr[2] - 1; q >= 0; q--) {
+    m *= z.rad[q];
+#define Z_INV(R) row_stage<R, +1, false>(z.p, m)
+    PLANE_RADIX(z.rad[q], Z_INV)
+#undef Z_INV
+    __syncthreads();
+  }
+  T *R = reinterpret_cast<T *>(pm.rgrid) + pl.grid0 + ((long long)x * ny + y0) * nz;
+  for (int e = threadIdx.x; e < npair * nz; e += ZT) {
+    const int pi = divf(e, rnz), k = e - pi * nz;
+    const T2 v = z.p.buf[pi * z.p.ld + k];
+    R[e + pi * nz] = v.x;
+    if (2 * pi + 1 < cnt) R[e + (pi + 1) * nz] = v.y;
   }
 }
 
@@ -1129,17 +1140,15 @@ int recip_t(const SystemDev &s, const NbListDev &nb, const PmeDev &pm, cudaStrea
     default: k_spread<MIXED, 8><<<slots(SLOT_THREADS<8>), TB, 0, st>>>(nb, pm);
   }
   if (mark) mark(mctx, "pme_spread");
-  // shared memory sized to the largest work item of the plan (caps ZMAXE / LMAXE)
-  const size_t zsmem = sizeof(T2) * (256 + 2 * (size_t)pm.zbuf);
+  // shared memory sized to the largest work item of the plan
   static bool zconf[PMB_MAX_DEVICES] = {}, lconf[PMB_MAX_DEVICES] = {};  // per device
   const int dev = device_slot();
   if (!zconf[dev]) {
-    const int zcap = (int)(sizeof(T2) * (256 + 2 * (size_t)ZMAXE));
-    cudaFuncSetAttribute(k_fft_z_fwd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, zcap);
-    cudaFuncSetAttribute(k_fft_z_inv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, zcap);
+    cudaFuncSetAttribute(k_fft_z_fwd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, Z_SMEM_MAX);
+    cudaFuncSetAttribute(k_fft_z_inv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, Z_SMEM_MAX);
     zconf[dev] = true;
   }
-  k_fft_z_fwd<T><<<pm.nzwork, ZT, zsmem, st>>>(pm);
+  k_fft_z_fwd<T><<<pm.nzwork, ZT, pm.zsmem, st>>>(pm);
   if (head) cudaEventRecord(head, st);
   const size_t lsmem = 32 * sizeof(double) + sizeof(T2) * (256 + 2 * (size_t)pm.lbuf);
   if (!lconf[dev]) {
@@ -1178,14 +1187,7 @@ int recip_t(const SystemDev &s, const NbListDev &nb, const PmeDev &pm, cudaStrea
     }
     fft_y(+1);
   }
-  switch (pm.wz) {
-    case 1: k_fft_z_inv_warp<T, 1><<<pm.nzwork, WZ, 0, st>>>(pm); break;
-    case 2: k_fft_z_inv_warp<T, 2><<<pm.nzwork, WZ, 0, st>>>(pm); break;
-    case 3: k_fft_z_inv_warp<T, 3><<<pm.nzwork, WZ, 0, st>>>(pm); break;
-    case 4: k_fft_z_inv_warp<T, 4><<<pm.nzwork, WZ, 0, st>>>(pm); break;
-    case 5: k_fft_z_inv_warp<T, 5><<<pm.nzwork, WZ, 0, st>>>(pm); break;
-    default: k_fft_z_inv<T><<<pm.nzwork, ZT, zsmem, st>>>(pm);
-  }
+  k_fft_z_inv<T><<<pm.nzwork, ZT, pm.zsmem, st>>>(pm);
   if (mark) mark(mctx, "pme_fft");
   switch (pm.order) {
     case 2: k_gather<MIXED, 2><<<slots(SLOT_THREADS<2>), TB, 0, st>>>(s, nb, pm); break;
@@ -1225,6 +1227,11 @@ bool pme_plane_radices(int n, std::vector<int> &rad) {
   search(n, 0, 0);
   rad = best;
   return !best.empty();
+}
+
+size_t pme_z_smem(int nz, int lines, int precision) {
+  const size_t c = precision ? sizeof(float2) : sizeof(double2);
+  return c * (nz + (nz & 1)) + sizeof(int) * ((nz + 3) / 4 * 4) + c * (size_t)((lines + 1) / 2) * z_line_stride(nz, (lines + 1) / 2, precision);
 }
 
 size_t pme_plane_smem(int nx, int ny, int precision) {
