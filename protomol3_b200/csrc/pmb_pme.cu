@@ -875,7 +875,8 @@ __device__ __forceinline__ void col_infl(const PlaneCtx<T2> &p, const T *th, dou
 // and y.  Two or three register stages a direction (96 = 6 x 4 x 4), so about ten barriers; the
 // three kernels before it had four or five each way and moved the spectrum through memory six
 // times.  Few CTAs (49 at 96^3) of long latency, which suits running beside the pair kernel: alone
-// 20 -> 13 us at 72^3, 36 -> 31 us at 125^3, 12 -> 8 us at 20^3, and two launches fewer.
+// 20 -> 13 us at 72^3, 36 -> 31 us at 125^3, 12 -> 8 us at 20^3 (22 -> 25 us at 96^3, where one line per
+// warp replaced these stages, but those kernels waited for room on every SM), and two launches fewer.
 template <typename T, bool VIR>
 __global__ void __launch_bounds__(PLANE_MAX_THREADS) k_fft_plane(const SystemDev s, PmeDev pm) {
   using T2 = typename C2<T>::t;
