@@ -112,10 +112,11 @@ __device__ __forceinline__ void sort_bin(const SystemDev &s, const NbListDev &nb
     nb.rank[i] = atomicAdd(nb.bin_count + b.key0 + kk, 1);  // (the bins are zero between builds)
   }
 }
-// by one CTA
+// By one CTA.  Each count is cleared as it is read, so the bins are zero for the next build whichever
+// kernels follow this one.
 __device__ __forceinline__ void sort_scan(const NbListDev &nb, const BoxDev &b) {
   const int nk = b.nc[0] * b.nc[0] * b.nc[0], T = blockDim.x;
-  const int *count = nb.bin_count + b.key0;
+  int *count = nb.bin_count + b.key0;
   int *start = nb.bin_start + b.key0;
   __shared__ int carry;
   if (threadIdx.x == 0) carry = 0;
@@ -128,7 +129,10 @@ __device__ __forceinline__ void sort_scan(const NbListDev &nb, const BoxDev &b) 
 #pragma unroll
     for (int q = 0; q < PER / 4; q++) {  // nk is 1 or a multiple of 8; regions start at multiples of 4
       v[q] = make_int4(0, 0, 0, 0);
-      if (k + 4 * q < nk) v[q] = __ldcg(reinterpret_cast<const int4 *>(count + k + 4 * q));
+      if (k + 4 * q < nk) {
+        v[q] = __ldcg(reinterpret_cast<const int4 *>(count + k + 4 * q));
+        *reinterpret_cast<int4 *>(count + k + 4 * q) = make_int4(0, 0, 0, 0);
+      }
       sum += v[q].x + v[q].y + v[q].z + v[q].w;
     }
     int tot;
@@ -154,8 +158,9 @@ __device__ __forceinline__ void sort_scatter(const NbListDev &nb, const BoxDev &
   }
 }
 __device__ __forceinline__ void sort_place(const SystemDev &s, const NbListDev &nb, const BoxDev &b, int bi, int t, int T) {
-  const int *count = nb.bin_count + b.key0, *start = nb.bin_start + b.key0;
+  const int *start = nb.bin_start + b.key0;
   const int *raw = nb.slot_raw + b.blk0 * BLOCK;
+  const int nk = b.nc[0] * b.nc[0] * b.nc[0];
   for (int p = t; p < b.nblk * BLOCK; p += T) {
     if (p >= b.natoms) {  // padding of the last block
       const int sl = b.blk0 * BLOCK + p;
@@ -169,7 +174,7 @@ __device__ __forceinline__ void sort_place(const SystemDev &s, const NbListDev &
     const int k = __ldcg(nb.key + i);
     const double x = s.pos[3 * i], y = s.pos[3 * i + 1], z = s.pos[3 * i + 2], q = s.charge[i];
     const int mol = s.molecule[i], type = s.type[i];
-    const int s0 = __ldcg(start + k), s1 = s0 + __ldcg(count + k);
+    const int s0 = __ldcg(start + k), s1 = k + 1 < nk ? __ldcg(start + k + 1) : b.natoms;
     int below = 0;
     for (int r = s0; r < s1; r++) below += __ldcg(raw + r) < i;
     const int sl = b.blk0 * BLOCK + s0 + below;
@@ -184,11 +189,8 @@ __device__ __forceinline__ void sort_place(const SystemDev &s, const NbListDev &
     nb.xref[3 * i + 2] = z;
   }
 }
-// extents in fractional fixed point, a warp per superblock and GROUPS blocks at a time; also
-// clears the bins for the next build
+// extents in fractional fixed point, a warp per superblock and GROUPS blocks at a time
 __device__ __forceinline__ void sort_extents(const NbListDev &nb, const BoxDev &b, int t, int T) {
-  const int nk = b.nc[0] * b.nc[0] * b.nc[0];
-  for (int k = t; k < nk; k += T) nb.bin_count[b.key0 + k] = 0;
   const int lane = threadIdx.x & 31, li = lane & (BLOCK - 1), g = lane / BLOCK;
   for (int S = t >> 5; S * 32 < b.nblk; S += T / 32) {
     unsigned slo[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, shi[3] = {0u, 0u, 0u};

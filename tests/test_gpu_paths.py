@@ -133,3 +133,28 @@ def test_forces_outlive_the_list(kind):
         md.run(5)
         out.append(np.concatenate(md.state()))
     assert rel(out[1], out[0]) < 1e-10
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("extra", ["", "bonded"])
+def test_slots_rebuilt_without_pair_lists(precision, extra):
+    """Sets without a pair term sort their atoms but build no lists.  1,100 waters take the launch per
+    phase: two unrelated configurations, then a pair set and the first set again on the same system,
+    so every build starts from the bins that a build of either kind left."""
+    b, other = shaken(1100, 61), shaken(1100, 62)
+    grid = (20, 24, 18)
+    topo = F.Topology(b, precision)
+    slow = [F.NonbondedPMEwaldSystemForce(grid, 7.0, real=False, correction=False)]
+    if extra:
+        slow.append(F.BondedSystemForce())
+    fast = [F.NonbondedCutoffSystemForce(lj=("C2", 6.0, 7.0), coulomb=("C1", 0.0, 7.0))]
+    pme = O.pme_params(grid, 7.0, real=0, recip=1, corr=0)
+    cut = O.cutoff_params(lj=("C2", 6.0, 7.0), coul=("C1", 0.0, 7.0))
+    for pos, fl in [(b["pos"], slow), (other["pos"], slow), (b["pos"], fast), (other["pos"], slow), (b["pos"], slow),
+                    (other["pos"], fast)]:
+        pos = np.ascontiguousarray(pos)
+        f = np.zeros((topo.n_atoms, 3))
+        F.evaluate_all(topo, fl, pos, f, F.ScalarStructure(1))
+        kw = dict(cutoff=cut) if fl is fast else dict(pme=pme, bonded=bool(extra))
+        fo, _, _, _ = O.evaluate(O.System(b), pos, **kw)
+        assert rel(f, fo) < TOL[precision]
