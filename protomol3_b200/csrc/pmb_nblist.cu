@@ -347,8 +347,8 @@ __device__ __forceinline__ int build_block(const SystemDev &s, NbListDev &nb, do
   // radius of one of them, the exact Verlet condition per pair (the bounding-box gap alone would
   // list about a third more atoms).  In shared memory, FP32 relative to the block's first atom, as
   // -2 q and |q|^2 of pairs of atoms {t, t + BLOCK/2}: x x' y y' | z z' n n', so that a pair of
-  // atoms takes three two-wide products, |p - q|^2 <= r^2 as |q|^2 - 2 p.q <= r^2 - |p|^2 (rounding
-  // 1e-4 A^2 against the list radius' margin of 0.02 A^2); padding atoms have |q|^2 = 1e12.
+  // atoms takes three two-wide products, |p - q|^2 <= r^2 as |q|^2 - 2 p.q <= r^2 - |p|^2 (rounding:
+  // see `diff` below); padding atoms have |q|^2 = 1e12.
   int imol[BLOCK];
   unsigned r0[3];
   {
@@ -383,13 +383,20 @@ __device__ __forceinline__ int build_block(const SystemDev &s, NbListDev &nb, do
   const float rlf = sqrtf(rl2);
   const bool rewrap = rlf + 2.f * hI[0] >= 0.5f * (float)b.L[0] || rlf + 2.f * hI[1] >= 0.5f * (float)b.L[1] ||
                       rlf + 2.f * hI[2] >= 0.5f * (float)b.L[2];
+  // The expanded test cancels |p|^2 and |q|^2.  With |q| <= X, the block's extent, and |p| <= P = X + r
+  // its ten roundings, u = 2^-24 each, add up to at most u (3 X^2 + 3 (X^2 + 2 X P) + 4 P^2) <= 16 u P^2
+  // = 9.5e-7 P^2 A^2.  The list radius r exceeds what is needed by 1e-3 A, 2e-3 r A^2: half of that is
+  // left to the coordinates' own rounding.  A block spread wider (P > 104 A at r = 10.8; blocks of a
+  // liquid have P < 20) takes the differences themselves, as the re-wrapped test does.
+  const float P = rlf + 2.f * sqrtf(fmaf(hI[2], hI[2], fmaf(hI[1], hI[1], hI[0] * hI[0])));
+  const bool diff = rewrap || 1e-6f * P * P > 1e-3f * rlf;
   const float Lf[3] = {(float)b.L[0], (float)b.L[1], (float)b.L[2]},
               Lrf[3] = {(float)b.Lr[0], (float)b.Lr[1], (float)b.Lr[2]};
   auto near_any = [&](uint4 f) {
     const float px = (float)(int)(f.x - r0[0]) * sL[0], py = (float)(int)(f.y - r0[1]) * sL[1],
                 pz = (float)(int)(f.z - r0[2]) * sL[2];
     bool near = false;
-    if (rewrap) {
+    if (diff) {
 #pragma unroll
       for (int t = 0; t < BLOCK / 2; t++) {
         const float4 a = ipos[2 * t], c = ipos[2 * t + 1];

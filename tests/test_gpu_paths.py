@@ -158,3 +158,27 @@ def test_slots_rebuilt_without_pair_lists(precision, extra):
         kw = dict(cutoff=cut) if fl is fast else dict(pme=pme, bonded=bool(extra))
         fo, _, _, _ = O.evaluate(O.System(b), pos, **kw)
         assert rel(f, fo) < TOL[precision]
+
+
+@pytest.mark.parametrize("rc", [5.0, 10.0])
+@pytest.mark.parametrize("edge", [200.0, 2000.0, 4000.0])
+def test_list_of_a_dilute_box(edge, rc):
+    """Chains of three charges in a wide box, neighbours 1e-6 to 1e-4 A inside the cutoff, and no skin:
+    blocks of eight atoms spread over up to half the box (the list's test in FP32 has 1e-3 A to
+    spare).  A charge pair that the list leaves out changes two forces by 332 / rc^2."""
+    rng = np.random.default_rng(17)
+    n = 300
+    step = rng.normal(size=(n, 2, 3))
+    step *= ((rc - 10.0 ** rng.uniform(-6, -4, (n, 2))) / np.linalg.norm(step, axis=2))[:, :, None]
+    first = rng.uniform(0.0, edge, (n, 3))
+    pos = np.stack([first, first + step[:, 0], first + step.sum(1)], 1).reshape(-1, 3)
+    b = W.water_box(n, seed=1, edge=edge)
+    none = np.zeros((0, 2), np.int32)
+    b.update(pos=pos, charge=np.tile([18.2, -18.2, 18.2], n), molecule=np.arange(3 * n, dtype=np.int32),
+             excl_pairs=none, excl_kind=np.zeros(0, np.int32))
+    topo = F.Topology(b, "fp64")
+    topo.set_tuning(skin=0.0, sort_cell=50.0)
+    f = np.zeros_like(pos)
+    F.evaluate_all(topo, [F.NonbondedCutoffSystemForce(coulomb=("cutoff", 0.0, rc))], pos, f, F.ScalarStructure(1))
+    fo, _, _, _ = O.evaluate(O.System(b), pos, cutoff=O.cutoff_params(coul=("cutoff", 0.0, rc)))
+    assert rel(f, fo) < TOL["fp64"]
