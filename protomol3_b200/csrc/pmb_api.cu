@@ -2488,6 +2488,7 @@ int pmb_md_energies(pmb_md *m, double *energies, double *kinetic) {
   int max_box_atoms = 0;
   for (const BoxDev &b : s->hbox) max_box_atoms = std::max(max_box_atoms, b.natoms);
   kinetic_energy(sd, m->in, m->d_kin, m->d_kin_parts, m->d_kin_done, max_box_atoms, s->stream);
+  CK(cudaGetLastError());
   CK(cudaMemcpyAsync(m->h_e.data(), s->d_eout, sizeof(double) * m->h_e.size(), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaMemcpyAsync(m->h_k.data(), m->d_kin, sizeof(double) * m->h_k.size(), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));

@@ -298,9 +298,9 @@ __global__ void k_step_inc(long long *step) { *step += 1; }
 // fixed order, then the last of them adds the parts in order (one block took 126 us at 98,304 atoms).
 constexpr int KIN_ATOMS = 2048;  // atoms of a part, more in boxes over KIN_PARTS times that
 __global__ void __launch_bounds__(256) k_kinetic(const SystemDev s, IntegratorDev in, double *out, double *parts, unsigned *done) {
-  const int b = blockIdx.y, n = s.box[b].natoms;
+  const int b = blockIdx.x, n = s.box[b].natoms;  // (boxes on x: more than 65,535 are accepted)
   const int per = max(KIN_ATOMS, (n + KIN_PARTS - 1) / KIN_PARTS), np = (n + per - 1) / per;
-  const int part = blockIdx.x;
+  const int part = blockIdx.y;
   if (part >= np) return;
   const int i0 = s.box[b].atom0, end = i0 + min(n, (part + 1) * per);
   double acc = 0.0;
@@ -863,7 +863,7 @@ int integrate_half_kick(const SystemDev &s, const IntegratorDev &in, cudaStream_
 int kinetic_energy(const SystemDev &s, const IntegratorDev &in, double *out, double *parts, unsigned *done,
                    int max_box_atoms, cudaStream_t st) {
   const int np = std::max(1, std::min(KIN_PARTS, (max_box_atoms + KIN_ATOMS - 1) / KIN_ATOMS));
-  k_kinetic<<<dim3(np, s.nbox), 256, 0, st>>>(s, in, out, parts, done);
+  k_kinetic<<<dim3(s.nbox, np), 256, 0, st>>>(s, in, out, parts, done);
   return 0;
 }
 

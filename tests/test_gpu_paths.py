@@ -182,3 +182,16 @@ def test_list_of_a_dilute_box(edge, rc):
     F.evaluate_all(topo, [F.NonbondedCutoffSystemForce(coulomb=("cutoff", 0.0, rc))], pos, f, F.ScalarStructure(1))
     fo, _, _, _ = O.evaluate(O.System(b), pos, cutoff=O.cutoff_params(coul=("cutoff", 0.0, rc)))
     assert rel(f, fo) < TOL["fp64"]
+
+
+def test_kinetic_energy_of_many_boxes():
+    """More boxes than a grid's second dimension holds (65,535)."""
+    n = 65600
+    one = dict(box=np.full(3, 10.0), charge=[0.0], type=[0], molecule=[0], lj=np.zeros(4), mass=[2.0])
+    topo = F.Topology([one] * n, "mixed")
+    md = F.Integrator(topo, [F.BondedSystemForce()])
+    vel = np.zeros((n, 3))
+    vel[:, 0] = np.arange(n)
+    md.set_state(np.ones((n, 3)), vel)
+    _, kin = md.energies()
+    np.testing.assert_array_equal(kin, vel[:, 0] ** 2)
