@@ -504,6 +504,16 @@ int nblist_alloc(pmb_system *s, double rl) {
   nb.rank = s->nba.get<int>(s->natoms);
   nb.bin_count = s->nba.get<int>(nb.nkeys);
   nb.bin_start = s->nba.get<int>(nb.nkeys);
+  std::vector<int2> scan;
+  for (int bi = 0; bi < s->nbox; bi++) {
+    const int nc = s->hbox[bi].nc[0], nk = nc * nc * nc;
+    for (int c = 0; nk > SCAN_ONE_CTA && c * SCAN_CHUNK < nk; c++) scan.push_back(make_int2(bi, c));
+  }
+  int2 *d_scan;
+  if (upload(s->nba, d_scan, scan)) return PMB_ERR_CUDA;
+  nb.scan_work = d_scan;
+  nb.nscan = (int)scan.size();
+  nb.bin_sums = s->nba.get<int>(scan.size(), false);
   nb.slot_raw = s->nba.get<int>(nb.nslot);
   nb.slot_of = s->nba.get<int>(s->natoms, false);
   if (nb.slot_of) cudaMemset(nb.slot_of, 0xff, sizeof(int) * s->natoms);  // -1: no slot yet
@@ -528,7 +538,7 @@ int nblist_alloc(pmb_system *s, double rl) {
   CK(cudaMemcpy(nb.ctl, ctl0, sizeof(ctl0), cudaMemcpyHostToDevice));
   s->nb_build_rl = -1.0;
   if (!nb.blk_lo || !nb.blk_hi || !nb.blk_c || !nb.blk_h || !nb.sblk_c || !nb.sblk_h || !nb.jlist || !nb.units ||
-      !nb.slot_meta || !nb.fslot || !nb.key || !nb.rank || !nb.bin_count || !nb.bin_start)
+      !nb.slot_meta || !nb.fslot || !nb.key || !nb.rank || !nb.bin_count || !nb.bin_start || !nb.bin_sums)
     return fail(PMB_ERR_CUDA, "cudaMalloc failed for the neighbour list");
   s->nb_cutoff = rl;
   s->nb_ready = true;

@@ -47,6 +47,9 @@ enum {
   CTL_UNITS = 12,   // pair units of boxes without and with lattice images
   CTL_WORDS = 16
 };
+// Sort bins: one CTA scans a box's up to here, in chunks of SCAN_CHUNK; more are scanned chunk by chunk
+// over the whole chip.
+constexpr int SCAN_CHUNK = 8192, SCAN_ONE_CTA = 4 * SCAN_CHUNK;
 struct NbListDev {
   // per block
   int nblk_total;
@@ -81,6 +84,9 @@ struct NbListDev {
   int *rank;                   // [natoms]
   int *bin_count;              // [nkeys] zero between builds
   int *bin_start;              // [nkeys] relative to the box's first slot
+  const int2 *scan_work;       // [nscan] bins of boxes of more than SCAN_ONE_CTA: box, chunk of SCAN_CHUNK
+  int nscan;
+  int *bin_sums;               // [nscan] atoms in each of those chunks
   int *slot_raw;               // [nslot] atoms by bin, before they are ordered within the bins
   int *slot_of;                // [natoms] slot of each atom (-1 before the first build)
   int max_box_atoms, n_sm;     // largest box; SMs of the device

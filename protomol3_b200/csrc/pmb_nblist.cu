@@ -112,38 +112,53 @@ __device__ __forceinline__ void sort_bin(const SystemDev &s, const NbListDev &nb
     nb.rank[i] = atomicAdd(nb.bin_count + b.key0 + kk, 1);  // (the bins are zero between builds)
   }
 }
-// By one CTA.  Each count is cleared as it is read, so the bins are zero for the next build whichever
-// kernels follow this one.
+constexpr int SCAN_PER = 16;  // bins of a thread per round of the scan
+// The bins k .. k + SCAN_PER of a thread: counts in v, their sum returned.  (nk is 1 or a multiple of 8; the
+// boxes' regions start at multiples of 4.)
+__device__ __forceinline__ int scan_load(const int *count, int k, int nk, int4 v[SCAN_PER / 4]) {
+  int sum = 0;
+#pragma unroll
+  for (int q = 0; q < SCAN_PER / 4; q++) {
+    v[q] = make_int4(0, 0, 0, 0);
+    if (k + 4 * q < nk) v[q] = __ldcg(reinterpret_cast<const int4 *>(count + k + 4 * q));
+    sum += v[q].x + v[q].y + v[q].z + v[q].w;
+  }
+  return sum;
+}
+// Their starts, ex the first.
+__device__ __forceinline__ void scan_store(int *start, int k, int nk, int ex, const int4 v[SCAN_PER / 4]) {
+#pragma unroll
+  for (int q = 0; q < SCAN_PER / 4; q++) {
+    if (k + 4 * q < nk)
+      *reinterpret_cast<int4 *>(start + k + 4 * q) =
+          make_int4(ex, ex + v[q].x, ex + v[q].x + v[q].y, ex + v[q].x + v[q].y + v[q].z);
+    ex += v[q].x + v[q].y + v[q].z + v[q].w;
+  }
+}
+// The counts of a CTA's round, k0 the first, cleared once all its threads have read theirs: the bins are
+// zero for the next build whichever kernels follow the scan.
+__device__ __forceinline__ void scan_clear(int *count, int k0, int nk) {
+#pragma unroll
+  for (int q = 0; q < SCAN_PER / 4; q++) {
+    const int k = k0 + 4 * (q * blockDim.x + threadIdx.x);
+    if (k < nk) *reinterpret_cast<int4 *>(count + k) = make_int4(0, 0, 0, 0);
+  }
+}
+// by one CTA
 __device__ __forceinline__ void sort_scan(const NbListDev &nb, const BoxDev &b) {
   const int nk = b.nc[0] * b.nc[0] * b.nc[0], T = blockDim.x;
-  int *count = nb.bin_count + b.key0;
-  int *start = nb.bin_start + b.key0;
+  int *count = nb.bin_count + b.key0, *start = nb.bin_start + b.key0;
   __shared__ int carry;
   if (threadIdx.x == 0) carry = 0;
   __syncthreads();
-  constexpr int PER = 16;  // bins of a thread per round
-  for (int k0 = 0; k0 < nk; k0 += PER * T) {
-    const int k = k0 + PER * threadIdx.x;
-    int4 v[PER / 4];
-    int sum = 0;
-#pragma unroll
-    for (int q = 0; q < PER / 4; q++) {  // nk is 1 or a multiple of 8; regions start at multiples of 4
-      v[q] = make_int4(0, 0, 0, 0);
-      if (k + 4 * q < nk) {
-        v[q] = __ldcg(reinterpret_cast<const int4 *>(count + k + 4 * q));
-        *reinterpret_cast<int4 *>(count + k + 4 * q) = make_int4(0, 0, 0, 0);
-      }
-      sum += v[q].x + v[q].y + v[q].z + v[q].w;
-    }
+  for (int k0 = 0; k0 < nk; k0 += SCAN_PER * T) {
+    const int k = k0 + SCAN_PER * threadIdx.x;
+    int4 v[SCAN_PER / 4];
+    const int sum = scan_load(count, k, nk, v);
     int tot;
-    int ex = carry + block_exclusive_scan(sum, &tot);
-#pragma unroll
-    for (int q = 0; q < PER / 4; q++) {
-      if (k + 4 * q < nk)
-        *reinterpret_cast<int4 *>(start + k + 4 * q) =
-            make_int4(ex, ex + v[q].x, ex + v[q].x + v[q].y, ex + v[q].x + v[q].y + v[q].z);
-      ex += v[q].x + v[q].y + v[q].z + v[q].w;
-    }
+    const int ex = carry + block_exclusive_scan(sum, &tot);
+    scan_store(start, k, nk, ex, v);
+    scan_clear(count, k0, nk);  // (the block scan holds barriers)
     __syncthreads();
     if (threadIdx.x == 0) carry += tot;
     __syncthreads();
@@ -267,7 +282,7 @@ __global__ void __launch_bounds__(SORT_BOX_THREADS) k_sort_box(SystemDev s, NbLi
 }
 
 // One launch per phase over the whole chip (blockIdx.y: box): large boxes.  The last CTA of a box
-// to finish its histogram also scans the box's bins.
+// to finish its histogram also scans the box's bins, if they are few.
 __global__ void __launch_bounds__(SORT_THREADS) k_sort_bin(SystemDev s, NbListDev nb) {
   if (!nb.ctl[CTL_REBUILD] || !nb.box_rb[blockIdx.y]) return;
   const BoxDev &b = s.box[blockIdx.y];
@@ -280,7 +295,43 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_bin(SystemDev s, NbListDe
   if (!last) return;
   __threadfence();
   if (threadIdx.x == 0) nb.box_done[blockIdx.y] = 0u;
-  sort_scan(nb, b);
+  if (b.nc[0] * b.nc[0] * b.nc[0] <= SCAN_ONE_CTA) sort_scan(nb, b);
+}
+// The bins of a wide box, SCAN_CHUNK to a CTA and turn: the chunks' sums, then each chunk from the sum
+// of those before it.  (The number of bins follows the longest edge, not the atoms: 32,768 up to 154 A,
+// 2.1 million at 307 to 614 A.)  An evaluation that rebuilds, by one CTA's scan and by these: 217,000 atoms
+// in 60 x 60 x 600 A 1224 and 619 us, 30,000 atoms within 1000 A 5027 and 208 us, 216 atoms within 700 A
+// 5240 and 132 us; the 97,000 atoms of a 99 A cube (32,768 bins, scanned by one CTA) take 271 us.
+static_assert(SCAN_CHUNK == SORT_THREADS * SCAN_PER, "a thread scans SCAN_PER bins of a chunk");
+__global__ void __launch_bounds__(SORT_THREADS) k_scan_sums(SystemDev s, NbListDev nb) {
+  if (!nb.ctl[CTL_REBUILD]) return;
+  for (int w = blockIdx.x; w < nb.nscan; w += gridDim.x) {
+    const int2 it = nb.scan_work[w];  // box, chunk
+    if (!nb.box_rb[it.x]) continue;
+    const BoxDev &b = s.box[it.x];
+    const int nk = b.nc[0] * b.nc[0] * b.nc[0], k = it.y * SCAN_CHUNK + SCAN_PER * threadIdx.x;
+    int4 v[SCAN_PER / 4];
+    int tot;
+    block_exclusive_scan(scan_load(nb.bin_count + b.key0, k, nk, v), &tot);
+    if (threadIdx.x == 0) nb.bin_sums[w] = tot;
+  }
+}
+__global__ void __launch_bounds__(SORT_THREADS) k_scan_apply(SystemDev s, NbListDev nb) {
+  if (!nb.ctl[CTL_REBUILD]) return;
+  for (int w = blockIdx.x; w < nb.nscan; w += gridDim.x) {
+    const int2 it = nb.scan_work[w];
+    if (!nb.box_rb[it.x]) continue;
+    const BoxDev &b = s.box[it.x];
+    const int nk = b.nc[0] * b.nc[0] * b.nc[0], k = it.y * SCAN_CHUNK + SCAN_PER * threadIdx.x;
+    int before = 0, base;
+    for (int c = w - it.y + threadIdx.x; c < w; c += SORT_THREADS) before += __ldg(nb.bin_sums + c);
+    block_exclusive_scan(before, &base);
+    int4 v[SCAN_PER / 4];
+    const int sum = scan_load(nb.bin_count + b.key0, k, nk, v);
+    const int ex = base + block_exclusive_scan(sum, nullptr);
+    scan_store(nb.bin_start + b.key0, k, nk, ex, v);
+    scan_clear(nb.bin_count + b.key0, it.y * SCAN_CHUNK, nk);
+  }
 }
 __global__ void __launch_bounds__(SORT_THREADS) k_sort_scatter(SystemDev s, NbListDev nb) {
   if (!nb.ctl[CTL_REBUILD] || !nb.box_rb[blockIdx.y]) return;
@@ -570,9 +621,11 @@ __global__ void __launch_bounds__(BL_THREADS, BL_MINB) k_build_lists(SystemDev s
 }
 constexpr int CLAIMS_PER_WARP = 4;  // at least, before a claim takes more than one block
 
-// One CTA per box up to SORT_SMALL atoms, and up to SORT_MANY when the boxes alone fill the chip.
+// One CTA per box up to SORT_SMALL atoms, and up to SORT_MANY when the boxes alone fill the chip;
+// not where a box has more bins than one CTA scans.
 constexpr int SORT_SMALL = 3072, SORT_MANY = 32768;
 bool sort_by_box(const SystemDev &s, const NbListDev &nb) {
+  if (nb.nscan > 0) return false;
   return nb.max_box_atoms <= SORT_SMALL || (s.nbox >= nb.n_sm / 2 && nb.max_box_atoms <= SORT_MANY);
 }
 
@@ -592,6 +645,11 @@ int nblist_sort(const SystemDev &s, NbListDev &nb, bool updated, cudaStream_t st
   }
   const dim3 grid((nb.max_box_atoms + SORT_THREADS - 1) / SORT_THREADS, s.nbox);
   k_sort_bin<<<grid, SORT_THREADS, 0, st>>>(s, nb);
+  if (nb.nscan > 0) {
+    const int scan_grid = std::min(nb.nscan, 4 * nb.n_sm);
+    k_scan_sums<<<scan_grid, SORT_THREADS, 0, st>>>(s, nb);
+    k_scan_apply<<<scan_grid, SORT_THREADS, 0, st>>>(s, nb);
+  }
   k_sort_scatter<<<grid, SORT_THREADS, 0, st>>>(s, nb);
   k_sort_place<<<grid, SORT_THREADS, 0, st>>>(s, nb);
   return 0;

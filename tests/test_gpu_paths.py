@@ -195,3 +195,31 @@ def test_kinetic_energy_of_many_boxes():
     md.set_state(np.ones((n, 3)), vel)
     _, kin = md.energies()
     np.testing.assert_array_equal(kin, vel[:, 0] ** 2)
+
+
+# a slab of 2.1 million sort cells, a cluster alone in such a box (fewer atoms than one CTA sorts), and
+# the latter beside an ordinary box
+@pytest.mark.parametrize("boxes", [["slab"], ["cluster"], ["cluster", "liquid"]])
+def test_sort_of_a_wide_box(boxes):
+    """Sort cells follow the longest edge: many are scanned by the whole chip, and cleared for the next
+    build.  Several unrelated configurations, each against the oracle."""
+    rng = np.random.default_rng(23)
+    rc = 8.0
+    fill = {"slab": ([40.0, 40.0, 400.0], [40.0, 40.0, 400.0], 5000), "cluster": ([400.0] * 3, [20.0] * 3, 300),
+            "liquid": ([30.0] * 3, [30.0] * 3, 2000)}
+    systems = []
+    for name in boxes:
+        edges, _, n = fill[name]
+        systems.append(dict(box=np.array(edges), charge=np.where(np.arange(n) % 2, 18.2, -18.2), type=np.zeros(n, np.int32),
+                            molecule=np.arange(n, dtype=np.int32), lj=np.zeros(4), mass=np.ones(n)))
+    topo = F.Topology(systems, "fp64")
+    force = F.NonbondedCutoffSystemForce(coulomb=("C1", 0.0, rc))
+    for _ in range(3):
+        pos = [rng.uniform(0.0, 1.0, (fill[n][2], 3)) * fill[n][1] for n in boxes]
+        f = np.zeros((topo.n_atoms, 3))
+        F.evaluate_all(topo, [force], np.concatenate(pos), f, F.ScalarStructure(len(boxes)))
+        at = 0
+        for b, p in zip(systems, pos):
+            fo, _, _, _ = O.evaluate(O.System(dict(b, pos=p)), p, cutoff=O.cutoff_params(coul=("C1", 0.0, rc)))
+            assert rel(f[at:at + len(p)], fo) < TOL["fp64"]
+            at += len(p)
