@@ -504,13 +504,16 @@ int nblist_alloc(pmb_system *s, double rl) {
   nb.rank = s->nba.get<int>(s->natoms);
   nb.bin_count = s->nba.get<int>(nb.nkeys);
   nb.bin_start = s->nba.get<int>(nb.nkeys);
-  std::vector<int2> scan;
+  std::vector<int2> parts, scan;
   for (int bi = 0; bi < s->nbox; bi++) {
+    for (int p = 0; p * SORT_PART < s->hbox[bi].nblk * BLOCK; p++) parts.push_back(make_int2(bi, p));
     const int nc = s->hbox[bi].nc[0], nk = nc * nc * nc;
     for (int c = 0; nk > SCAN_ONE_CTA && c * SCAN_CHUNK < nk; c++) scan.push_back(make_int2(bi, c));
   }
-  int2 *d_scan;
-  if (upload(s->nba, d_scan, scan)) return PMB_ERR_CUDA;
+  int2 *d_parts, *d_scan;
+  if (upload(s->nba, d_parts, parts) || upload(s->nba, d_scan, scan)) return PMB_ERR_CUDA;
+  nb.sort_work = d_parts;
+  nb.nsort = (int)parts.size();
   nb.scan_work = d_scan;
   nb.nscan = (int)scan.size();
   nb.bin_sums = s->nba.get<int>(scan.size(), false);

@@ -47,6 +47,7 @@ enum {
   CTL_UNITS = 12,   // pair units of boxes without and with lattice images
   CTL_WORDS = 16
 };
+constexpr int SORT_PART = 512;  // slots of a CTA of the sort's launches per phase
 // Sort bins: one CTA scans a box's up to here, in chunks of SCAN_CHUNK; more are scanned chunk by chunk
 // over the whole chip.
 constexpr int SCAN_CHUNK = 8192, SCAN_ONE_CTA = 4 * SCAN_CHUNK;
@@ -84,6 +85,8 @@ struct NbListDev {
   int *rank;                   // [natoms]
   int *bin_count;              // [nkeys] zero between builds
   int *bin_start;              // [nkeys] relative to the box's first slot
+  const int2 *sort_work;       // [nsort] box, part of SORT_PART slots
+  int nsort;
   const int2 *scan_work;       // [nscan] bins of boxes of more than SCAN_ONE_CTA: box, chunk of SCAN_CHUNK
   int nscan;
   int *bin_sums;               // [nscan] atoms in each of those chunks

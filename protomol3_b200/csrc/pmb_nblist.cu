@@ -281,20 +281,26 @@ __global__ void __launch_bounds__(SORT_BOX_THREADS) k_sort_box(SystemDev s, NbLi
   sort_extents(nb, b, t, SORT_BOX_THREADS);
 }
 
-// One launch per phase over the whole chip (blockIdx.y: box): large boxes.  The last CTA of a box
-// to finish its histogram also scans the box's bins, if they are few.
+// One launch per phase over the whole chip: large boxes.  A CTA takes one item of nb.sort_work,
+// SORT_PART slots of one box, so the launches follow the atoms however uneven the boxes are.  The last
+// CTA of a box to finish its histogram also scans the box's bins, if they are few.
+static_assert(SORT_THREADS == SORT_PART, "a thread takes a slot");
+constexpr int EXT_THREADS = SORT_PART / 8;  // a warp takes a superblock, 32 blocks of 8 slots
+static_assert(BLOCK == 8, "256 slots a superblock");
 __global__ void __launch_bounds__(SORT_THREADS) k_sort_bin(SystemDev s, NbListDev nb) {
-  if (!nb.ctl[CTL_REBUILD] || !nb.box_rb[blockIdx.y]) return;
-  const BoxDev &b = s.box[blockIdx.y];
-  sort_bin(s, nb, b, blockIdx.x * SORT_THREADS + threadIdx.x, gridDim.x * SORT_THREADS);
+  const int2 it = nb.sort_work[blockIdx.x];  // box, part
+  if (!nb.ctl[CTL_REBUILD] || !nb.box_rb[it.x]) return;
+  const BoxDev &b = s.box[it.x];
+  const int parts = (b.nblk * BLOCK + SORT_PART - 1) / SORT_PART;
+  sort_bin(s, nb, b, it.y * SORT_PART + threadIdx.x, parts * SORT_PART);
   __threadfence();
   __shared__ bool last;
   __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(nb.box_done + blockIdx.y, 1u) == gridDim.x - 1;
+  if (threadIdx.x == 0) last = atomicAdd(nb.box_done + it.x, 1u) == (unsigned)parts - 1u;
   __syncthreads();
   if (!last) return;
   __threadfence();
-  if (threadIdx.x == 0) nb.box_done[blockIdx.y] = 0u;
+  if (threadIdx.x == 0) nb.box_done[it.x] = 0u;
   if (b.nc[0] * b.nc[0] * b.nc[0] <= SCAN_ONE_CTA) sort_scan(nb, b);
 }
 // The bins of a wide box, SCAN_CHUNK to a CTA and turn: the chunks' sums, then each chunk from the sum
@@ -334,16 +340,22 @@ __global__ void __launch_bounds__(SORT_THREADS) k_scan_apply(SystemDev s, NbList
   }
 }
 __global__ void __launch_bounds__(SORT_THREADS) k_sort_scatter(SystemDev s, NbListDev nb) {
-  if (!nb.ctl[CTL_REBUILD] || !nb.box_rb[blockIdx.y]) return;
-  sort_scatter(nb, s.box[blockIdx.y], blockIdx.x * SORT_THREADS + threadIdx.x, gridDim.x * SORT_THREADS);
+  const int2 it = nb.sort_work[blockIdx.x];
+  if (!nb.ctl[CTL_REBUILD] || !nb.box_rb[it.x]) return;
+  const BoxDev &b = s.box[it.x];
+  sort_scatter(nb, b, it.y * SORT_PART + threadIdx.x, b.nblk * BLOCK + SORT_PART);
 }
 __global__ void __launch_bounds__(SORT_THREADS) k_sort_place(SystemDev s, NbListDev nb) {
-  if (!nb.ctl[CTL_REBUILD] || !nb.box_rb[blockIdx.y]) return;
-  sort_place(s, nb, s.box[blockIdx.y], blockIdx.y, blockIdx.x * SORT_THREADS + threadIdx.x, gridDim.x * SORT_THREADS);
+  const int2 it = nb.sort_work[blockIdx.x];
+  if (!nb.ctl[CTL_REBUILD] || !nb.box_rb[it.x]) return;
+  const BoxDev &b = s.box[it.x];
+  sort_place(s, nb, b, it.x, it.y * SORT_PART + threadIdx.x, b.nblk * BLOCK + SORT_PART);
 }
-__global__ void __launch_bounds__(SORT_THREADS) k_sort_extents(SystemDev s, NbListDev nb) {
-  if (!nb.ctl[CTL_REBUILD] || !nb.box_rb[blockIdx.y]) return;
-  sort_extents(nb, s.box[blockIdx.y], blockIdx.x * SORT_THREADS + threadIdx.x, gridDim.x * SORT_THREADS);
+__global__ void __launch_bounds__(EXT_THREADS) k_sort_extents(SystemDev s, NbListDev nb) {
+  const int2 it = nb.sort_work[blockIdx.x];
+  if (!nb.ctl[CTL_REBUILD] || !nb.box_rb[it.x]) return;
+  const BoxDev &b = s.box[it.x];
+  sort_extents(nb, b, it.y * EXT_THREADS + threadIdx.x, b.nblk + EXT_THREADS);
 }
 
 // Gap^2 (A^2) between the box (c1, h1 half extents in A) and the box (c2, h2 fixed-point half
@@ -621,12 +633,17 @@ __global__ void __launch_bounds__(BL_THREADS, BL_MINB) k_build_lists(SystemDev s
 }
 constexpr int CLAIMS_PER_WARP = 4;  // at least, before a claim takes more than one block
 
-// One CTA per box up to SORT_SMALL atoms, and up to SORT_MANY when the boxes alone fill the chip;
-// not where a box has more bins than one CTA scans.
-constexpr int SORT_SMALL = 3072, SORT_MANY = 32768;
+// One CTA per box up to SORT_SMALL atoms, and up to SORT_MANY when the boxes alone fill the chip and the
+// largest is not the one that all wait for; not where a box has more bins than one CTA scans.  An
+// evaluation that rebuilds every box, by one CTA per box and by a launch per phase: 80 boxes of 6,000
+// atoms 934 and 945 us, of 12,000 1641 and 1639, of 24,000 3365 and 3340; 80 of 600 beside one of 24,000
+// 347 and 222.
+constexpr int SORT_SMALL = 3072, SORT_MANY = 8192;
 bool sort_by_box(const SystemDev &s, const NbListDev &nb) {
   if (nb.nscan > 0) return false;
-  return nb.max_box_atoms <= SORT_SMALL || (s.nbox >= nb.n_sm / 2 && nb.max_box_atoms <= SORT_MANY);
+  if (nb.max_box_atoms <= SORT_SMALL) return true;
+  return s.nbox >= nb.n_sm / 2 && nb.max_box_atoms <= SORT_MANY &&
+         (long long)nb.max_box_atoms * s.nbox <= 3ll * s.natoms;
 }
 
 }  // namespace
@@ -643,25 +660,21 @@ int nblist_sort(const SystemDev &s, NbListDev &nb, bool updated, cudaStream_t st
     k_sort_box<<<s.nbox, SORT_BOX_THREADS, 0, st>>>(s, nb);
     return 0;
   }
-  const dim3 grid((nb.max_box_atoms + SORT_THREADS - 1) / SORT_THREADS, s.nbox);
-  k_sort_bin<<<grid, SORT_THREADS, 0, st>>>(s, nb);
+  k_sort_bin<<<nb.nsort, SORT_THREADS, 0, st>>>(s, nb);
   if (nb.nscan > 0) {
     const int scan_grid = std::min(nb.nscan, 4 * nb.n_sm);
     k_scan_sums<<<scan_grid, SORT_THREADS, 0, st>>>(s, nb);
     k_scan_apply<<<scan_grid, SORT_THREADS, 0, st>>>(s, nb);
   }
-  k_sort_scatter<<<grid, SORT_THREADS, 0, st>>>(s, nb);
-  k_sort_place<<<grid, SORT_THREADS, 0, st>>>(s, nb);
+  k_sort_scatter<<<nb.nsort, SORT_THREADS, 0, st>>>(s, nb);
+  k_sort_place<<<nb.nsort, SORT_THREADS, 0, st>>>(s, nb);
   return 0;
 }
 
 // Second half: the extents of the blocks (large boxes), the cluster j-lists and the units of the pair kernel.
 int nblist_lists(const SystemDev &s, NbListDev &nb, double list_cutoff, cudaStream_t st) {
   if (s.natoms <= 0) return 0;
-  if (!sort_by_box(s, nb)) {
-    const dim3 grid((nb.max_box_atoms + SORT_THREADS - 1) / SORT_THREADS, s.nbox);
-    k_sort_extents<<<grid, SORT_THREADS, 0, st>>>(s, nb);
-  }
+  if (!sort_by_box(s, nb)) k_sort_extents<<<nb.nsort, EXT_THREADS, 0, st>>>(s, nb);
   // as many blocks as fit at once (blocks are claimed), so that the exit without a rebuild is short
   const int warps = BL_THREADS / 32, need = (nb.nblk_total + warps - 1) / warps;
   nb.claim_blocks = std::max(1, std::min(8, nb.nblk_total / (nb.n_sm * BL_MINB * warps * CLAIMS_PER_WARP)));

@@ -223,3 +223,30 @@ def test_sort_of_a_wide_box(boxes):
             fo, _, _, _ = O.evaluate(O.System(dict(b, pos=p)), p, cutoff=O.cutoff_params(coul=("C1", 0.0, rc)))
             assert rel(f[at:at + len(p)], fo) < TOL["fp64"]
             at += len(p)
+
+
+# 80 boxes at both sides of the largest that one CTA each sorts (8,192 atoms), and small ones beside one
+# that all would wait for
+@pytest.mark.parametrize("sizes", [[8192, 8185], [8200, 8185], [24, 5000]])
+def test_sort_of_many_boxes(sizes):
+    """Each box of a system of many gets the forces it gets alone, bit for bit, at the first build and
+    at the next one."""
+    rng = np.random.default_rng(29)
+    edge = lambda n: (10.0 * n) ** (1.0 / 3.0)  # noqa: E731
+    box = lambda n: dict(box=np.full(3, max(edge(n), 15.0)), charge=np.where(np.arange(n) % 2, 18.2, -18.2),  # noqa: E731
+                         type=np.zeros(n, np.int32), molecule=np.arange(n, dtype=np.int32), lj=np.zeros(4), mass=np.ones(n))
+    boxes = [box(sizes[0])] * 40 + [box(sizes[1])] + [box(sizes[0])] * 39
+    at = np.concatenate([[0], np.cumsum([len(b["charge"]) for b in boxes])])
+    force = lambda: [F.NonbondedCutoffSystemForce(coulomb=("C1", 0.0, 6.0))]  # noqa: E731
+    topo = F.Topology(boxes, "mixed")
+    fl = force()
+    alone = {k: (F.Topology(boxes[k], "mixed"), force()) for k in (0, 40, 79)}
+    for _ in range(2):
+        pos = np.concatenate([rng.uniform(0.0, b["box"][0], (len(b["charge"]), 3)) for b in boxes])
+        f = np.zeros_like(pos)
+        F.evaluate_all(topo, fl, pos, f, F.ScalarStructure(len(boxes)))
+        for k, (t, one) in alone.items():
+            p = np.ascontiguousarray(pos[at[k]:at[k + 1]])
+            g = np.zeros_like(p)
+            F.evaluate_all(t, one, p, g, F.ScalarStructure(1))
+            np.testing.assert_array_equal(f[at[k]:at[k + 1]], g)
