@@ -159,3 +159,24 @@ def test_langevin_run_split_anywhere_gives_the_same_bits(precision):
     topo.close()
     assert np.array_equal(pa, pb) and np.array_equal(va, vb)
     assert np.array_equal(ea, eb) and np.array_equal(ka, kb)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_reciprocal_energy_of_a_box_among_many(precision):
+    """Enough boxes that the plane transform runs fewer threads than for one alone; charges thirty
+    times those of water lift the rounding of the sums (1e-16 of the energy) to where the last bit of
+    the fixed point (2^-32 kcal/mol) shows it."""
+    grid = (20, 24, 32)
+    boxes = [W.water_box(60, seed=90 + k) for k in range(64)]
+    for b in boxes:
+        b["charge"] = 30.0 * b["charge"]
+    pme = lambda n: [F.NonbondedPMEwaldSystemForce((0, 0, 0), 6.0, real=False, box_grids=[list(grid)] * n)]  # noqa: E731
+    topo = F.Topology(boxes, precision)
+    fb, eb = np.zeros((topo.n_atoms, 3)), F.ScalarStructure(len(boxes), virial=True)
+    F.evaluate_all(topo, pme(len(boxes)), np.concatenate([b["pos"] for b in boxes]), fb, eb)
+    for k in range(0, 64, 9):
+        t1 = F.Topology(boxes[k], precision)
+        f1, e1 = np.zeros((t1.n_atoms, 3)), F.ScalarStructure(1, virial=True)
+        F.evaluate_all(t1, pme(1), boxes[k]["pos"], f1, e1)
+        assert np.array_equal(fb[180 * k:180 * (k + 1)], f1), k
+        assert np.array_equal(eb.table[k], e1.table[0]), k
