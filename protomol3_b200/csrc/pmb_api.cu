@@ -1364,33 +1364,39 @@ pmb_force *pmb_force_create(pmb_system *s, const pmb_force_desc *d) {
     std::vector<double> infl;
     std::vector<int> radix;
     std::vector<int4> zwork;
-    std::vector<int4> ywork, xwork;
+    std::vector<int4> ywork[6], xwork[6];  // by R of the warp-shuffle transforms, 0: the shared-memory ones
     long long g0 = 0, c0 = 0;
     const int lcap = pme_line_capacity();
     size_t zsmem = 0;
     int lbuf = 1;
     std::vector<double> theta;
-    // the plane kernel takes every plan whose planes fit shared memory
+    // the plane kernel takes every box whose planes fit shared memory (a box's transforms, and so its
+    // bits, do not depend on the other boxes)
     std::vector<int2> pwork;
     std::vector<int> pradix, perm;
     size_t psmem = 0;
-    double plane_points = 0.0;
-    for (int bi = 0; bi < nbox; bi++) {
-      const int nx = d->box_grids ? d->box_grids[3 * bi] : d->grid[0], ny = d->box_grids ? d->box_grids[3 * bi + 1] : d->grid[1];
-      if (nx > 0 && ny > 0) psmem = std::max(psmem, pme_plane_smem(nx, ny, s->precision));
-      plane_points += (double)nx * ny / nbox;
-    }
-    const bool planes = psmem <= (size_t)PLANE_SMEM_MAX;
+    double points = 0.0, plane_points = 0.0;  // points of a plane: all boxes, those of the plane kernel
+    int plane_boxes = 0;
+    for (int bi = 0; bi < nbox; bi++)
+      points += d->box_grids ? (double)d->box_grids[3 * bi] * d->box_grids[3 * bi + 1] : (double)d->grid[0] * d->grid[1];
     // z-lines a CTA: eight where sixteen would leave fewer than four CTAs an SM (216 waters: 25
     // steps 975 us with eight, 989 with all 20 lines of a plane in one CTA; 96^3, just under the line:
     // the same either way)
-    const int zlines = plane_points * nbox < 16.0 * 4 * 148 ? 8 : 16;
+    const int zlines = points < 16.0 * 4 * 148 ? 8 : 16;
     double th0[8];
     bspline_h(P, 0.0, th0);
     for (int bi = 0; bi < nbox; bi++) {
       const BoxDev &b = s->hbox[bi];
       PmeBoxPlan pl;
       std::memset(&pl, 0, sizeof(pl));
+      const int *bg = d->box_grids ? d->box_grids + 3 * bi : d->grid;
+      const size_t smem = bg[0] > 0 && bg[1] > 0 ? pme_plane_smem(bg[0], bg[1], s->precision) : 0;
+      const bool planes = smem <= (size_t)PLANE_SMEM_MAX;
+      if (planes) {
+        psmem = std::max(psmem, smem);
+        plane_points += (double)bg[0] * bg[1];
+        plane_boxes++;
+      }
       for (int k = 0; k < 3; k++) {
         int n = d->box_grids ? d->box_grids[3 * bi + k] : d->grid[k];
         std::vector<int> rad;
@@ -1459,14 +1465,17 @@ pmb_force *pmb_force_create(pmb_system *s, const pmb_force_desc *d) {
         }
       const int rows = std::max(1, std::min(PME_YROWS, lcap / pl.n[1])),
                 cols = std::max(1, std::min(PME_XCOLS, lcap / pl.n[0]));
-      lbuf = std::max(lbuf, std::max(rows * pl.n[1], cols * pl.n[0]));
+      // (one row per warp of a 4-warp block, one column per warp of an 8-warp block)
+      auto warp_r = [](int n) { return n % 32 == 0 && n <= 160 ? n / 32 : 0; };
+      const int ry = PME_YROWS <= 4 ? warp_r(pl.n[1]) : 0, rx = PME_XCOLS * 32 <= PME_WX_THREADS ? warp_r(pl.n[0]) : 0;
+      if (!planes) lbuf = std::max(lbuf, std::max(rows * pl.n[1], cols * pl.n[0]));
       for (int kz = 0; kz <= pl.n[2] / 2; kz++) {
         if (planes) {
           pwork.push_back(make_int2(bi, kz));
           continue;
         }
-        for (int x0 = 0; x0 < pl.n[0]; x0 += rows) ywork.push_back(make_int4(bi, kz, x0, std::min(rows, pl.n[0] - x0)));
-        for (int y0 = 0; y0 < pl.n[1]; y0 += cols) xwork.push_back(make_int4(bi, kz, y0, std::min(cols, pl.n[1] - y0)));
+        for (int x0 = 0; x0 < pl.n[0]; x0 += rows) ywork[ry].push_back(make_int4(bi, kz, x0, std::min(rows, pl.n[0] - x0)));
+        for (int y0 = 0; y0 < pl.n[1]; y0 += cols) xwork[rx].push_back(make_int4(bi, kz, y0, std::min(cols, pl.n[1] - y0)));
       }
       // influence function per half-spectrum point [kz][x][y] (Grid.h:236-341): B(m)
       // exp(-pi^2 m^2/alpha^2) / (pi V m^2), 0 at m = 0
@@ -1519,8 +1528,17 @@ pmb_force *pmb_force_create(pmb_system *s, const pmb_force_desc *d) {
     }
     rc |= upload(f->a, drad, radix);
     rc |= upload(f->a, dz, zwork);
-    rc |= upload(f->a, dy, ywork);
-    rc |= upload(f->a, dx, xwork);
+    std::vector<int4> yall, xall;
+    for (int r = 0; r < 6; r++) {
+      pm.nywork[r] = (int)yall.size();
+      pm.nxwork[r] = (int)xall.size();
+      yall.insert(yall.end(), ywork[r].begin(), ywork[r].end());
+      xall.insert(xall.end(), xwork[r].begin(), xwork[r].end());
+    }
+    pm.nywork[6] = (int)yall.size();
+    pm.nxwork[6] = (int)xall.size();
+    rc |= upload(f->a, dy, yall);
+    rc |= upload(f->a, dx, xall);
     int2 *dpw;
     int *dpr, *dperm;
     rc |= upload(f->a, dpw, pwork);
@@ -1535,7 +1553,7 @@ pmb_force *pmb_force_create(pmb_system *s, const pmb_force_desc *d) {
     // latency counts, of radix 8 where they fill the chip (256 boxes: 218 -> 138 us), up to
     // PLANE_MAX_THREADS
     const int stage = pwork.size() >= 1024 ? 8 : 4;
-    pm.pthreads = std::max(64, std::min(PLANE_MAX_THREADS, ((int)(plane_points / stage) + 63) / 64 * 64));
+    pm.pthreads = std::max(64, std::min(PLANE_MAX_THREADS, ((int)(plane_points / std::max(1, plane_boxes) / stage) + 63) / 64 * 64));
     pm.plan = dplan;
     pm.twiddle = dtw;
     pm.twiddlef = dtwf;
@@ -1544,25 +1562,10 @@ pmb_force *pmb_force_create(pmb_system *s, const pmb_force_desc *d) {
     pm.zwork = dz;
     pm.nzwork = (int)zwork.size();
     pm.ywork = dy;
-    pm.nywork = (int)ywork.size();
     pm.xwork = dx;
-    pm.nxwork = (int)xwork.size();
     pm.zsmem = zsmem;
     pm.zpairs = zlines / 2;
     pm.lbuf = lbuf;
-    // the warp-shuffle transforms take lines of 32 R points (R <= 5), the same R in every box
-    auto warp_r = [&](int d) {
-      int r = 0;
-      for (size_t bi = 0; bi < f->plans.size(); bi++) {
-        const int n = f->plans[bi].n[d];
-        if (n % 32 != 0 || n / 32 > 5 || (r && n / 32 != r)) return 0;
-        r = n / 32;
-      }
-      return r;
-    };
-    // (one row per warp of a 4-warp block, one column per warp of an 8-warp block)
-    pm.wy = PME_YROWS <= 4 ? warp_r(1) : 0;
-    pm.wx = PME_XCOLS * 32 <= PME_WX_THREADS ? warp_r(0) : 0;
     pm.qgrid = f->a.get<long long>(g0);
     pm.rgrid = s->precision ? (void *)f->a.get<float>(g0) : (void *)f->a.get<double>(g0);
     pm.cgrid = s->precision ? (void *)f->a.get<float2>(c0) : (void *)f->a.get<double2>(c0);

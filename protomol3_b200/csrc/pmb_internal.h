@@ -184,11 +184,13 @@ struct PmeDev {
   const int *radix;           // radices per dim
   const int4 *zwork;          // z-pass work items: box, x, y0, count
   int nzwork;
-  const int4 *ywork;          // y-line work items: box, kz, x0, rows
-  int nywork;
-  const int4 *xwork;          // x-line work items: box, kz, y0, columns
-  int nxwork;
-  const int2 *pwork;          // planes of the plane kernel: box, kz (npwork 0: it is not used)
+  // planes too large for the plane kernel: line work items, those of lines of 32 R points (R <= 5, the
+  // warp-shuffle transforms) from item [R] up to [R + 1], those of the shared-memory ones from [0]
+  const int4 *ywork;          // box, kz, x0, rows
+  int nywork[7];
+  const int4 *xwork;          // box, kz, y0, columns
+  int nxwork[7];
+  const int2 *pwork;          // planes of the plane kernel: box, kz
   int npwork, pthreads;
   size_t psmem;
   const int *pradix;          // its radices
@@ -197,8 +199,6 @@ struct PmeDev {
   int zpairs;                 // packed lines of a full work item of the z kernels
   size_t zsmem;               // shared memory of the z kernels
   int lbuf;                   // complex elements per ping-pong buffer of the line kernels
-  int wy, wx;                 // R > 0: every box's y (x) lines have 32 R points and the y passes (the
-                              // x pass) run the warp-shuffle transforms; 0: the shared-memory ones
   double alpha, a2pi;
   int virial;
 };

@@ -1193,28 +1193,40 @@ int recip_t(const SystemDev &s, const NbListDev &nb, const PmeDev &pm, cudaStrea
       pconf[pm.virial != 0][dev] = true;
     }
     kern<<<pm.npwork, pm.pthreads, pm.psmem, st>>>(s, pm);
-  } else {
-    auto fft_y = [&](int sign) {
-      switch (pm.wy) {
-        case 1: k_fft_y_warp<T, 1><<<pm.nywork, WT, 0, st>>>(pm, sign); break;
-        case 2: k_fft_y_warp<T, 2><<<pm.nywork, WT, 0, st>>>(pm, sign); break;
-        case 3: k_fft_y_warp<T, 3><<<pm.nywork, WT, 0, st>>>(pm, sign); break;
-        case 4: k_fft_y_warp<T, 4><<<pm.nywork, WT, 0, st>>>(pm, sign); break;
-        case 5: k_fft_y_warp<T, 5><<<pm.nywork, WT, 0, st>>>(pm, sign); break;
-        default: k_fft_y<T><<<pm.nywork, LT, lsmem, st>>>(pm, sign);
-      }
-    };
-    fft_y(-1);
-    switch (pm.wx) {
-      case 1: k_fft_x_warp<T, 1><<<pm.nxwork, WX, 0, st>>>(s, pm); break;
-      case 2: k_fft_x_warp<T, 2><<<pm.nxwork, WX, 0, st>>>(s, pm); break;
-      case 3: k_fft_x_warp<T, 3><<<pm.nxwork, WX, 0, st>>>(s, pm); break;
-      case 4: k_fft_x_warp<T, 4><<<pm.nxwork, WX, 0, st>>>(s, pm); break;
-      case 5: k_fft_x_warp<T, 5><<<pm.nxwork, WX, 0, st>>>(s, pm); break;
-      default: k_fft_x_infl<T><<<pm.nxwork, LT, lsmem, st>>>(s, pm);
-    }
-    fft_y(+1);
   }
+  // planes too large for that: y, x with the influence function, y, a launch per form of the lines
+  auto fft_y = [&](int sign) {
+    for (int r = 0; r < 6; r++) {
+      const int n = pm.nywork[r + 1] - pm.nywork[r];
+      if (n <= 0) continue;
+      PmeDev q = pm;
+      q.ywork += pm.nywork[r];
+      switch (r) {
+        case 1: k_fft_y_warp<T, 1><<<n, WT, 0, st>>>(q, sign); break;
+        case 2: k_fft_y_warp<T, 2><<<n, WT, 0, st>>>(q, sign); break;
+        case 3: k_fft_y_warp<T, 3><<<n, WT, 0, st>>>(q, sign); break;
+        case 4: k_fft_y_warp<T, 4><<<n, WT, 0, st>>>(q, sign); break;
+        case 5: k_fft_y_warp<T, 5><<<n, WT, 0, st>>>(q, sign); break;
+        default: k_fft_y<T><<<n, LT, lsmem, st>>>(q, sign);
+      }
+    }
+  };
+  fft_y(-1);
+  for (int r = 0; r < 6; r++) {
+    const int n = pm.nxwork[r + 1] - pm.nxwork[r];
+    if (n <= 0) continue;
+    PmeDev q = pm;
+    q.xwork += pm.nxwork[r];
+    switch (r) {
+      case 1: k_fft_x_warp<T, 1><<<n, WX, 0, st>>>(s, q); break;
+      case 2: k_fft_x_warp<T, 2><<<n, WX, 0, st>>>(s, q); break;
+      case 3: k_fft_x_warp<T, 3><<<n, WX, 0, st>>>(s, q); break;
+      case 4: k_fft_x_warp<T, 4><<<n, WX, 0, st>>>(s, q); break;
+      case 5: k_fft_x_warp<T, 5><<<n, WX, 0, st>>>(s, q); break;
+      default: k_fft_x_infl<T><<<n, LT, lsmem, st>>>(s, q);
+    }
+  }
+  fft_y(+1);
   k_fft_z_inv<T><<<pm.nzwork, ZT, pm.zsmem, st>>>(pm);
   if (mark) mark(mctx, "pme_fft");
   switch (pm.order) {

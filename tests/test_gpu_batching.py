@@ -180,3 +180,22 @@ def test_reciprocal_energy_of_a_box_among_many(precision):
         F.evaluate_all(t1, pme(1), boxes[k]["pos"], f1, e1)
         assert np.array_equal(fb[180 * k:180 * (k + 1)], f1), k
         assert np.array_equal(eb.table[k], e1.table[0]), k
+
+
+# planes that fit the plane kernel beside planes that do not (above 227 KB), the latter with lines of
+# both forms in either direction
+@pytest.mark.parametrize("precision,grids", [
+    ("mixed", [(12, 15, 16), (160, 192, 8), (32, 30, 18), (240, 128, 8), (192, 160, 8), (250, 200, 8)]),
+    ("fp64", [(12, 15, 16), (64, 240, 8), (32, 30, 18), (250, 96, 8), (128, 128, 8), (160, 125, 8)])])
+def test_small_planes_beside_large_ones(precision, grids):
+    boxes = [W.water_box(40 + 7 * k, seed=70 + k) for k in range(len(grids))]
+    pme = lambda g: [F.NonbondedPMEwaldSystemForce((0, 0, 0), 6.0, real=False, box_grids=[list(v) for v in g])]  # noqa: E731
+    topo = F.Topology(boxes, precision)
+    fb, eb = np.zeros((topo.n_atoms, 3)), F.ScalarStructure(len(boxes), virial=True)
+    F.evaluate_all(topo, pme(grids), np.concatenate([b["pos"] for b in boxes]), fb, eb)
+    for k, (b, sl) in enumerate(zip(boxes, slices(boxes))):
+        t1 = F.Topology(b, precision)
+        f1, e1 = np.zeros((t1.n_atoms, 3)), F.ScalarStructure(1, virial=True)
+        F.evaluate_all(t1, pme(grids[k:k + 1]), b["pos"], f1, e1)
+        assert np.array_equal(fb[sl], f1), k
+        assert np.array_equal(eb.table[k], e1.table[0]), k
