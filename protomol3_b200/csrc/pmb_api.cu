@@ -10,8 +10,6 @@
 #include <algorithm>
 #include <atomic>
 #include <chrono>
-#include <condition_variable>
-#include <mutex>
 #include <thread>
 #include <cmath>
 #include <cstring>
@@ -27,6 +25,7 @@
 #endif
 
 #include "../../include/pmb200.h"
+#include "pmb_addpool.h"
 #include "pmb_internal.h"
 
 namespace pmb {
@@ -187,86 +186,6 @@ int valid_switch(int k) { return k == SW_CUTOFF || k == SW_C1 || k == SW_C2; }
 }  // namespace
 
 // ================================================================================== system
-// Threads that add the forces of a host-pointer evaluation into the caller's array, or copy the state
-// of an MD run into it, while the device->host copies land piece by piece: worker k (the calling
-// thread is worker 0) waits for each piece's event and adds or copies its share of the piece.  Between evaluations the workers sleep on
-// a condition variable (spinning would take cores from the caller's own threads).
-struct AddPool {
-  int nthreads = 1, device = 0;
-  std::vector<std::thread> th;
-  std::mutex mu;
-  std::condition_variable cv;
-  std::atomic<long long> gen{0};
-  std::atomic<int> pending{0};
-  std::atomic<bool> stop{false};
-  // the job
-  double *dst = nullptr;
-  const double *src = nullptr;
-  long long n = 0, chunk = 0;
-  int nchunks = 0;
-  const cudaEvent_t *ev = nullptr;  // ev[c]: piece c has landed
-  bool copy = false;                // dst = src instead of dst += src
-
-  void part(int k) {
-    for (int c = 0; c < nchunks; c++) {
-      cudaEventSynchronize(ev[c]);
-      const long long b0 = c * chunk, b1 = std::min(n, b0 + chunk), len = b1 - b0;
-      const long long q0 = b0 + len * k / nthreads, q1 = b0 + len * (k + 1) / nthreads;
-      double *__restrict__ d = dst;
-      const double *__restrict__ s = src;
-      if (copy) std::memcpy(d + q0, s + q0, sizeof(double) * (size_t)(q1 - q0));
-      else
-        for (long long i = q0; i < q1; i++) d[i] += s[i];
-    }
-  }
-  void worker(int k) {
-    cudaSetDevice(device);
-    long long seen = 0;
-    for (;;) {
-      {
-        std::unique_lock<std::mutex> lk(mu);
-        cv.wait(lk, [&] { return stop.load() || gen.load(std::memory_order_acquire) != seen; });
-        if (stop) return;
-        seen = gen.load(std::memory_order_acquire);
-      }
-      part(k);
-      pending.fetch_sub(1, std::memory_order_acq_rel);
-    }
-  }
-  void start(int threads, int dev) {
-    nthreads = threads;
-    device = dev;
-    for (int k = 1; k < nthreads; k++) th.emplace_back([this, k] { worker(k); });
-  }
-  // dst[0..n) += src[0..n) (or =), piece c of `chunk` elements once ev[c] has completed
-  void run(double *d, const double *s, long long n_, long long chunk_, int nchunks_, const cudaEvent_t *ev_,
-           bool copy_ = false) {
-    copy = copy_;
-    dst = d;
-    src = s;
-    n = n_;
-    chunk = chunk_;
-    nchunks = nchunks_;
-    ev = ev_;
-    pending.store(nthreads - 1, std::memory_order_release);
-    {
-      std::lock_guard<std::mutex> lk(mu);
-      gen.fetch_add(1, std::memory_order_acq_rel);
-    }
-    cv.notify_all();
-    part(0);
-    while (pending.load(std::memory_order_acquire) > 0) std::this_thread::yield();
-  }
-  ~AddPool() {
-    {
-      std::lock_guard<std::mutex> lk(mu);
-      stop = true;
-    }
-    cv.notify_all();
-    for (std::thread &t : th) t.join();
-  }
-};
-
 // A host-pointer evaluation captured as a CUDA graph: the force passes, the conversions and the
 // device->host copies with their events, for one force set and virial flag.
 struct EvalGraph {
@@ -922,9 +841,10 @@ int ensure_add_pool(pmb_system *s) {
   int dev = 0;
   CK(cudaGetDevice(&dev));
   s->add_pool = new AddPool();
-  s->add_pool->start((int)std::max(1u, std::min(4u, hw / 4)), dev);
+  s->add_pool->start((int)std::max(1u, std::min(4u, hw / 4)), [](int d) { cudaSetDevice(d); }, dev);
   return PMB_OK;
 }
+int wait_event(const void *events, int c) { return (int)cudaEventSynchronize(static_cast<const cudaEvent_t *>(events)[c]); }
 
 // True when both ends of the n doubles at p are page-locked host memory (cudaMallocHost,
 // cudaHostAlloc or cudaHostRegister), which the copy engines read and write directly.
@@ -1821,7 +1741,7 @@ int pmb_evaluate(pmb_system *s, pmb_force *const *fs, int n, const double *pos, 
     } else if (forces && nf >= (1 << 16)) {
       // large systems: the pool's threads share every piece as it lands
       if (int rc2 = ensure_add_pool(s)) return rc2;
-      s->add_pool->run(forces, s->h_fout, nf, chunk, pmb_system::EVAL_CHUNKS, s->ev_out + 1);
+      CK((cudaError_t)s->add_pool->run(forces, s->h_fout, nf, chunk, pmb_system::EVAL_CHUNKS, wait_event, s->ev_out + 1));
     } else {
       for (int c = 0; c < pmb_system::EVAL_CHUNKS; c++) {
         CK(cudaEventSynchronize(s->ev_out[c + 1]));
@@ -2478,7 +2398,8 @@ int pmb_md_get_state(pmb_md *m, double *pos, double *vel) {
         CK(cudaEventRecord(m->ev_state[q * NC + c], s->stream));
       }
     for (int q = 0; q < 2; q++)
-      if (parts[q].dst) s->add_pool->run(parts[q].dst, parts[q].stage, nf, chunk, NC, m->ev_state + q * NC, true);
+      if (parts[q].dst)
+        CK((cudaError_t)s->add_pool->run(parts[q].dst, parts[q].stage, nf, chunk, NC, wait_event, m->ev_state + q * NC, true));
     return check_status(s);
   }
   if (pos) CK(cudaMemcpyAsync(pos, s->d_pos, sizeof(double) * nf, cudaMemcpyDeviceToHost, s->stream));
