@@ -1386,7 +1386,9 @@ pmb_force *pmb_force_create(pmb_system *s, const pmb_force_desc *d) {
       const int rows = std::max(1, std::min(PME_YROWS, lcap / pl.n[1])),
                 cols = std::max(1, std::min(PME_XCOLS, lcap / pl.n[0]));
       // (one row per warp of a 4-warp block, one column per warp of an 8-warp block)
-      auto warp_r = [](int n) { return n % 32 == 0 && n <= 160 ? n / 32 : 0; };
+      auto warp_r = [&](int n) {
+        return n % 32 == 0 && n / 32 >= WARP_R_MIN[s->precision ? 1 : 0] && n / 32 <= WARP_R_MAX ? n / 32 : 0;
+      };
       const int ry = PME_YROWS <= 4 ? warp_r(pl.n[1]) : 0, rx = PME_XCOLS * 32 <= PME_WX_THREADS ? warp_r(pl.n[0]) : 0;
       if (!planes) lbuf = std::max(lbuf, std::max(rows * pl.n[1], cols * pl.n[0]));
       for (int kz = 0; kz <= pl.n[2] / 2; kz++) {

@@ -184,8 +184,8 @@ struct PmeDev {
   const int *radix;           // radices per dim
   const int4 *zwork;          // z-pass work items: box, x, y0, count
   int nzwork;
-  // planes too large for the plane kernel: line work items, those of lines of 32 R points (R <= 5, the
-  // warp-shuffle transforms) from item [R] up to [R + 1], those of the shared-memory ones from [0]
+  // planes too large for the plane kernel: line work items, those of lines of 32 R points
+  // (WARP_R_MIN <= R <= WARP_R_MAX, the warp-shuffle transforms) from item [R] up to [R + 1], those of the shared-memory ones from [0]
   const int4 *ywork;          // box, kz, x0, rows
   int nywork[7];
   const int4 *xwork;          // box, kz, y0, columns
@@ -215,6 +215,8 @@ int pme_line_capacity();
 // Plane kernel: most threads, most shared memory, the stages of a line, a plane's shared memory.
 constexpr int PLANE_MAX_THREADS = 512;
 constexpr int PLANE_SMEM_MAX = 227 * 1024;
+// Warp-shuffle lines of 32 R points: the shortest in a plane that does not fit (FP64, mixed), the longest.
+constexpr int WARP_R_MIN[2] = {2, 4}, WARP_R_MAX = 5;
 bool pme_plane_radices(int n, std::vector<int> &radices);
 size_t pme_plane_smem(int nx, int ny, int precision);
 constexpr int Z_SMEM_MAX = 48 * 1024;  // z kernels: 16 lines of 256 points in FP64 take 37 KB

@@ -87,12 +87,6 @@ __device__ __forceinline__ void dft_small(T2 *v, int sign) {
   }
 }
 
-// dft_small for R = 1 .. 5 (R = 1: nothing to do).
-template <int R, typename T2>
-__device__ __forceinline__ void dft_small_any(T2 *v, int sign) {
-  if constexpr (R > 1) dft_small<R>(v, sign);
-}
-
 // floor(a / d) for 0 <= a < 2^21 from r ~ 1/d (a few ulp suffice: (a + 1/2) / d stays at least
 // 1/(2d) away from an integer), without an integer division.
 __device__ __forceinline__ int divf(int a, float r) { return __float2int_rz(((float)a + 0.5f) * r); }
@@ -522,7 +516,7 @@ __device__ __forceinline__ WarpTw<R, T2> warp_twiddles(const TW *tw) {
 template <int R, typename T2>
 __device__ __forceinline__ void warp_fft_fwd(T2 v[R], const WarpTw<R, T2> &w) {
   const int lane = threadIdx.x & 31;
-  dft_small_any<R>(v, -1);
+  dft_small<R>(v, -1);
 #pragma unroll
   for (int k = 1; k < R; k++) v[k] = cmul(v[k], w.rk[k]);
 #pragma unroll
@@ -553,7 +547,7 @@ __device__ __forceinline__ void warp_fft_inv(T2 v[R], const WarpTw<R, T2> &w) {
   }
 #pragma unroll
   for (int k = 1; k < R; k++) v[k] = cmulc(v[k], w.rk[k]);
-  dft_small_any<R>(v, +1);
+  dft_small<R>(v, +1);
 }
 
 constexpr int WT = 128;  // threads of the warp-transform y kernel (one row per warp)
@@ -733,7 +727,7 @@ __device__ __forceinline__ void dft_composite(T2 *v) {
 }
 template <int R, int SIGN, typename T2>
 __device__ __forceinline__ void dft_reg(T2 *v) {
-  if constexpr (R <= 5) dft_small_any<R>(v, SIGN);
+  if constexpr (R <= 5) dft_small<R>(v, SIGN);
   else if constexpr (R == 6) dft_composite<2, 3, SIGN>(v);
   else dft_composite<2, 4, SIGN>(v);
 }
@@ -1195,19 +1189,20 @@ int recip_t(const SystemDev &s, const NbListDev &nb, const PmeDev &pm, cudaStrea
     kern<<<pm.npwork, pm.pthreads, pm.psmem, st>>>(s, pm);
   }
   // planes too large for that: y, x with the influence function, y, a launch per form of the lines
+  // (lines are of at most 256 points, so such planes have lines of 64, in FP32 of 128 points or more:
+  // WARP_R_MIN of the plan)
   auto fft_y = [&](int sign) {
     for (int r = 0; r < 6; r++) {
       const int n = pm.nywork[r + 1] - pm.nywork[r];
       if (n <= 0) continue;
       PmeDev q = pm;
       q.ywork += pm.nywork[r];
-      switch (r) {
-        case 1: k_fft_y_warp<T, 1><<<n, WT, 0, st>>>(q, sign); break;
-        case 2: k_fft_y_warp<T, 2><<<n, WT, 0, st>>>(q, sign); break;
-        case 3: k_fft_y_warp<T, 3><<<n, WT, 0, st>>>(q, sign); break;
-        case 4: k_fft_y_warp<T, 4><<<n, WT, 0, st>>>(q, sign); break;
-        case 5: k_fft_y_warp<T, 5><<<n, WT, 0, st>>>(q, sign); break;
-        default: k_fft_y<T><<<n, LT, lsmem, st>>>(q, sign);
+      if (r == 0) k_fft_y<T><<<n, LT, lsmem, st>>>(q, sign);
+      else if (r == 5) k_fft_y_warp<T, 5><<<n, WT, 0, st>>>(q, sign);
+      else if (r == 4) k_fft_y_warp<T, 4><<<n, WT, 0, st>>>(q, sign);
+      else if constexpr (!MIXED) {
+        if (r == 3) k_fft_y_warp<T, 3><<<n, WT, 0, st>>>(q, sign);
+        else k_fft_y_warp<T, 2><<<n, WT, 0, st>>>(q, sign);
       }
     }
   };
@@ -1217,13 +1212,12 @@ int recip_t(const SystemDev &s, const NbListDev &nb, const PmeDev &pm, cudaStrea
     if (n <= 0) continue;
     PmeDev q = pm;
     q.xwork += pm.nxwork[r];
-    switch (r) {
-      case 1: k_fft_x_warp<T, 1><<<n, WX, 0, st>>>(s, q); break;
-      case 2: k_fft_x_warp<T, 2><<<n, WX, 0, st>>>(s, q); break;
-      case 3: k_fft_x_warp<T, 3><<<n, WX, 0, st>>>(s, q); break;
-      case 4: k_fft_x_warp<T, 4><<<n, WX, 0, st>>>(s, q); break;
-      case 5: k_fft_x_warp<T, 5><<<n, WX, 0, st>>>(s, q); break;
-      default: k_fft_x_infl<T><<<n, LT, lsmem, st>>>(s, q);
+    if (r == 0) k_fft_x_infl<T><<<n, LT, lsmem, st>>>(s, q);
+    else if (r == 5) k_fft_x_warp<T, 5><<<n, WX, 0, st>>>(s, q);
+    else if (r == 4) k_fft_x_warp<T, 4><<<n, WX, 0, st>>>(s, q);
+    else if constexpr (!MIXED) {
+      if (r == 3) k_fft_x_warp<T, 3><<<n, WX, 0, st>>>(s, q);
+      else k_fft_x_warp<T, 2><<<n, WX, 0, st>>>(s, q);
     }
   }
   fft_y(+1);

@@ -250,3 +250,17 @@ def test_sort_of_many_boxes(sizes):
             g = np.zeros_like(p)
             F.evaluate_all(t, one, p, g, F.ScalarStructure(1))
             np.testing.assert_array_equal(f[at[k]:at[k + 1]], g)
+
+
+# planes above 227 KB: lines of both forms in either direction, the shortest and longest of each
+@pytest.mark.parametrize("precision,grid", [
+    ("mixed", (160, 192, 8)), ("mixed", (240, 128, 9)), ("mixed", (192, 160, 8)), ("mixed", (128, 240, 10)),
+    ("mixed", (250, 200, 8)), ("mixed", (256, 256, 8)), ("fp64", (64, 240, 8)), ("fp64", (240, 64, 9)),
+    ("fp64", (250, 96, 8)), ("fp64", (96, 250, 10)), ("fp64", (128, 128, 8)), ("fp64", (160, 160, 8)), ("fp64", (150, 125, 8))])
+def test_planes_too_large_for_shared_memory(precision, grid):
+    b = shaken(60, 7)
+    pme = F.NonbondedPMEwaldSystemForce(grid, 6.0, real=False, correction=False)
+    f, e, _ = evaluate(b, [pme], precision, virial=True)
+    fo, eo, vo, _ = O.evaluate(O.System(b), b["pos"], pme=O.pme_params(grid, 6.0, real=0, recip=1, corr=0), virial=True)
+    assert rel(f, fo) < TOL[precision]
+    np.testing.assert_allclose(e.virial().ravel(), vo, rtol=0, atol=10 * TOL[precision] * np.abs(vo).max())
