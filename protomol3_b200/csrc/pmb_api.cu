@@ -1025,9 +1025,8 @@ pmb_system *pmb_system_create(const pmb_box_desc *boxes, int n_boxes, int precis
     epart[estart[b] + fill[b]] = a;
     ekind[estart[b] + fill[b]++] = s->h_excl_kind[k];
   }
-  // Slot blocks of the boxes in order of decreasing smallest edge (stable): boxes small enough to
-  // need Ewald lattice images come last in the tile map, so the pair kernel's lattice-image
-  // instance runs over that suffix alone.  Atoms keep the caller's order.
+  // Slot blocks of the boxes in order of decreasing smallest edge (stable): the list build claims blocks in
+  // ascending order, the work of the large boxes first.  Atoms keep the caller's order.
   {
     std::vector<int> order(s->nbox);
     for (int bi = 0; bi < s->nbox; bi++) order[bi] = bi;
@@ -1302,7 +1301,10 @@ pmb_force *pmb_force_create(pmb_system *s, const pmb_force_desc *d) {
     // z-lines a CTA: eight where sixteen would leave fewer than four CTAs an SM (216 waters: 25
     // steps 975 us with eight, 989 with all 20 lines of a plane in one CTA; 96^3, just under the line:
     // the same either way)
-    const int zlines = points < 16.0 * 4 * 148 ? 8 : 16;
+    int dev = 0, n_sm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      return bad(PMB_ERR_CUDA, "device query failed");
+    const int zlines = points < 16.0 * 4 * n_sm ? 8 : 16;
     double th0[8];
     bspline_h(P, 0.0, th0);
     for (int bi = 0; bi < nbox; bi++) {

@@ -1,10 +1,11 @@
 """A box gives the same bits alone and inside a batch of boxes (one system, one launch per force
 stage), and when it moves from one batched run to another part-way.
 
-What makes it so: neighbour-list rebuilds are decided box by box; every box's pair tiles start at
-a multiple of the pair kernel's warp assignment, so the kernel's floating-point partial sums are
-grouped as when the box is alone; energies are rounded to fixed point term by term; the Langevin
-noise of an atom is keyed by its box's seed, its index within the box and its box's step count.
+What makes it so: neighbour-list rebuilds are decided box by box; the pair kernel closes its
+floating-point partial sums every two tiles of a list, however the lists are cut into work; each box
+takes the transforms of its own grid, and their energy sums do not depend on the order; energies are
+rounded to fixed point term by term; the Langevin noise of an atom is keyed by its box's seed, its
+index within the box and its box's step count.
 The oracle comparisons of batched systems are in test_gpu_parity.py; here the GPU path is
 compared with itself, bit for bit.
 """

@@ -94,8 +94,8 @@ def test_pme_vs_oracle(precision, nw, grid, rc):
                                         ((96, 128, 128), 4)])
 def test_pme_anisotropic_grid_and_order(precision, grid, order):
     """Grid lengths of pure radix 5, 3 and 2 in different dimensions and interpolation orders
-    other than 4 (the generic spread/gather instance); lengths of 32 R points (R = 1 to 5) take
-    the warp-shuffle transforms in that dimension, the others the shared-memory ones."""
+    other than 4 (their own spread/gather instances); planes of up to 96 x 128 points, which
+    all fit the plane kernel (larger ones: test_gpu_paths.py)."""
     b = W.water_box(216, seed=11)
     pme = F.NonbondedPMEwaldSystemForce(grid, 8.0, order=order)
     f, e, topo = gpu_eval(b, [pme], precision, virial=True)
