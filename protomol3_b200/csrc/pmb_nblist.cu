@@ -287,8 +287,11 @@ __global__ void __launch_bounds__(SORT_BOX_THREADS) k_sort_box(SystemDev s, NbLi
 static_assert(SORT_THREADS == SORT_PART, "a thread takes a slot");
 constexpr int EXT_THREADS = SORT_PART / 8;  // a warp takes a superblock, 32 blocks of 8 slots
 static_assert(BLOCK == 8, "256 slots a superblock");
+__device__ __forceinline__ int2 sort_item(const NbListDev &nb) {  // box, part (of one box: no table to wait for)
+  return nb.nbox == 1 ? make_int2(0, blockIdx.x) : nb.sort_work[blockIdx.x];
+}
 __global__ void __launch_bounds__(SORT_THREADS) k_sort_bin(SystemDev s, NbListDev nb) {
-  const int2 it = nb.sort_work[blockIdx.x];  // box, part
+  const int2 it = sort_item(nb);
   if (!nb.ctl[CTL_REBUILD] || !nb.box_rb[it.x]) return;
   const BoxDev &b = s.box[it.x];
   const int parts = (b.nblk * BLOCK + SORT_PART - 1) / SORT_PART;
@@ -340,19 +343,19 @@ __global__ void __launch_bounds__(SORT_THREADS) k_scan_apply(SystemDev s, NbList
   }
 }
 __global__ void __launch_bounds__(SORT_THREADS) k_sort_scatter(SystemDev s, NbListDev nb) {
-  const int2 it = nb.sort_work[blockIdx.x];
+  const int2 it = sort_item(nb);
   if (!nb.ctl[CTL_REBUILD] || !nb.box_rb[it.x]) return;
   const BoxDev &b = s.box[it.x];
   sort_scatter(nb, b, it.y * SORT_PART + threadIdx.x, b.nblk * BLOCK + SORT_PART);
 }
 __global__ void __launch_bounds__(SORT_THREADS) k_sort_place(SystemDev s, NbListDev nb) {
-  const int2 it = nb.sort_work[blockIdx.x];
+  const int2 it = sort_item(nb);
   if (!nb.ctl[CTL_REBUILD] || !nb.box_rb[it.x]) return;
   const BoxDev &b = s.box[it.x];
   sort_place(s, nb, b, it.x, it.y * SORT_PART + threadIdx.x, b.nblk * BLOCK + SORT_PART);
 }
 __global__ void __launch_bounds__(EXT_THREADS) k_sort_extents(SystemDev s, NbListDev nb) {
-  const int2 it = nb.sort_work[blockIdx.x];
+  const int2 it = sort_item(nb);
   if (!nb.ctl[CTL_REBUILD] || !nb.box_rb[it.x]) return;
   const BoxDev &b = s.box[it.x];
   sort_extents(nb, b, it.y * EXT_THREADS + threadIdx.x, b.nblk + EXT_THREADS);
