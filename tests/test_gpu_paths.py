@@ -264,3 +264,19 @@ def test_planes_too_large_for_shared_memory(precision, grid):
     fo, eo, vo, _ = O.evaluate(O.System(b), b["pos"], pme=O.pme_params(grid, 6.0, real=0, recip=1, corr=0), virial=True)
     assert rel(f, fo) < TOL[precision]
     np.testing.assert_allclose(e.virial().ravel(), vo, rtol=0, atol=10 * TOL[precision] * np.abs(vo).max())
+
+
+# the largest box of each block size of the one-CTA sort (64 to 1,024 threads), and one atom more
+@pytest.mark.parametrize("atoms", [63, 64, 65, 128, 129, 256, 257, 512, 513, 1023, 1025])
+def test_one_cta_sort_of_each_size(atoms):
+    rng = np.random.default_rng(atoms)
+    edge = max(10.0, (10.0 * atoms) ** (1.0 / 3.0))
+    b = dict(box=np.full(3, edge), charge=np.where(np.arange(atoms) % 2, 18.2, -18.2), type=np.zeros(atoms, np.int32),
+             molecule=np.arange(atoms, dtype=np.int32), lj=np.zeros(4), mass=np.ones(atoms))
+    topo = F.Topology(b, "fp64")
+    for _ in range(2):
+        pos = rng.uniform(0.0, edge, (atoms, 3))
+        f = np.zeros_like(pos)
+        F.evaluate_all(topo, [F.NonbondedCutoffSystemForce(coulomb=("C1", 0.0, 4.5))], pos, f, F.ScalarStructure(1))
+        fo, _, _, _ = O.evaluate(O.System(dict(b, pos=pos)), pos, cutoff=O.cutoff_params(coul=("C1", 0.0, 4.5)))
+        assert rel(f, fo) < TOL["fp64"]
